@@ -176,7 +176,7 @@ struct cfsa_ns {
   double *cg1_vec[3] = {nullptr, nullptr, nullptr};  // second r, w, s buffers of k_cg1_resident
   int cg_res_grid = 0, cg_res_bpc_sell = 0, cg_res_bpc_nat = 0, cg_res_col_cap = 0;
   size_t cg_res_smem = 0;
-  unsigned int *bar_count = nullptr, *bar_gen = nullptr;
+  unsigned int *bar_count = nullptr;
   int *bar_err = nullptr;
   long long bar_spin_limit = kBarrierSpinLimit;
   // raw Poisson operator of solvePressureBiCGSTAB (no penalty rows), column-scaled by its inverse
@@ -590,12 +590,9 @@ struct cfsa_ns {
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_persistent, kBlock, 0));
       const int nblk_sell = (int)blocks_for(s1.nrows_pad), nblk_nat = (int)blocks_for(nv);
       cg_grid = std::min(nsm * per_sm, std::max(nblk_sell, nblk_nat));
-      cg_grid = std::min(cg_grid, kBarrierGroupSize * kBarrierGroups);
-      bar_count = dalloc<unsigned int>(1 + kBarrierGroups);
-      bar_gen = dalloc<unsigned int>(1);
+      bar_count = dalloc<unsigned int>(1);
       bar_err = dalloc<int>(1);
-      CK(cudaMemsetAsync(bar_count, 0, (1 + kBarrierGroups) * sizeof(unsigned int), stream));
-      CK(cudaMemsetAsync(bar_gen, 0, sizeof(unsigned int), stream));
+      CK(cudaMemsetAsync(bar_count, 0, sizeof(unsigned int), stream));
       CK(cudaMemsetAsync(bar_err, 0, sizeof(int), stream));
       cg_part_a = dalloc<double>((size_t)std::max(nblk_sell, nblk_nat) * kMaxRed);
       cg_part_b = dalloc<double>((size_t)std::max(nblk_sell, nblk_nat) * kMaxRed);
@@ -1304,7 +1301,7 @@ struct cfsa_ns {
     c.part_b = cg_part_b;
     c.cs = state;
     c.st = s_out;
-    c.bar = GridBarrier{bar_count, bar_gen, bar_err, bar_spin_limit};
+    c.bar = GridBarrier{bar_count, bar_err, bar_spin_limit};
     c.scaled = (conv_norm == CFSA_NORM_JACOBI) ? 1 : 0;
     CgResidentArgs rz{};
     rz.P = c;
@@ -1339,7 +1336,7 @@ struct cfsa_ns {
   // One cooperative launch of the two-level CG on `s` (barrier words and coarse accumulators
   // cleared first; the caller zeroes p and s[0] of the form it launches).
   void launch_cg2l(const Cg2lArgs &c2, bool f32, cudaStream_t s) {
-    CK(cudaMemsetAsync(bar_count, 0, (1 + kBarrierGroups) * sizeof(unsigned int), s));
+    CK(cudaMemsetAsync(bar_count, 0, sizeof(unsigned int), s));
     CK(cudaMemsetAsync(bar_err, 0, sizeof(int), s));
     if (coarse_view.nc > 0)
       CK(cudaMemsetAsync(coarse_view.gacc, 0, (size_t)27 * coarse_view.nc * sizeof(unsigned long long), s));
@@ -1467,9 +1464,9 @@ struct cfsa_ns {
       c.part_b = cg_part_b;
       c.cs = cs;
       c.st = s_out;
-      c.bar = GridBarrier{bar_count, bar_gen, bar_err, bar_spin_limit};
+      c.bar = GridBarrier{bar_count, bar_err, bar_spin_limit};
       c.scaled = (conv_norm == CFSA_NORM_JACOBI) ? 1 : 0;
-      CK(cudaMemsetAsync(bar_count, 0, (1 + kBarrierGroups) * sizeof(unsigned int), stream));
+      CK(cudaMemsetAsync(bar_count, 0, sizeof(unsigned int), stream));
       CK(cudaMemsetAsync(bar_err, 0, sizeof(int), stream));
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned int)cg_grid);
