@@ -8,6 +8,7 @@
 #include "ns_adjoint.cuh"
 #include "ns_kernels.cuh"
 #include "ns_mixed.cuh"
+#include "ns_resident.cuh"
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -36,31 +37,43 @@ struct NvtxRange {
   ~NvtxRange() { nvtxRangePop(); }
 };
 
+// Operators of at most this many rows are solved by one CTA, whose barriers are block-wide ones: a
+// momentum CG iteration of 549 rows takes 17 us in one CTA and 20 us on several, of 1037 rows 23 and 20.
+constexpr int kOneCtaRows = 768;
+
 struct Sell {
   int *sptr = nullptr, *col = nullptr, *len = nullptr, *perm = nullptr, *posmap = nullptr;
   int nrows = 0, nrows_pad = 0, nslices = 0;
   int64_t nentries = 0;
   std::vector<int> h_sptr;  // host copy of sptr
   int *rfirst = nullptr;    // slice runs of the run-walking kernels (one per SM)
-  double *spart = nullptr;  // their per-slice warp sums
-  int nruns = 0;
-  SellView view() const { return SellView{sptr, col, len, perm, nrows_pad, rfirst, spart}; }
+  int nruns = 0, max_run = 0;  // CTAs, most slices of one CTA
+  SellView view() const { return SellView{sptr, col, len, perm, nrows_pad, rfirst}; }
 };
 
-// Entry-balanced runs of slices, one per CTA of a run-walking kernel, split on 256-row block
-// boundaries: run c starts at the first block boundary at or after c/nruns of the entries.
-std::vector<int> slice_runs(const std::vector<int> &sptr, int nslices, int nruns) {
-  std::vector<int> f(nruns + 1, 0);
-  const int64_t ne = sptr[nslices];
-  for (int c = 1; c < nruns; ++c) {
-    const int64_t target = ne * c / nruns;
-    int sl = (int)(std::lower_bound(sptr.begin(), sptr.begin() + nslices + 1, target,
-                                    [](int a, int64_t t) { return (int64_t)a < t; }) -
-                   sptr.begin());
-    sl = (sl + kSlicesPerBlock - 1) / kSlicesPerBlock * kSlicesPerBlock;
-    f[c] = std::max(f[c - 1], std::min(sl, nslices));
+// Slice runs of the resident Krylov solves, on 256-row block boundaries (cut, the first slice of the
+// second part, is one): CTA c takes [f[c], f[c+1]) of the slices below cut and [g[c], g[c+1]) of the
+// rest, g = f + nruns + 1. The first part (vertex rows, 65 entries) is split by entries; the second
+// (edge rows, 23 entries) so that the entries of both parts together are balanced. Splitting the two
+// parts side by side instead of the whole range in one run per CTA spreads the long rows over all CTAs
+// (one run: the CTAs of the vertex rows took 42 us of a 250k-tet product whose mean is 30 us).
+std::vector<int> slice_runs(const std::vector<int> &sptr, int cut, int nslices, int nruns) {
+  std::vector<int> f;
+  const auto boundary = [&](int lo, int hi, int64_t entry) {  // first block boundary at or after `entry`
+    const int sl = (int)(std::lower_bound(sptr.begin() + lo, sptr.begin() + hi + 1, entry,
+                                          [](int x, int64_t t) { return (int64_t)x < t; }) -
+                         sptr.begin());
+    return std::min(hi, (sl + kSlicesPerBlock - 1) / kSlicesPerBlock * kSlicesPerBlock);
+  };
+  const int64_t na = sptr[cut], n = sptr[nslices];
+  for (int c = 0; c <= nruns; ++c)
+    f.push_back(boundary(0, cut, na * c / nruns));
+  for (int c = 0; c <= nruns; ++c) {
+    const int64_t target = std::max(na, na + n * c / nruns - sptr[f[c]]);
+    f.push_back(boundary(cut, nslices, target));
   }
-  f[nruns] = nslices;
+  for (int c = 0; c < nruns; ++c) f[nruns + 2 + c] = std::max(f[nruns + 2 + c], f[nruns + 1 + c]);
+  f[2 * nruns + 1] = nslices;
   return f;
 }
 
@@ -176,6 +189,10 @@ struct cfsa_ns {
   double *cg1_vec[3] = {nullptr, nullptr, nullptr};  // second r, w, s buffers of k_cg1_resident
   int cg_res_grid = 0, cg_res_bpc_sell = 0, cg_res_bpc_nat = 0, cg_res_col_cap = 0;
   size_t cg_res_smem = 0;
+  double *res_part = nullptr;  // block partials of the resident Krylov solves, [2][kMaxRed][res_stride]
+  int res_stride = 0;
+  double *res_slots = nullptr;  // their chunk sums where shared memory would cost too much L1
+  double *pv2 = nullptr, *pp2 = nullptr;  // second buffers of the pressure BiCGSTAB's v and p
   unsigned int *bar_count = nullptr;
   int *bar_err = nullptr;
   long long bar_spin_limit = kBarrierSpinLimit;
@@ -295,7 +312,7 @@ struct cfsa_ns {
   }
 
   // ------------------------------------------------------------------ set-up
-  void build_sell(int n, const std::vector<int> &rp, Sell &S, const int *d_rp, const int *d_ci) {
+  void build_sell(int n, int split, const std::vector<int> &rp, Sell &S, const int *d_rp, const int *d_ci) {
     S.nrows = n;
     S.nrows_pad = (n + kSellC - 1) / kSellC * kSellC;
     S.nslices = S.nrows_pad / kSellC;
@@ -324,9 +341,13 @@ struct cfsa_ns {
     {
       int nsm = 0;
       CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-      S.nruns = std::max(1, nsm);
-      S.rfirst = dupload(slice_runs(sptr, S.nslices, S.nruns));
-      S.spart = dalloc<double>((size_t)S.nslices * kMaxRed);
+      // two runs per SM (rows below `split`, a block boundary, and the rest), no more CTAs than blocks
+      S.nruns = n <= kOneCtaRows ? 1 : std::max(1, std::min(nsm, (S.nslices + kSlicesPerBlock - 1) / kSlicesPerBlock));
+      const int cut = std::min(S.nslices, split / kBlock * kSlicesPerBlock);
+      const std::vector<int> first = slice_runs(sptr, cut, S.nslices, S.nruns);
+      for (int c = 0; c < S.nruns; ++c)
+        S.max_run = std::max(S.max_run, first[c + 1] - first[c] + first[S.nruns + c + 2] - first[S.nruns + c + 1]);
+      S.rfirst = dupload(first);
     }
     S.perm = dupload(perm);
     S.len = dupload(len);
@@ -441,8 +462,8 @@ struct cfsa_ns {
     k_diag_pos<<<blocks_for(N2), kBlock, 0, stream>>>((int)N2, rp2, ci2, dpos2);
     k_diag_pos<<<blocks_for(nv), kBlock, 0, stream>>>((int)nv, rp1, ci1, dpos1);
     CK(cudaGetLastError());
-    build_sell((int)N2, h_rp2, s2, rp2, ci2);
-    build_sell((int)nv, h_rp1, s1, rp1, ci1);
+    build_sell((int)N2, (int)nv, h_rp2, s2, rp2, ci2);
+    build_sell((int)nv, 0, h_rp1, s1, rp1, ci1);
     tpos1 = dalloc<int>((size_t)nnz1);
     k_transpose_slots<<<blocks_for(nnz1), kBlock, 0, stream>>>(nnz1, rows1, rp1, ci1, tpos1, d_err);
     CK(cudaGetLastError());
@@ -488,6 +509,10 @@ struct cfsa_ns {
     // reductions and states
     const int64_t maxrows = std::max<int64_t>({(int64_t)s2.nrows_pad, nt, N2});
     red.partials = dalloc<double>((size_t)(blocks_for(maxrows) + 1) * kMaxRed);
+    res_stride = (int)blocks_for(maxrows);
+    res_part = dalloc<double>((size_t)2 * kMaxRed * res_stride);
+    res_slots = dalloc<double>((size_t)s2.nruns * resident_chunks(s2) * 6);
+    for (double **w : {&pv2, &pp2}) *w = dalloc<double>(nv);
     red.counter = dalloc<unsigned int>(1);
     CK(cudaMemsetAsync(red.counter, 0, sizeof(unsigned int), stream));
     bs_mom = dalloc<BicgState>(1);
@@ -575,25 +600,19 @@ struct cfsa_ns {
           CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kBlock, 0));
           stride_ctas_of[fn] = std::max(o, 1) * nsm;
         };
-        q((const void *)k_bicg_xr<3>);
-        q((const void *)k_bicg_xr<1>);
-        q((const void *)k_mcg_xr<3>);
         q((const void *)k_momentum_rhs);
         q((const void *)k_finish_step);
-        q((const void *)k_mpc_xr);
         q((const void *)k_mpc_init);
         q((const void *)k_mcg_init<3>);
-        q((const void *)k_mp_xr);
         q((const void *)k_mp_init);
         q((const void *)k_pmx_prep);
       }
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_persistent, kBlock, 0));
       const int nblk_sell = (int)blocks_for(s1.nrows_pad), nblk_nat = (int)blocks_for(nv);
       cg_grid = std::min(nsm * per_sm, std::max(nblk_sell, nblk_nat));
-      bar_count = dalloc<unsigned int>(1);
-      bar_err = dalloc<int>(1);
-      CK(cudaMemsetAsync(bar_count, 0, sizeof(unsigned int), stream));
-      CK(cudaMemsetAsync(bar_err, 0, sizeof(int), stream));
+      bar_count = dalloc<unsigned int>(2);  // arrivals, then the error word: one memset clears both
+      bar_err = reinterpret_cast<int *>(bar_count + 1);
+      clear_barrier(stream);
       cg_part_a = dalloc<double>((size_t)std::max(nblk_sell, nblk_nat) * kMaxRed);
       cg_part_b = dalloc<double>((size_t)std::max(nblk_sell, nblk_nat) * kMaxRed);
       for (double *&v : cg1_vec) v = dalloc<double>((size_t)nv);
@@ -1017,21 +1036,52 @@ struct cfsa_ns {
     return std::min(nblk, std::max(need, (unsigned int)it->second));
   }
 
-  template <int NC>
-  void bicg_body(BicgArgs a, cudaStream_t s, const Sell &S, int n) {
-    const unsigned int gs = blocks_for(S.nrows_pad), gp = blocks_for(n);
-    k_bicg_p<NC><<<gs, kBlock, 0, s>>>(a);
-    k_bicg_v<NC><<<S.nruns, kRunThreads, 0, s>>>(a);
-    k_bicg_s<NC><<<gp, kBlock, 0, s>>>(a);
-    k_bicg_t<NC><<<S.nruns, kRunThreads, 0, s>>>(a);
-    k_bicg_xr<NC><<<strided(k_bicg_xr<NC>, gp), kBlock, 0, s>>>(a);
+  void clear_barrier(cudaStream_t s) { CK(cudaMemsetAsync(bar_count, 0, 2 * sizeof(unsigned int), s)); }
+
+  // One cooperative launch of a resident Krylov solve (ns_resident.cuh) over the runs of S. The chunk
+  // sums of a CTA's phase stay in shared memory up to kMaxSlotBytes (1M tets: 14 KB, 4M: 55 KB); past
+  // that they go to global memory, since shared memory taken here is L1 the gathers lose.
+  static constexpr size_t kMaxSlotBytes = 32768;
+  static int resident_chunks(const Sell &S) {
+    const int nblk = (int)blocks_for(S.nrows);
+    return std::max(S.max_run, kSlicesPerBlock * ((nblk + S.nruns - 1) / S.nruns));
+  }
+  // Two forms of each kernel: many threads with short chunks of a row in flight, or fewer threads with
+  // longer chunks. Rows to spare per thread hide the chunk's latency in the first form, a short run of
+  // rows wants it paid less often. Measured per momentum iteration, CG / BiCGSTAB, FP64, us:
+  //   rows        1024 threads, 4 entries   640 threads, 5 entries
+  //   144,499     48.8 /  84.6              37.4 /  74.8
+  //   355,395     66.2 / 119                59.9 / 121
+  //   696,987     110.5 / 213               108 / 228
+  //   1,378,515   182 (CG)                  193 (CG)
+  static constexpr int kFewRows = 450000;
+#define CFSA_RESIDENT(kernel, args, S, s, ...)                                                              \
+  ((S).nrows < kFewRows ? launch_resident(kernel<640, 5 __VA_OPT__(, 6)>, 640, args, S, s)                 \
+                        : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
+  template <class Args>
+  void launch_resident(void (*kernel)(Args, ResidentArgs), int threads, const Args &a, const Sell &S, cudaStream_t s) {
+    const int chunks = resident_chunks(S);
+    const size_t slot_bytes = (size_t)chunks * 6 * sizeof(double);
+    ResidentArgs r{};
+    r.bar = GridBarrier{bar_count, bar_err, kBarrierSpinLimit};
+    r.part = res_part;
+    r.stride = res_stride;
+    r.slots = slot_bytes > kMaxSlotBytes ? res_slots : nullptr;
+    r.slots_per_cta = chunks * 6;
+    clear_barrier(s);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned int)S.nruns);
+    cfg.blockDim = dim3((unsigned int)threads);
+    cfg.dynamicSmemBytes = r.slots ? 0 : slot_bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, kernel, a, r));
   }
 
-  bool poll_bicg(const BicgState *d) {
-    CK(cudaMemcpyAsync(h_bs, d, sizeof(BicgState), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
-    return h_bs->active != 0;
-  }
   bool poll_cg() {
     CK(cudaMemcpyAsync(h_cs, cs, sizeof(CgState), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
@@ -1097,40 +1147,26 @@ struct cfsa_ns {
     m.cw = (conv_norm == CFSA_NORM_JACOBI) ? invA : nullptr;
     k_momentum_rhs<<<strided(k_momentum_rhs, blocks_for(s2.nrows_pad)), kBlock, 0, stream>>>(m);
     CK(cudaGetLastError());
-    enqueue_momentum_krylov(capture, ustar, st);
+    enqueue_momentum_krylov(ustar, st);
   }
 
   // Batched momentum Krylov solve (x = 0, r = b in wb set up by k_momentum_rhs) into x; the
   // check kernel records failures and iteration counts in `s`.
-  void enqueue_momentum_krylov(bool capture, double *x, DevStatus *s_out) {
+  void enqueue_momentum_krylov(double *x, DevStatus *s_out) {
     if (momentum_mixed()) {
-      enqueue_momentum_mixed(capture, x, s_out);
+      enqueue_momentum_mixed(x, s_out);
       return;
     }
-    BicgArgs a = momentum_args(x, s_out);
-    const bool cg = (mom_krylov == CFSA_KRYLOV_CG);
+    const BicgArgs a = momentum_args(x, s_out);
     const unsigned int gp = blocks_for(N2);
-    if (cg) {
+    if (mom_krylov == CFSA_KRYLOV_CG) {
       k_mcg_init<3><<<strided(k_mcg_init<3>, gp), kBlock, 0, stream>>>(a);
       CK(cudaGetLastError());
+      CFSA_RESIDENT(k_mcg_solve, a, s2, stream);
+    } else {
+      CFSA_RESIDENT(k_bicg_solve3, a, s2, stream);
     }
-    auto body = [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) {
-      BicgArgs b = a;
-      b.cond = h;
-      b.use_cond = use;
-      if (cg) {
-        k_mcg_q<3><<<s2.nruns, kRunThreads, 0, s>>>(b);
-        k_mcg_xr<3><<<strided(k_mcg_xr<3>, gp), kBlock, 0, s>>>(b);
-        k_mcg_p<3><<<gp, kBlock, 0, s>>>(b);
-      } else {
-        bicg_body<3>(b, s, s2, (int)N2);
-      }
-    };
-    if (capture)
-      capture_while(body);
-    else
-      eager_while(body, [&] { return poll_bicg(bs_mom); }, maxit_mom);
-    k_check_bicg<<<1, 1, 0, stream>>>(bs_mom, 3, 0, s_out);
+    k_check_bicg<<<1, 1, 0, stream>>>(bs_mom, 3, 0, s_out, bar_err);
     CK(cudaGetLastError());
   }
 
@@ -1144,7 +1180,6 @@ struct cfsa_ns {
     a.invA32 = invA32;
     a.b = wb;
     a.x = x_out;
-    a.r64 = wr;
     a.xs = wv;
     a.r = fr;
     a.r0 = fr0;
@@ -1162,85 +1197,22 @@ struct cfsa_ns {
     return a;
   }
 
-  // FP32 BiCGSTAB with FP64 reliable updates (ns_mixed.cuh). Captured: a WHILE node whose body
-  // is one iteration followed by an IF node holding the reliable update; eager: the update
-  // kernels run after every iteration and return at once when no component asked for one.
-  void enqueue_momentum_mixed(bool capture, double *x, DevStatus *s_out) {
+  // FP32 CG or BiCGSTAB with FP64 reliable updates.
+  void enqueue_momentum_mixed(double *x, DevStatus *s_out) {
+    const MixedArgs a = mixed_args(x, s_out);
+    const unsigned int gp = blocks_for(N2);
+    const double delta = mixed_delta_of_method();
     if (mom_krylov == CFSA_KRYLOV_CG) {
-      enqueue_momentum_mixed_cg(capture, x, s_out);
-      return;
+      k_mpc_init<<<strided(k_mpc_init, gp), kBlock, 0, stream>>>(a, tol_mom, maxit_mom, delta);
+      CK(cudaGetLastError());
+      CFSA_RESIDENT(k_mpc_solve, a, s2, stream, 4);
+    } else {
+      k_mp_init<<<strided(k_mp_init, gp), kBlock, 0, stream>>>(a, tol_mom, maxit_mom, delta);
+      CK(cudaGetLastError());
+      CFSA_RESIDENT(k_mp_solve, a, s2, stream, 4);
     }
-    const MixedArgs a = mixed_args(x, s_out);
-    const unsigned int gp = blocks_for(N2);
-    k_mp_init<<<strided(k_mp_init, gp), kBlock, 0, stream>>>(a, tol_mom, maxit_mom, mixed_delta_of_method());
+    k_mp_check<<<1, 1, 0, stream>>>(ms, s_out, bar_err);
     CK(cudaGetLastError());
-    auto update_body = [&](cudaStream_t s, MixedArgs b) {
-      k_mp_xupdate<<<gp, kBlock, 0, s>>>(b);
-      k_mp_residual<<<s2.nruns, kRunThreads, 0, s>>>(b);
-    };
-    auto body = [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) {
-      MixedArgs b = a;
-      b.cond = h;
-      b.use_cond = use;
-      b.use_if = use;
-      if (b.use_if) b.cond_upd = new_cond_handle(s, 0);
-      k_mp_p<<<gp, kBlock, 0, s>>>(b);
-      k_mp_v<<<s2.nruns, kRunThreads, 0, s>>>(b);
-      k_mp_s<<<gp, kBlock, 0, s>>>(b);
-      k_mp_t<<<s2.nruns, kRunThreads, 0, s>>>(b);
-      k_mp_xr<<<strided(k_mp_xr, gp), kBlock, 0, s>>>(b);
-      if (b.use_if)
-        capture_cond_with(s, body_stream2, b.cond_upd, cudaGraphCondTypeIf,
-                          [&](cudaStream_t ss, cudaGraphConditionalHandle, int) { update_body(ss, b); });
-      else
-        update_body(s, b);
-    };
-    if (capture)
-      capture_while(body);
-    else
-      eager_while(body, [&] { return poll_mixed(); }, maxit_mom);
-    k_mp_check<<<1, 1, 0, stream>>>(ms, s_out);
-    CK(cudaGetLastError());
-  }
-
-  // FP32 CG with FP64 reliable updates (ns_mixed.cuh, k_mpc_*): per iteration the product, the
-  // x/r update and, after the reliable-update IF node, the direction update.
-  void enqueue_momentum_mixed_cg(bool capture, double *x, DevStatus *s_out) {
-    const MixedArgs a = mixed_args(x, s_out);
-    const unsigned int gp = blocks_for(N2);
-    k_mpc_init<<<strided(k_mpc_init, gp), kBlock, 0, stream>>>(a, tol_mom, maxit_mom, mixed_delta_of_method());
-    CK(cudaGetLastError());
-    auto update_body = [&](cudaStream_t s, MixedArgs b) {
-      k_mpc_xupdate<<<gp, kBlock, 0, s>>>(b);
-      k_mpc_residual<<<s2.nruns, kRunThreads, 0, s>>>(b);
-    };
-    auto body = [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) {
-      MixedArgs b = a;
-      b.cond = h;
-      b.use_cond = use;
-      b.use_if = use;
-      if (b.use_if) b.cond_upd = new_cond_handle(s, 0);
-      k_mpc_q<<<s2.nruns, kRunThreads, 0, s>>>(b);
-      k_mpc_xr<<<strided(k_mpc_xr, gp), kBlock, 0, s>>>(b);
-      if (b.use_if)
-        capture_cond_with(s, body_stream2, b.cond_upd, cudaGraphCondTypeIf,
-                          [&](cudaStream_t ss, cudaGraphConditionalHandle, int) { update_body(ss, b); });
-      else
-        update_body(s, b);
-      k_mpc_p<<<gp, kBlock, 0, s>>>(b);
-    };
-    if (capture)
-      capture_while(body);
-    else
-      eager_while(body, [&] { return poll_mixed(); }, maxit_mom);
-    k_mp_check<<<1, 1, 0, stream>>>(ms, s_out);
-    CK(cudaGetLastError());
-  }
-
-  bool poll_mixed() {
-    CK(cudaMemcpyAsync(h_ms, ms, sizeof(MixedState), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
-    return h_ms->active != 0;
   }
 
   void enqueue_pressure_solve(bool capture) {
@@ -1336,8 +1308,7 @@ struct cfsa_ns {
   // One cooperative launch of the two-level CG on `s` (barrier words and coarse accumulators
   // cleared first; the caller zeroes p and s[0] of the form it launches).
   void launch_cg2l(const Cg2lArgs &c2, bool f32, cudaStream_t s) {
-    CK(cudaMemsetAsync(bar_count, 0, sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(bar_err, 0, sizeof(int), s));
+    clear_barrier(s);
     if (coarse_view.nc > 0)
       CK(cudaMemsetAsync(coarse_view.gacc, 0, (size_t)27 * coarse_view.nc * sizeof(unsigned long long), s));
     cudaLaunchConfig_t cfg = {};
@@ -1435,17 +1406,8 @@ struct cfsa_ns {
       b.st = s_out;
       b.slot = 1;
       b.cw = (conv_norm == CFSA_NORM_JACOBI) ? invL : nullptr;
-      auto body = [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) {
-        BicgArgs c = b;
-        c.cond = h;
-        c.use_cond = use;
-        bicg_body<1>(c, s, s1, (int)nv);
-      };
-      if (capture)
-        capture_while(body);
-      else
-        eager_while(body, [&] { return poll_bicg(bs_p); }, maxit_p);
-      k_check_bicg<<<1, 1, 0, stream>>>(bs_p, 1, 1, s_out);
+      CFSA_RESIDENT(k_bicg_solve1, (PBicgArgs{b, pp2, pv2}), s1, stream);
+      k_check_bicg<<<1, 1, 0, stream>>>(bs_p, 1, 1, s_out, bar_err);
     } else if (cg_persistent || krylov == CFSA_KRYLOV_CG1 || krylov == CFSA_KRYLOV_CG2L) {
       CgPersistentArgs c{};
       c.S = s1.view();
@@ -1466,8 +1428,7 @@ struct cfsa_ns {
       c.st = s_out;
       c.bar = GridBarrier{bar_count, bar_err, bar_spin_limit};
       c.scaled = (conv_norm == CFSA_NORM_JACOBI) ? 1 : 0;
-      CK(cudaMemsetAsync(bar_count, 0, sizeof(unsigned int), stream));
-      CK(cudaMemsetAsync(bar_err, 0, sizeof(int), stream));
+      clear_barrier(stream);
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned int)cg_grid);
       cfg.blockDim = dim3(kBlock);
@@ -1600,14 +1561,8 @@ struct cfsa_ns {
     b.st = st;
     b.slot = 1;
     b.cw = nullptr;
-    auto body = [&](cudaStream_t s, cudaGraphConditionalHandle hc, int use) {
-      BicgArgs c = b;
-      c.cond = hc;
-      c.use_cond = use;
-      bicg_body<1>(c, s, s1, (int)nv);
-    };
-    eager_while(body, [&] { return poll_bicg(bs_p); }, maxit);
-    k_check_bicg<<<1, 1, 0, stream>>>(bs_p, 1, 1, st);
+    CFSA_RESIDENT(k_bicg_solve1, (PBicgArgs{b, pp2, pv2}), s1, stream);
+    k_check_bicg<<<1, 1, 0, stream>>>(bs_p, 1, 1, st, bar_err);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(x_host, d_x, (size_t)nv * sizeof(double), cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(h_st, st, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
@@ -1726,12 +1681,11 @@ struct cfsa_ns {
   bool pressure_mixed() const { return precision == CFSA_PRECISION_MIXED_FULL && krylov == CFSA_KRYLOV_CG2L; }
   int pressure_body_kernels() const {
     if (pressure_mixed()) return 4;  // prep, float two-level CG, x update, FP64 residual
-    if (krylov == CFSA_KRYLOV_BICGSTAB) return 5;
+    if (krylov == CFSA_KRYLOV_BICGSTAB) return 1;
     return (cg_persistent || krylov == CFSA_KRYLOV_CG1 || krylov == CFSA_KRYLOV_CG2L) ? 1 : 3;
   }
-  // Kernels of one momentum-solve body run (DevStatus::body_runs[0]): BiCGSTAB 5, CG 3.
+  // A momentum solve is one kernel (DevStatus::body_runs[0]).
   bool momentum_cg() const { return !momentum_mixed() && mom_krylov == CFSA_KRYLOV_CG; }
-  int momentum_body_kernels() const { return mom_krylov == CFSA_KRYLOV_CG ? 3 : 5; }
   int mixed_fixed_kernels() const {
     return (momentum_mixed() ? 1 : 0) + (pressure_mixed() ? 1 : 0) + (momentum_cg() ? 1 : 0);
   }
@@ -1746,9 +1700,7 @@ struct cfsa_ns {
     // reliable update (x update, residual) and an init kernel per solve, as has FP64 CG; mixed
     // two-level CG pressure: 4 kernels per sweep plus its init
     batch_launches = (int64_t)launched_steps * (launches_per_step + mixed_fixed_kernels()) +
-                     momentum_body_kernels() * (int64_t)h_st->body_runs[0] +
-                     pressure_body * (int64_t)h_st->body_runs[1] +
-                     2 * (int64_t)h_st->body_runs[2];
+                     (int64_t)h_st->body_runs[0] + pressure_body * (int64_t)h_st->body_runs[1];
     batch_iters[0] = (int64_t)h_st->iters[0];
     batch_iters[1] = (int64_t)h_st->iters[1];
     for (int64_t k = 0; k < h_st->steps_done; ++k) time += dt;
@@ -2122,7 +2074,7 @@ struct cfsa_ns {
     m.tpos = tpos1;
     k_momentum_rhs<<<strided(k_momentum_rhs, blocks_for(s2.nrows_pad)), kBlock, 0, stream>>>(m);
     CK(cudaGetLastError());
-    enqueue_momentum_krylov(capture, a_x, st_adj);
+    enqueue_momentum_krylov(a_x, st_adj);
     k_adj_conv_tet<<<blocks_for(nt), kBlock, 0, stream>>>((int)nt, N2, nv, tnode, grad, vol, a_x, a_un,
                                                           a_tsc, st_adj);
     AdjMomOutArgs o{};
@@ -2233,9 +2185,7 @@ struct cfsa_ns {
     adj_stats.backward_ms = ms;
     const int pressure_body = pressure_body_kernels();
     adj_stats.kernel_launches = (int64_t)adj_steps * adj_launches_fixed +
-                                momentum_body_kernels() * (int64_t)hs_adj.body_runs[0] +
-                                pressure_body * (int64_t)hs_adj.body_runs[1] +
-                                2 * (int64_t)hs_adj.body_runs[2];
+                                (int64_t)hs_adj.body_runs[0] + pressure_body * (int64_t)hs_adj.body_runs[1];
     if (h_st->code != CFSA_OK) {
       err = "forward recomputation failed with status " + std::to_string(h_st->code);
       return h_st->code;
@@ -2283,10 +2233,9 @@ struct cfsa_ns {
       a.p = fs;
       a.r0 = fs;
       a.v = ft;   // scratch output
-      auto *kern = (mom_krylov == CFSA_KRYLOV_CG) ? k_mpc_q : k_mp_v;  // the method's FP32 product
-      kern<<<s2.nruns, kRunThreads, 0, stream>>>(a);  // warm-up
+      CFSA_RESIDENT(k_mixed_product, (MixedProductArgs{a, 1}), s2, stream, 4);  // warm-up
       CK(cudaEventRecord(ev0, stream));
-      for (int k = 0; k < iters; ++k) kern<<<s2.nruns, kRunThreads, 0, stream>>>(a);
+      CFSA_RESIDENT(k_mixed_product, (MixedProductArgs{a, iters}), s2, stream, 4);
       CK(cudaEventRecord(ev1, stream));
       *alg_bytes = 8.0 * (double)nnz2 + 8.0 * s2.nrows_pad + 4.0 * (s2.nslices + 1) + 36.0 * (double)N2;
     } else if (which == CFSA_KERNEL_MOMENTUM_SPMV) {
@@ -2299,12 +2248,12 @@ struct cfsa_ns {
       a.bs = bs_prof;
       a.st = nullptr;
       a.v = ws;  // scratch output
-      // the product kernel of the selected momentum method (BiCGSTAB: v = At p with r0.v; CG:
-      // q = A p with p.q); same matrix stream, gathers and algorithmic bytes
-      auto *kern = (mom_krylov == CFSA_KRYLOV_CG) ? k_mcg_q<3> : k_bicg_v<3>;
-      kern<<<s2.nruns, kRunThreads, 0, stream>>>(a);  // warm-up
+      // the product phase of the momentum solve (BiCGSTAB: v = At p with r0.v; CG: q = A p with p.q);
+      // same matrix stream, gathers and algorithmic bytes
+      if (mom_krylov == CFSA_KRYLOV_CG) a.r0 = a.pk;
+      CFSA_RESIDENT(k_momentum_product, (MomentumProductArgs{a, 1}), s2, stream);  // warm-up
       CK(cudaEventRecord(ev0, stream));
-      for (int k = 0; k < iters; ++k) kern<<<s2.nruns, kRunThreads, 0, stream>>>(a);
+      CFSA_RESIDENT(k_momentum_product, (MomentumProductArgs{a, iters}), s2, stream);
       CK(cudaEventRecord(ev1, stream));
       *alg_bytes = 12.0 * (double)nnz2 + 8.0 * s2.nrows_pad + 4.0 * (s2.nslices + 1) + 72.0 * (double)N2;
     } else if (which == CFSA_KERNEL_PRESSURE_SPMV) {

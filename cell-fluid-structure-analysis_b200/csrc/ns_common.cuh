@@ -36,10 +36,10 @@ struct SellView {
   const int *len;   // [nrows_pad] row length
   const int *perm;  // [nrows_pad] original row, -1 for padding rows
   int nrows_pad;
-  // Slice runs of the run-walking product kernels: CTA c owns slices [rfirst[c], rfirst[c+1]),
-  // runs balanced by entries and split on 256-row block boundaries (multiples of 8 slices).
-  const int *rfirst;  // [nruns+1]
-  double *spart;      // [nslices * kMaxRed] warp sums of each slice (reduction scratch)
+  // Slice runs of the resident Krylov solves: CTA c takes the slices [rfirst[c], rfirst[c+1]) and
+  // [rfirst[G+1+c], rfirst[G+2+c]) of a grid of G CTAs; runs start on 256-row block boundaries
+  // (multiples of 8 slices) and are balanced by entries.
+  const int *rfirst;  // [2][G+1]
 };
 
 struct CsrView {
@@ -238,73 +238,15 @@ __device__ bool grid_reduce_strided(WarpSums<NV> &S, int nslots, unsigned int nb
   return true;
 }
 
-// Run-walking form for the SELL products of the Krylov loops: one CTA of kRunThreads per SM walks
-// a contiguous run of slices (SellView::rfirst), warp w taking slices s0 + w, s0 + w + 32, ...
-// Neighbouring rows gather from neighbouring parts of x, so the window of x that a CTA reads
-// slides through the SM's L1 instead of being spread over the whole vector (one CTA per 256-row
-// block puts blocks far apart in the row order on the same SM): 115 vs 137 us for the FP64
-// 3-right-hand-side momentum product at 1M tets.
-// Reduction: the warp that computes slice sl leaves its warp sums at spart[sl]; at the end each CTA
-// forms the partials of the 256-row blocks of its run (the 8 slice sums in slice order, which is
-// the warp order of grid_reduce) and the last CTA to take a ticket combines all block partials with
-// the tree of grid_reduce. Same tree, same bits as grid_reduce over one block per 256 rows.
-constexpr int kRunThreads = 1024;
-constexpr int kRunWarps = kRunThreads / 32;
-constexpr int kSlicesPerBlock = kBlock / kSellC;
-
-// Slice scheduling inside a run: warp w starts with slice s0 + w and then takes the next slice
-// nobody has claimed from a shared-memory counter. A static stride (w, w + 32, ...) gave a warp
-// the same position in every 256-row window (rows are sorted by length inside a window, so warps
-// 0, 8, 16, 24 always got the longest rows) and left the other warps waiting at the run's closing
-// barrier (ncu, 415k tets: 7.8 barrier stalls per issued instruction). Which warp computes a slice
-// does not matter for the results: each slice's sums go to its own slot of spart.
-__device__ __forceinline__ int run_first_slice(int *next, int s0) {
-  if (threadIdx.x == 0) *next = s0 + (int)(blockDim.x >> 5);
-  __syncthreads();
-  return s0 + (int)(threadIdx.x >> 5);
-}
+// The next slice nobody has claimed, from a shared-memory counter (slices differ in length; a static
+// stride gave a warp the same position in every length-sorted 256-row window). Which warp computes a
+// slice does not matter for the results.
 __device__ __forceinline__ int run_next_slice(int *next) {
   int v = 0;
   if ((threadIdx.x & 31) == 0) v = atomicAdd(next, 1);
   return __shfl_sync(0xffffffffu, v, 0);
 }
 
-template <int NV>
-__device__ __forceinline__ void slice_partial(const double (&v)[NV], const SellView &S, int sl) {
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    const double w = warp_sum(v[j]);
-    if ((threadIdx.x & 31) == 0) __stcg(&S.spart[(size_t)sl * kMaxRed + j], w);
-  }
-}
-
-template <int NV>
-__device__ bool grid_reduce_runs(const SellView &S, const Reduce &red, double (&out)[NV]) {
-  __shared__ bool last;
-  __syncthreads();  // every slice sum of this run is written
-  const int nsl = S.nrows_pad / kSellC;
-  const int s0 = S.rfirst[blockIdx.x], s1 = S.rfirst[blockIdx.x + 1];
-  const int b0 = s0 / kSlicesPerBlock, b1 = (s1 + kSlicesPerBlock - 1) / kSlicesPerBlock;
-  for (int t = threadIdx.x; t < (b1 - b0) * NV; t += blockDim.x) {
-    const int b = b0 + t / NV, j = t % NV;
-    double s = 0.0;
-    for (int w = 0; w < kSlicesPerBlock && kSlicesPerBlock * b + w < nsl; ++w)
-      s += __ldcg(&S.spart[(size_t)(kSlicesPerBlock * b + w) * kMaxRed + j]);
-    red.partials[(size_t)b * kMaxRed + j] = s;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> ctr(*red.counter);
-    const unsigned int ticket = ctr.fetch_add(1u, cuda::memory_order_acq_rel);
-    last = (ticket == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  combine_partials<NV>(red, (unsigned int)((nsl + kSlicesPerBlock - 1) / kSlicesPerBlock), out);
-  if (threadIdx.x == 0) *red.counter = 0u;
-  return true;
-}
+constexpr int kSlicesPerBlock = kBlock / kSellC;
 
 }  // namespace cfsa

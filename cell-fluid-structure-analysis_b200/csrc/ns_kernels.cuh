@@ -685,250 +685,11 @@ struct BicgArgs {
   int n;
   BicgState *bs;
   Reduce red;
-  cudaGraphConditionalHandle cond;
-  int use_cond;
   DevStatus *st;  // launch counters
   int slot;       // 0 momentum, 1 pressure
   const double *cw;  // convergence-norm weights, nullptr: unscaled ||r||
   double tol;        // relative tolerance (read by the momentum CG's initialisation)
 };
-
-// K1: p = r + beta (p - omega v); on restart: r = b - A x, r0 = r, p = r, rho = |r|^2.
-template <int NC>
-__global__ void k_bicg_p(BicgArgs A) {
-  const int active = A.bs->active;
-  if (!active) return;
-  const int restart = A.bs->restart;
-  // the scalars are read once, before any store the compiler could not prove disjoint from them
-  double beta_c[NC], omega_c[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) beta_c[c] = A.bs->beta[c], omega_c[c] = A.bs->omega[c];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (r < A.S.nrows_pad) ? A.S.perm[r] : -1;
-  const int64_t n = A.n;
-  double part[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) part[c] = 0.0;
-  if (i >= 0) {
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      if (!((active >> c) & 1)) continue;
-      const int64_t o = c * n + i;
-      if ((restart >> c) & 1) {
-        const int base = A.S.sptr[r >> 5] + (r & 31), len = A.S.len[r];
-        double acc = 0.0;
-        for (int k = 0; k < len; ++k) {
-          const int pos = base + k * kSellC;
-          const int j = A.S.col[pos];
-          acc += A.At[pos] * (A.diagA[j] * A.x[c * n + j]);
-        }
-        const double ri = A.b[o] - acc;
-        A.r[o] = ri;
-        A.r0[o] = ri;
-        A.pk[o] = ri;
-        part[c] = ri * ri;
-      } else {
-        A.pk[o] = A.r[o] + beta_c[c] * (A.pk[o] - omega_c[c] * A.v[o]);
-      }
-    }
-  }
-  if (restart) {
-    double tot[NC];
-    if (grid_reduce<NC>(part, A.red, tot) && threadIdx.x == 0) {
-      for (int c = 0; c < NC; ++c)
-        if ((restart >> c) & 1) {
-          A.bs->rho[c] = tot[c];
-          A.bs->r0norm2[c] = tot[c];
-        }
-      A.bs->restart = 0;
-    }
-  }
-}
-
-// K2: v = At p, alpha = rho / (r0 . v)
-template <int NC>
-__global__ void __launch_bounds__(kRunThreads, 1) k_bicg_v(BicgArgs A) {
-  const int active = A.bs->active;
-  if (!active) return;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<NC>(active, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) part[c] = 0.0;
-      if (i >= 0) {
-        double acc[NC];
-        sell_spmv_row<NC, kU64, MASK>(A.S, A.At, A.pk, n, r, acc);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.v[o] = acc[c];
-          part[c] = A.r0[o] * acc[c];
-        }
-      }
-      slice_partial<NC>(part, A.S, sl);
-    }
-  });
-  double tot[NC];
-  if (grid_reduce_runs<NC>(A.S, A.red, tot) && threadIdx.x == 0) {
-    for (int c = 0; c < NC; ++c) {
-      if (!((active >> c) & 1)) continue;
-      if (tot[c] == 0.0) {
-        A.bs->status[c] = KS_BREAKDOWN;
-        A.bs->active &= ~(1 << c);
-      } else {
-        A.bs->alpha[c] = A.bs->rho[c] / tot[c];
-      }
-    }
-  }
-}
-
-// K3: s = r - alpha v
-template <int NC>
-__global__ void k_bicg_s(BicgArgs A) {
-  const int active = A.bs->active;
-  if (!active) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const int64_t n = A.n;
-  double alpha[NC], rv[NC], vv[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    alpha[c] = A.bs->alpha[c];
-    if ((active >> c) & 1) rv[c] = A.r[c * n + i], vv[c] = A.v[c * n + i];
-  }
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-    if ((active >> c) & 1) A.s[c * n + i] = rv[c] - alpha[c] * vv[c];
-}
-
-// K4: t = At s, omega = (t . s) / (t . t) (0 when t . t == 0)
-template <int NC>
-__global__ void __launch_bounds__(kRunThreads, 1) k_bicg_t(BicgArgs A) {
-  const int active = A.bs->active;
-  if (!active) return;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<NC>(active, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[2 * NC];
-#pragma unroll
-      for (int c = 0; c < 2 * NC; ++c) part[c] = 0.0;
-      if (i >= 0) {
-        double acc[NC];
-        sell_spmv_row<NC, kU64, MASK>(A.S, A.At, A.s, n, r, acc);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.t[o] = acc[c];
-          part[c] = acc[c] * acc[c];
-          part[NC + c] = acc[c] * A.s[o];
-        }
-      }
-      slice_partial<2 * NC>(part, A.S, sl);
-    }
-  });
-  double tot[2 * NC];
-  if (grid_reduce_runs<2 * NC>(A.S, A.red, tot) && threadIdx.x == 0) {
-    for (int c = 0; c < NC; ++c) {
-      if (!((active >> c) & 1)) continue;
-      A.bs->omega[c] = (tot[c] > 0.0) ? tot[NC + c] / tot[c] : 0.0;
-    }
-  }
-}
-
-// K5: x += alpha D^-1 p + omega D^-1 s, r = s - omega t; convergence test and next beta.
-template <int NC>
-__global__ void k_bicg_xr(BicgArgs A) {
-  const int active = A.bs->active;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[A.slot] += 1;
-  if (!active) {
-    if (A.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(A.cond, 0);
-    return;
-  }
-  __shared__ WarpSums<2 * NC> S;
-  const int nblk = (A.n + kBlock - 1) / kBlock;
-  const int64_t n = A.n;
-  double alpha_c[NC], omega_c[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) alpha_c[c] = A.bs->alpha[c], omega_c[c] = A.bs->omega[c];
-  int slot = 0;
-  for (int b = blockIdx.x; b < nblk; b += gridDim.x, ++slot) {
-    const int i = b * kBlock + threadIdx.x;
-    double part[2 * NC];
-#pragma unroll
-    for (int c = 0; c < 2 * NC; ++c) part[c] = 0.0;
-    if (i < A.n) {
-      const double dinv = A.invA[i];
-      const double w = A.cw ? A.cw[i] : 1.0;
-      double pv[NC], sv[NC], tv[NC], xv[NC], r0v[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (!((active >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        pv[c] = A.pk[o], sv[c] = A.s[o], tv[c] = A.t[o], xv[c] = A.x[o], r0v[c] = A.r0[o];
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (!((active >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        const double y = dinv * pv[c];
-        const double z = dinv * sv[c];
-        A.x[o] = xv[c] + (alpha_c[c] * y + omega_c[c] * z);
-        const double ri = sv[c] - omega_c[c] * tv[c];
-        A.r[o] = ri;
-        part[c] = (ri * ri) * w;
-        part[NC + c] = r0v[c] * ri;
-      }
-    }
-    warp_partial<2 * NC>(part, S, slot);
-  }
-  double tot[2 * NC];
-  if (grid_reduce_strided<2 * NC>(S, slot, nblk, A.red, tot) && threadIdx.x == 0) {
-    BicgState *s = A.bs;
-    const double eps = 2.220446049250313e-16;
-    for (int c = 0; c < NC; ++c) {
-      if (!((active >> c) & 1)) continue;
-      s->iters[c] += 1;
-      s->rnorm2[c] = tot[c];
-      if (isnan(tot[c]) || isnan(tot[NC + c])) {
-        s->status[c] = KS_BREAKDOWN;
-        s->active &= ~(1 << c);
-      } else if (tot[c] <= s->tol2[c]) {
-        s->status[c] = KS_CONVERGED;
-        s->active &= ~(1 << c);
-      } else if (s->iters[c] >= s->maxit) {
-        s->status[c] = KS_MAXIT;
-        s->active &= ~(1 << c);
-      } else if (s->omega[c] == 0.0) {
-        s->status[c] = KS_BREAKDOWN;
-        s->active &= ~(1 << c);
-      } else {
-        const double rho_new = tot[NC + c];
-        if (fabs(rho_new) < eps * eps * s->r0norm2[c]) {
-          s->restart |= 1 << c;
-        } else {
-          s->beta[c] = (rho_new / s->rho[c]) * (s->alpha[c] / s->omega[c]);
-          s->rho[c] = rho_new;
-        }
-      }
-    }
-    if (A.use_cond) cudaGraphSetConditional(A.cond, s->active ? 1u : 0u);
-  }
-}
 
 // ------------------------------------------------------------------------------------------
 // Batched Jacobi-preconditioned CG for the momentum system (selectable; the reference solves it
@@ -997,147 +758,12 @@ __global__ void k_mcg_init(BicgArgs A) {
   }
 }
 
-// G1: q = A p (into v), alpha = absnew / (p . q)
-template <int NC>
-__global__ void __launch_bounds__(kRunThreads, 1) k_mcg_q(BicgArgs A) {
-  const int active = A.bs->active;
-  if (!active) return;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<NC>(active, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) part[c] = 0.0;
-      if (i >= 0) {
-        double acc[NC];
-        sell_spmv_row<NC, kU64, MASK>(A.S, A.At, A.pk, n, r, acc);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.v[o] = acc[c];
-          part[c] = A.pk[o] * acc[c];
-        }
-      }
-      slice_partial<NC>(part, A.S, sl);
-    }
-  });
-  double tot[NC];
-  if (grid_reduce_runs<NC>(A.S, A.red, tot) && threadIdx.x == 0) {
-    for (int c = 0; c < NC; ++c) {
-      if (!((active >> c) & 1)) continue;
-      if (tot[c] == 0.0) {
-        A.bs->status[c] = KS_BREAKDOWN;
-        A.bs->active &= ~(1 << c);
-      } else {
-        A.bs->alpha[c] = A.bs->rho[c] / tot[c];
-      }
-    }
-  }
-}
-
-// G2: x += alpha p, r -= alpha q, z = D^-1 r; r.r and r.z; convergence test and next beta.
-template <int NC>
-__global__ void k_mcg_xr(BicgArgs A) {
-  const int active = A.bs->active;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[A.slot] += 1;
-  if (!active) {
-    if (A.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(A.cond, 0);
-    return;
-  }
-  __shared__ WarpSums<2 * NC> S;
-  const int nblk = (A.n + kBlock - 1) / kBlock;
-  const int64_t n = A.n;
-  double alpha_c[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) alpha_c[c] = A.bs->alpha[c];
-  int slot = 0;
-  for (int b = blockIdx.x; b < nblk; b += gridDim.x, ++slot) {
-    const int i = b * kBlock + threadIdx.x;
-    double part[2 * NC];
-#pragma unroll
-    for (int c = 0; c < 2 * NC; ++c) part[c] = 0.0;
-    if (i < A.n) {
-      const double dinv = A.invA[i];
-      double xv[NC], pv[NC], rv[NC], qv[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (!((active >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        xv[c] = A.x[o], pv[c] = A.pk[o], rv[c] = A.r[o], qv[c] = A.v[o];
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (!((active >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        A.x[o] = xv[c] + alpha_c[c] * pv[c];
-        const double ri = rv[c] - alpha_c[c] * qv[c];
-        A.r[o] = ri;
-        const double zi = dinv * ri;
-        part[c] = ri * ri;
-        part[NC + c] = ri * zi;
-      }
-    }
-    warp_partial<2 * NC>(part, S, slot);
-  }
-  double tot[2 * NC];
-  if (grid_reduce_strided<2 * NC>(S, slot, nblk, A.red, tot) && threadIdx.x == 0) {
-    BicgState *s = A.bs;
-    for (int c = 0; c < NC; ++c) {
-      if (!((active >> c) & 1)) continue;
-      s->iters[c] += 1;
-      const double rr = tot[c], rz = tot[NC + c];
-      const double crit = A.cw ? rz : rr;
-      s->rnorm2[c] = crit;
-      if (isnan(rr) || isnan(rz)) {
-        s->status[c] = KS_BREAKDOWN;
-        s->active &= ~(1 << c);
-      } else if (crit <= s->tol2[c]) {
-        s->status[c] = KS_CONVERGED;
-        s->active &= ~(1 << c);
-      } else if (s->iters[c] >= s->maxit) {
-        s->status[c] = KS_MAXIT;
-        s->active &= ~(1 << c);
-      } else {
-        s->beta[c] = rz / s->rho[c];
-        s->rho[c] = rz;
-      }
-    }
-    if (A.use_cond) cudaGraphSetConditional(A.cond, s->active ? 1u : 0u);
-  }
-}
-
-// G3: p = z + beta p with z = D^-1 r
-template <int NC>
-__global__ void k_mcg_p(BicgArgs A) {
-  const int active = A.bs->active;
-  if (!active) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const int64_t n = A.n;
-  const double dinv = A.invA[i];
-  double beta[NC], rv[NC], pv[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    beta[c] = A.bs->beta[c];
-    if ((active >> c) & 1) rv[c] = A.r[c * n + i], pv[c] = A.pk[c * n + i];
-  }
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-    if ((active >> c) & 1) A.pk[c * n + i] = dinv * rv[c] + beta[c] * pv[c];
-}
-
 // After a Krylov loop: record a failure and halt the rest of the batch (pisoStep returns false
 // right after a failed solve, NavierStokes.cpp:387-398).
-__global__ void k_check_bicg(const BicgState *__restrict__ bs, int ncomp, int slot, DevStatus *st) {
+__global__ void k_check_bicg(const BicgState *__restrict__ bs, int ncomp, int slot, DevStatus *st,
+                             const int *__restrict__ barrier_err) {
   if (st->halt) return;
-  int code = 0, it = 0;
+  int code = *barrier_err ? 4 : 0, it = 0;  // 4: the solve gave up waiting at a grid barrier
   for (int c = 0; c < ncomp; ++c) it = max(it, bs->iters[c]);
   st->iters[slot] += (unsigned long long)it;
   for (int c = 0; c < ncomp; ++c) {
@@ -1363,9 +989,9 @@ __global__ void k_cg_p(CgArgs A) {
 // all CTAs take the same decisions and the iterates equal those of k_cg_q / k_cg_xr / k_cg_p bit
 // for bit. Data written by other CTAs inside the launch is read with L1-bypassing loads.
 // Barriers spin with a bound; on expiry the kernel records an error and every CTA returns (those
-// that had passed, at their next barrier). The bound is a launch argument (default kBarrierSpinLimit polls, over a second), so that a
+// that had passed, at their next barrier). The bound is a launch argument (default kBarrierSpinLimit polls of about 0.6 us, over two seconds), so that a
 // test can make a wait run out on purpose and check that the step reports it.
-constexpr long long kBarrierSpinLimit = 1LL << 25;
+constexpr long long kBarrierSpinLimit = 1LL << 22;
 
 struct GridBarrier {
   unsigned int *count;  // arrivals since the launch began (zeroed before each launch)
@@ -1384,6 +1010,7 @@ __device__ __forceinline__ bool grid_sync(const GridBarrier &B, unsigned int &ph
   __shared__ int s_ok;
   ++phase;
   __syncthreads();
+  if (gridDim.x == 1 && B.spin_limit > 0) return true;
   if (threadIdx.x == 0) {
     cuda::atomic_ref<unsigned int, cuda::thread_scope_device> count(*B.count);
     const unsigned int target = phase * gridDim.x;

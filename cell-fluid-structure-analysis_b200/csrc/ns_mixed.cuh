@@ -48,72 +48,15 @@ struct MixedArgs {
   const double *At64, *diagA, *invA;
   const float *invA32;
   const double *b;
-  double *x, *r64, *xs;  // FP64 solution, true residual, scaled solution D x
+  double *x, *xs;  // FP64 solution, scaled solution D x
   float *r, *r0, *p, *v, *s, *t, *dx;
   int n;
   MixedState *ms;
   DevStatus *st;
   Reduce red;
-  cudaGraphConditionalHandle cond;      // WHILE node of the iteration
-  cudaGraphConditionalHandle cond_upd;  // IF node of the reliable update
-  int use_cond;
-  int use_if;  // cond_upd is a live IF node (otherwise the update kernels run every iteration)
   const double *cw;   // convergence-norm weights (diag(A)^-1), nullptr: unscaled ||r||
   const float *cw32;  // the same for the FP32 residual
 };
-
-template <int U = 8, int MASK = 7>
-__device__ __forceinline__ void sell_spmv_row_f32x3(const SellView &S, const float *__restrict__ val,
-                                                    const float *__restrict__ x, int64_t n, int r,
-                                                    float acc[3]) {
-  const int base = S.sptr[r >> 5] + (r & 31), len = S.len[r];
-  acc[0] = acc[1] = acc[2] = 0.f;
-  int k = 0;
-  for (; k + U <= len; k += U) {
-    int j[U];
-    float a[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int pos = base + (k + u) * kSellC;
-      j[u] = __ldcs(S.col + pos);
-      a[u] = __ldcs(val + pos);
-    }
-    float xv[U][3];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((MASK >> c) & 1) xv[u][c] = __ldg(x + c * n + j[u]);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((MASK >> c) & 1) acc[c] += a[u] * xv[u][c];
-  }
-  if (k < len) {  // the last len % U entries as one predicated chunk: one memory round trip
-    int j[U];
-    float a[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int pos = base + (k + u) * kSellC;
-      const bool in = k + u < len;
-      j[u] = in ? __ldcs(S.col + pos) : 0;
-      a[u] = in ? __ldcs(val + pos) : 0.f;
-    }
-    float xv[U][3];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((MASK >> c) & 1) xv[u][c] = (k + u < len) ? __ldg(x + c * n + j[u]) : 0.f;
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if (((MASK >> c) & 1) && k + u < len) acc[c] += a[u] * xv[u][c];
-  }
-}
-
 
 // Init (after k_momentum_rhs wrote b and x = 0): r = r0 = (float) b, p = v = dx = 0;
 // FP64 ||b|| in the convergence norm, rho = r0 . r.
@@ -179,344 +122,9 @@ __global__ void k_mp_init(MixedArgs A, double tol, int maxit, double delta) {
   }
 }
 
-// K1: p = r + beta (p - omega v)  (beta = 0 after a restart: p = r). Components whose FP32
-// recurrence drifted from the true residual (flagged by the last update) restart here instead:
-// r0 = p = r and rho = r0 . r, the one reduction of this kernel (taken only when a restart is due).
-__global__ void k_mp_p(MixedArgs A) {
-  const int act = A.ms->active;
-  if (!act) return;
-  const int rs = A.ms->restart_next & act;
-  float beta[3], omega[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) beta[c] = (float)A.ms->beta[c], omega[c] = (float)A.ms->omega[c];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n = A.n;
-  double part[3] = {0.0, 0.0, 0.0};
-  if (i < A.n) {
-    float rv[3], pv[3], vv[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      if ((act >> c) & 1) rv[c] = A.r[c * n + i], pv[c] = A.p[c * n + i], vv[c] = A.v[c * n + i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (!((act >> c) & 1)) continue;
-      const int64_t o = c * n + i;
-      if ((rs >> c) & 1) {
-        A.p[o] = rv[c];
-        A.r0[o] = rv[c];
-        part[c] = (double)rv[c] * (double)rv[c];
-      } else {
-        A.p[o] = rv[c] + beta[c] * (pv[c] - omega[c] * vv[c]);
-      }
-    }
-  }
-  if (!rs) return;
-  double tot[3];
-  if (grid_reduce<3>(part, A.red, tot) && threadIdx.x == 0) {
-    MixedState *m = A.ms;
-    for (int c = 0; c < 3; ++c)
-      if ((rs >> c) & 1) {
-        m->rho[c] = tot[c];
-        m->r0norm2[c] = tot[c];
-        m->restarts[c] += 1;
-      }
-    m->restart_next = 0;
-  }
-}
-
-// K2: v = At32 p, alpha = rho / (r0 . v)
-__global__ void __launch_bounds__(kRunThreads, 1) k_mp_v(MixedArgs A) {
-  const int act = A.ms->active;
-  if (!act) return;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<3>(act, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[3] = {0.0, 0.0, 0.0};
-      if (i >= 0) {
-        float acc[3];
-        sell_spmv_row_f32x3<8, MASK>(A.S, A.At32, A.p, n, r, acc);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          A.v[c * n + i] = acc[c];
-          part[c] = (double)A.r0[c * n + i] * (double)acc[c];
-        }
-      }
-      slice_partial<3>(part, A.S, sl);
-    }
-  });
-  double tot[3];
-  if (grid_reduce_runs<3>(A.S, A.red, tot) && threadIdx.x == 0) {
-    for (int c = 0; c < 3; ++c) {
-      if (!((act >> c) & 1)) continue;
-      if (isnan(tot[c])) {
-        A.ms->status[c] = KS_BREAKDOWN;
-        A.ms->active &= ~(1 << c);
-      } else if (tot[c] == 0.0) {
-        // r0 . v vanished: no step along p; the iteration ends in an update and a restart
-        A.ms->alpha[c] = 0.0;
-        A.ms->force |= 1 << c;
-      } else {
-        A.ms->alpha[c] = A.ms->rho[c] / tot[c];
-      }
-    }
-  }
-}
-
-// K3: s = r - alpha v
-__global__ void k_mp_s(MixedArgs A) {
-  const int act = A.ms->active;
-  if (!act) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const int64_t n = A.n;
-  float alpha[3], rv[3], vv[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    alpha[c] = (float)A.ms->alpha[c];
-    if ((act >> c) & 1) rv[c] = A.r[c * n + i], vv[c] = A.v[c * n + i];
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-    if ((act >> c) & 1) A.s[c * n + i] = rv[c] - alpha[c] * vv[c];
-}
-
-// K4: t = At32 s, omega = (t . s) / (t . t)
-__global__ void __launch_bounds__(kRunThreads, 1) k_mp_t(MixedArgs A) {
-  const int act = A.ms->active;
-  if (!act) return;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<3>(act, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      if (i >= 0) {
-        float acc[3];
-        sell_spmv_row_f32x3<8, MASK>(A.S, A.At32, A.s, n, r, acc);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          A.t[c * n + i] = acc[c];
-          part[c] = (double)acc[c] * (double)acc[c];
-          part[3 + c] = (double)acc[c] * (double)A.s[c * n + i];
-        }
-      }
-      slice_partial<6>(part, A.S, sl);
-    }
-  });
-  double tot[6];
-  if (grid_reduce_runs<6>(A.S, A.red, tot) && threadIdx.x == 0) {
-    for (int c = 0; c < 3; ++c) {
-      if (!((act >> c) & 1)) continue;
-      A.ms->omega[c] = (tot[c] > 0.0) ? tot[3 + c] / tot[c] : 0.0;
-    }
-  }
-}
-
-// K5: dx += alpha D^-1 p + omega D^-1 s, r = s - omega t; ||r||, r0 . r; which components take a
-// reliable update at the end of this iteration (IF node), next beta for the others.
-__global__ void k_mp_xr(MixedArgs A) {
-  const int act = A.ms->active;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[0] += 1;
-  if (!act) {
-    if (A.use_cond && blockIdx.x == 0 && threadIdx.x == 0) {
-      if (A.use_if) cudaGraphSetConditional(A.cond_upd, 0);
-      cudaGraphSetConditional(A.cond, 0);
-    }
-    return;
-  }
-  const int64_t n = A.n;
-  __shared__ WarpSums<6> S;
-  const int nblk = (A.n + kBlock - 1) / kBlock;
-  float alpha_c[3], omega_c[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) alpha_c[c] = (float)A.ms->alpha[c], omega_c[c] = (float)A.ms->omega[c];
-  int slot = 0;
-  for (int bk = blockIdx.x; bk < nblk; bk += gridDim.x, ++slot) {
-    const int i = bk * kBlock + threadIdx.x;
-    double part[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (i < A.n) {
-      const float dinv = A.invA32[i];
-      const double w = A.cw32 ? (double)A.cw32[i] : 1.0;
-      float pv[3], sv[3], tv[3], dxv[3], r0v[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (!((act >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        pv[c] = A.p[o], sv[c] = A.s[o], tv[c] = A.t[o], dxv[c] = A.dx[o], r0v[c] = A.r0[o];
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (!((act >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        A.dx[o] = dxv[c] + (alpha_c[c] * (dinv * pv[c]) + omega_c[c] * (dinv * sv[c]));
-        const float ri = sv[c] - omega_c[c] * tv[c];
-        A.r[o] = ri;
-        part[c] = ((double)ri * (double)ri) * w;
-        part[3 + c] = (double)r0v[c] * (double)ri;
-      }
-    }
-    warp_partial<6>(part, S, slot);
-  }
-  double tot[6];
-  if (grid_reduce_strided<6>(S, slot, nblk, A.red, tot) && threadIdx.x == 0) {
-    MixedState *m = A.ms;
-    const double eps = 2.220446049250313e-16;
-    int upd = 0, rst = 0, live = 0;
-    for (int c = 0; c < 3; ++c) {
-      if (!((act >> c) & 1)) continue;
-      m->iters[c] += 1;
-      m->rin2[c] = tot[c];
-      const double rho_new = tot[3 + c];
-      if (isnan(tot[c]) || isnan(rho_new)) {
-        m->status[c] = KS_BREAKDOWN;
-        m->active &= ~(1 << c);
-        continue;
-      }
-      live |= 1 << c;
-      // near-breakdown, a vanished omega or r0 . v: the FP32 space is exhausted; the update
-      // replaces the residual and the Krylov space restarts from it
-      const bool restart = fabs(rho_new) < eps * eps * m->r0norm2[c] || m->omega[c] == 0.0 ||
-                           ((m->force >> c) & 1);
-      if (tot[c] <= m->tol2[c] || m->iters[c] >= m->maxit || tot[c] < m->delta2 * m->rmax2[c] || restart) {
-        upd |= 1 << c;
-        if (restart) rst |= 1 << c;
-      }
-    }
-    // Components update on their own triggers only: replacing a residual before it has dropped by
-    // delta perturbs BiCGSTAB's recurrences, and on the 4M-tet Y-bifurcation updates brought
-    // forward to share one FP64 product made the iteration erratic until it hit the cap.
-    for (int c = 0; c < 3; ++c) {
-      if (!(((live & ~upd) >> c) & 1)) continue;
-      const double rho_new = tot[3 + c];
-      m->beta[c] = (rho_new / m->rho[c]) * (m->alpha[c] / m->omega[c]);
-      m->rho[c] = rho_new;
-      m->rmax2[c] = fmax(m->rmax2[c], tot[c]);
-    }
-    m->upd = upd;
-    m->restart = rst;
-    m->force = 0;
-    if (A.use_cond) {
-      if (A.use_if) cudaGraphSetConditional(A.cond_upd, upd ? 1u : 0u);
-      cudaGraphSetConditional(A.cond, m->active ? 1u : 0u);
-    }
-  }
-}
-
-// Reliable update, part 1: x += dx (FP64), dx = 0, xs = diag(A) x for the updated components.
-__global__ void k_mp_xupdate(MixedArgs A) {
-  const int upd = A.ms->upd;
-  if (!upd) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const int64_t n = A.n;
-  const double d = A.diagA[i];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (!((upd >> c) & 1)) continue;
-    const int64_t o = c * n + i;
-    const double xi = A.x[o] + (double)A.dx[o];
-    A.x[o] = xi;
-    A.dx[o] = 0.f;
-    A.xs[o] = d * xi;
-  }
-}
-
-// Reliable update, part 2: r64 = b - At64 (D x) (FP64 true residual), r = (float) r64 (and r0 = r
-// for a restart); convergence on the true residual, next beta from the replaced residual.
-__global__ void __launch_bounds__(kRunThreads, 1) k_mp_residual(MixedArgs A) {
-  const int upd = A.ms->upd;
-  if (!upd) return;
-  const int rst = A.ms->restart;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[2] += 1;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<3>(upd, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      if (i >= 0) {
-        double acc[3];
-        sell_spmv_row<3, kU64, MASK>(A.S, A.At64, A.xs, n, r, acc);
-        const double w = A.cw ? A.cw[i] : 1.0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          const double ri = A.b[o] - acc[c];
-          A.r64[o] = ri;
-          const float rf = (float)ri;
-          A.r[o] = rf;
-          float r0 = A.r0[o];
-          if ((rst >> c) & 1) {
-            r0 = rf;
-            A.r0[o] = rf;
-          }
-          part[c] = (ri * ri) * w;
-          part[3 + c] = (double)r0 * (double)rf;
-        }
-      }
-      slice_partial<6>(part, A.S, sl);
-    }
-  });
-  double tot[6];
-  if (grid_reduce_runs<6>(A.S, A.red, tot) && threadIdx.x == 0) {
-    MixedState *m = A.ms;
-    for (int c = 0; c < 3; ++c) {
-      if (!((upd >> c) & 1)) continue;
-      m->updates[c] += 1;
-      const double prev2 = m->rnorm2[c];  // true residual at the previous update
-      m->rnorm2[c] = tot[c];
-      const double rho_new = tot[3 + c];
-      if (isnan(tot[c]) || isnan(rho_new)) {
-        m->status[c] = KS_BREAKDOWN;
-        m->active &= ~(1 << c);
-      } else if (tot[c] <= m->tol2[c]) {
-        m->status[c] = KS_CONVERGED;
-        m->active &= ~(1 << c);
-      } else if (m->iters[c] >= m->maxit) {
-        m->status[c] = KS_MAXIT;
-        m->active &= ~(1 << c);
-      } else {
-        if ((rst >> c) & 1) {
-          m->r0norm2[c] = rho_new;
-          m->beta[c] = 0.0;
-        } else {
-          m->beta[c] = (rho_new / m->rho[c]) * (m->alpha[c] / m->omega[c]);
-          // the true residual is more than 10x (in norm) the FP32 recurrence's (its Krylov space
-          // has drifted), or it grew since the previous update (erratic convergence): the next
-          // iteration restarts the space from the replaced residual
-          if (tot[c] > kMixedDrift2 * m->rin2[c] || tot[c] > prev2) m->restart_next |= 1 << c;
-        }
-        m->rho[c] = rho_new;
-        m->rin2[c] = tot[c];
-        m->rmax2[c] = tot[c];
-      }
-    }
-    m->upd = 0;
-    m->restart = 0;
-    if (A.use_cond) cudaGraphSetConditional(A.cond, m->active ? 1u : 0u);
-  }
-}
-
-__global__ void k_mp_check(const MixedState *__restrict__ m, DevStatus *st) {
+__global__ void k_mp_check(const MixedState *__restrict__ m, DevStatus *st, const int *__restrict__ barrier_err) {
   if (st->halt) return;
-  int code = 0, it = 0;
+  int code = *barrier_err ? 4 : 0, it = 0;  // 4: the solve gave up waiting at a grid barrier
   for (int c = 0; c < 3; ++c) {
     it = max(it, m->iters[c]);
     if (m->status[c] == KS_MAXIT && code == 0) code = 1;
@@ -605,229 +213,6 @@ __global__ void k_mpc_init(MixedArgs A, double tol, int maxit, double delta) {
       }
     }
   }
-}
-
-// C1: q = A32 p (into v), alpha = rho / (p . q)
-__global__ void __launch_bounds__(kRunThreads, 1) k_mpc_q(MixedArgs A) {
-  const int act = A.ms->active;
-  if (!act) return;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<3>(act, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[3] = {0.0, 0.0, 0.0};
-      if (i >= 0) {
-        float acc[3];
-        sell_spmv_row_f32x3<8, MASK>(A.S, A.At32, A.p, n, r, acc);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          A.v[c * n + i] = acc[c];
-          part[c] = (double)A.p[c * n + i] * (double)acc[c];
-        }
-      }
-      slice_partial<3>(part, A.S, sl);
-    }
-  });
-  double tot[3];
-  if (grid_reduce_runs<3>(A.S, A.red, tot) && threadIdx.x == 0) {
-    for (int c = 0; c < 3; ++c) {
-      if (!((act >> c) & 1)) continue;
-      if (isnan(tot[c]) || tot[c] == 0.0) {
-        A.ms->status[c] = KS_BREAKDOWN;
-        A.ms->active &= ~(1 << c);
-      } else {
-        A.ms->alpha[c] = A.ms->rho[c] / tot[c];
-      }
-    }
-  }
-}
-
-// C2: dx += alpha p, r -= alpha q, z = D^-1 r; the iterated residual (convergence norm) and r.z;
-// which components take a reliable update at the end of this iteration (IF node); next beta for
-// the others.
-__global__ void k_mpc_xr(MixedArgs A) {
-  const int act = A.ms->active;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[0] += 1;
-  if (!act) {
-    if (A.use_cond && blockIdx.x == 0 && threadIdx.x == 0) {
-      if (A.use_if) cudaGraphSetConditional(A.cond_upd, 0);
-      cudaGraphSetConditional(A.cond, 0);
-    }
-    return;
-  }
-  const int64_t n = A.n;
-  __shared__ WarpSums<6> S;
-  const int nblk = (A.n + kBlock - 1) / kBlock;
-  float alpha_c[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) alpha_c[c] = (float)A.ms->alpha[c];
-  int slot = 0;
-  for (int bk = blockIdx.x; bk < nblk; bk += gridDim.x, ++slot) {
-    const int i = bk * kBlock + threadIdx.x;
-    double part[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (i < A.n) {
-      const float dinv = A.invA32[i];
-      const double w = A.cw32 ? (double)A.cw32[i] : 1.0;
-      float pv[3], qv[3], rv[3], dxv[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (!((act >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        pv[c] = A.p[o], qv[c] = A.v[o], rv[c] = A.r[o], dxv[c] = A.dx[o];
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (!((act >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        A.dx[o] = dxv[c] + alpha_c[c] * pv[c];
-        const float ri = rv[c] - alpha_c[c] * qv[c];
-        A.r[o] = ri;
-        const float zi = dinv * ri;
-        part[c] = ((double)ri * (double)ri) * w;
-        part[3 + c] = (double)ri * (double)zi;
-      }
-    }
-    warp_partial<6>(part, S, slot);
-  }
-  double tot[6];
-  if (grid_reduce_strided<6>(S, slot, nblk, A.red, tot) && threadIdx.x == 0) {
-    MixedState *m = A.ms;
-    int upd = 0;
-    for (int c = 0; c < 3; ++c) {
-      if (!((act >> c) & 1)) continue;
-      m->iters[c] += 1;
-      m->rin2[c] = tot[c];
-      if (isnan(tot[c]) || isnan(tot[3 + c])) {
-        m->status[c] = KS_BREAKDOWN;
-        m->active &= ~(1 << c);
-        continue;
-      }
-      if (tot[c] <= m->tol2[c] || m->iters[c] >= m->maxit || tot[c] < m->delta2 * m->rmax2[c]) {
-        upd |= 1 << c;  // the update replaces rho and beta from the true residual
-      } else {
-        m->beta[c] = tot[3 + c] / m->rho[c];
-        m->rho[c] = tot[3 + c];
-        m->rmax2[c] = fmax(m->rmax2[c], tot[c]);
-      }
-    }
-    m->upd = upd;
-    if (A.use_cond) {
-      if (A.use_if) cudaGraphSetConditional(A.cond_upd, upd ? 1u : 0u);
-      cudaGraphSetConditional(A.cond, m->active ? 1u : 0u);
-    }
-  }
-}
-
-// Reliable update, part 1: x += dx (FP64) and dx = 0 for the updated components.
-__global__ void k_mpc_xupdate(MixedArgs A) {
-  const int upd = A.ms->upd;
-  if (!upd) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const int64_t n = A.n;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (!((upd >> c) & 1)) continue;
-    const int64_t o = c * n + i;
-    A.x[o] = A.x[o] + (double)A.dx[o];
-    A.dx[o] = 0.f;
-  }
-}
-
-// Reliable update, part 2: r64 = b - A x (FP64 operator, rows in SELL order), r = (float) r64;
-// convergence on the true residual; rho = r.z and the next beta from the replaced residual (0 when
-// the direction restarts).
-__global__ void __launch_bounds__(kRunThreads, 1) k_mpc_residual(MixedArgs A) {
-  const int upd = A.ms->upd;
-  if (!upd) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[2] += 1;
-  const int64_t n = A.n;
-  const int s1 = A.S.rfirst[blockIdx.x + 1];
-  __shared__ int s_next;
-  const int sl0 = run_first_slice(&s_next, A.S.rfirst[blockIdx.x]);
-  with_mask<3>(upd, [&](auto mk) {
-    constexpr int MASK = decltype(mk)::value;
-    for (int sl = sl0; sl < s1; sl = run_next_slice(&s_next)) {
-      const int r = sl * kSellC + (threadIdx.x & 31);
-      const int i = A.S.perm[r];
-      double part[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      if (i >= 0) {
-        double acc[3];
-        sell_spmv_row<3, kU64, MASK>(A.S, A.At64, A.x, n, r, acc);
-        const double w = A.cw ? A.cw[i] : 1.0;
-        const float dinv = A.invA32[i];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((MASK >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          const double ri = A.b[o] - acc[c];
-          A.r64[o] = ri;
-          const float rf = (float)ri;
-          A.r[o] = rf;
-          part[c] = (ri * ri) * w;
-          part[3 + c] = (double)rf * (double)(dinv * rf);
-        }
-      }
-      slice_partial<6>(part, A.S, sl);
-    }
-  });
-  double tot[6];
-  if (grid_reduce_runs<6>(A.S, A.red, tot) && threadIdx.x == 0) {
-    MixedState *m = A.ms;
-    for (int c = 0; c < 3; ++c) {
-      if (!((upd >> c) & 1)) continue;
-      m->updates[c] += 1;
-      const double prev2 = m->rnorm2[c];  // true residual at the previous update
-      m->rnorm2[c] = tot[c];
-      const double rz = tot[3 + c];
-      if (isnan(tot[c]) || isnan(rz)) {
-        m->status[c] = KS_BREAKDOWN;
-        m->active &= ~(1 << c);
-      } else if (tot[c] <= m->tol2[c]) {
-        m->status[c] = KS_CONVERGED;
-        m->active &= ~(1 << c);
-      } else if (m->iters[c] >= m->maxit) {
-        m->status[c] = KS_MAXIT;
-        m->active &= ~(1 << c);
-      } else {
-        // the FP32 recurrence drifted from the true residual, or convergence turned erratic:
-        // restart the direction from the replaced residual
-        const bool restart = tot[c] > kMixedDrift2 * m->rin2[c] || tot[c] > prev2;
-        m->beta[c] = restart ? 0.0 : rz / m->rho[c];
-        if (restart) m->restarts[c] += 1;
-        m->rho[c] = rz;
-        m->rin2[c] = tot[c];
-        m->rmax2[c] = tot[c];
-      }
-    }
-    m->upd = 0;
-    if (A.use_cond) cudaGraphSetConditional(A.cond, m->active ? 1u : 0u);
-  }
-}
-
-// C3: p = z + beta p with z = D^-1 r (after the update, which may have replaced r and beta)
-__global__ void k_mpc_p(MixedArgs A) {
-  const int act = A.ms->active;
-  if (!act) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const int64_t n = A.n;
-  const float dinv = A.invA32[i];
-  float beta[3], rv[3], pv[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    beta[c] = (float)A.ms->beta[c];
-    if ((act >> c) & 1) rv[c] = A.r[c * n + i], pv[c] = A.p[c * n + i];
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-    if ((act >> c) & 1) A.p[c * n + i] = dinv * rv[c] + beta[c] * pv[c];
 }
 
 // ------------------------------------------------------------------------------------------
