@@ -37,6 +37,15 @@ struct NvtxRange {
   ~NvtxRange() { nvtxRangePop(); }
 };
 
+// Windows of the CTAs of a resident solve (WindowView); longest == 0: none, some list is too long for
+// 16-bit positions.
+struct Windows {
+  int *ptr = nullptr, *col = nullptr;
+  unsigned short *idx = nullptr;
+  int longest = 0;
+  WindowView view() const { return WindowView{ptr, col, idx}; }
+};
+
 // Operators of at most this many rows are solved by one CTA, whose barriers are block-wide ones: a
 // momentum CG iteration of 549 rows takes 17 us in one CTA and 20 us on several, of 1037 rows 23 and 20.
 constexpr int kOneCtaRows = 768;
@@ -161,7 +170,7 @@ struct cfsa_ns {
   double *wb = nullptr, *wr = nullptr, *wr0 = nullptr, *wp = nullptr, *wv = nullptr, *ws = nullptr,
          *wt = nullptr;  // [3][N2]
   double *pb = nullptr, *pr = nullptr, *pz = nullptr, *pp = nullptr, *pq = nullptr, *ps = nullptr,
-         *pt = nullptr, *pv = nullptr, *pu = nullptr;  // [nv]
+         *pt = nullptr, *pv = nullptr;  // [nv]
   double *stash = nullptr;
   // boundary faces
   int *fverts = nullptr, *ftet = nullptr, *vf_ptr = nullptr, *vf = nullptr;
@@ -187,7 +196,9 @@ struct cfsa_ns {
   // SMEM-resident variant of the persistent CG (k_cg_resident): one 1024-thread CTA per SM
   bool cg_resident = false;
   double *cg1_vec[3] = {nullptr, nullptr, nullptr};  // second r, w, s buffers of k_cg1_resident
-  int cg_res_grid = 0, cg_res_bpc_sell = 0, cg_res_bpc_nat = 0, cg_res_col_cap = 0;
+  int cg_res_grid = 0, cg_res_bpc_sell = 0, cg_res_bpc_nat = 0, cg_res_entries = 0;  // entries: most of one CTA
+  int smem_optin = 0;
+  Windows win1;  // columns the resident pressure solvers' CTAs read
   size_t cg_res_smem = 0;
   double *res_part = nullptr;  // block partials of the resident Krylov solves, [2][kMaxRed][res_stride]
   int res_stride = 0;
@@ -206,7 +217,7 @@ struct cfsa_ns {
   int coarse_nc = 0;
   std::vector<void *> coarse_allocs;
   CoarseView coarse_view{};
-  int cg2l_col_cap = 0;
+  CgResidentArgs cg2l_caps{};
   size_t cg2l_smem = 0;
   double *cg_part_a = nullptr, *cg_part_b = nullptr;
   // mixed precision (FP32 BiCGSTAB with FP64 reliable updates)
@@ -216,7 +227,7 @@ struct cfsa_ns {
   MixedState *ms = nullptr;
   MixedState *h_ms = nullptr;
   // mixed-precision pressure (two-level CG in float storage inside FP64 defect correction)
-  float *Ls32 = nullptr, *invL32 = nullptr, *px32 = nullptr, *pp32 = nullptr, *pu32 = nullptr;
+  float *Ls32 = nullptr, *invL32 = nullptr, *px32 = nullptr, *pp32 = nullptr;
   float *pr32[2] = {nullptr, nullptr}, *pw32[2] = {nullptr, nullptr}, *ps32[2] = {nullptr, nullptr};
   CgState *cs_in = nullptr;
   PMixState *pmx = nullptr;
@@ -233,7 +244,6 @@ struct cfsa_ns {
     if (mixed_delta > 0.0) return mixed_delta;
     return mom_krylov == CFSA_KRYLOV_CG ? 1e-4 : 1e-2;
   }
-  bool cg2l_split = false;  // two-level CG iteration in two passes (u stored, one gather per entry)
 
   // discrete adjoint (ns_adjoint.cuh): transposed P1 slots, vertex -> (boundary face, local
   // index in the face's tet) incidence, host vertex coordinates for objective patches
@@ -358,6 +368,71 @@ struct cfsa_ns {
     k_sell_fill<<<blocks_for(S.nrows_pad), kBlock, 0, stream>>>(S.nrows_pad, S.sptr, S.perm, S.len,
                                                                 d_rp, d_ci, S.col, S.posmap);
     CK(cudaGetLastError());
+  }
+
+  // Windows of `grid` CTAs that own the slice ranges `runs` (format of SellView::rfirst) of S.
+  Windows build_windows(const Sell &S, const std::vector<int> &runs, int grid, int ncols) {
+    const int words = (ncols + 31) / 32;
+    struct Scratch {  // device memory of this call
+      std::vector<void *> p;
+      ~Scratch() {
+        for (void *q : p) cudaFree(q);
+      }
+      int *get(size_t n) {
+        void *q = nullptr;
+        CK(cudaMalloc(&q, n * sizeof(int)));
+        p.push_back(q);
+        return static_cast<int *>(q);
+      }
+    } tmp;
+    int *d_runs = tmp.get(runs.size()), *bits = tmp.get((size_t)grid * words), *pre = tmp.get((size_t)grid * words),
+        *count = tmp.get(grid);
+    CK(cudaMemcpyAsync(d_runs, runs.data(), runs.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemsetAsync(bits, 0, (size_t)grid * words * sizeof(int), stream));
+    k_window_mark<<<grid, 1024, 0, stream>>>(S.view(), d_runs, words, reinterpret_cast<unsigned int *>(bits));
+    k_window_scan<<<grid, 32, 0, stream>>>(words, reinterpret_cast<unsigned int *>(bits), pre, count);
+    CK(cudaGetLastError());
+    std::vector<int> h(grid), ptr(grid + 1, 0);
+    CK(cudaMemcpyAsync(h.data(), count, grid * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    Windows w;
+    for (int c = 0; c < grid; ++c) {
+      ptr[c + 1] = ptr[c] + h[c];
+      w.longest = std::max(w.longest, h[c]);
+    }
+    if (w.longest > 65535) return Windows{};
+    w.ptr = dupload(ptr);
+    w.col = dalloc<int>(ptr[grid]);
+    w.idx = dalloc<unsigned short>((size_t)S.nentries);
+    CK(cudaMemsetAsync(w.idx, 0, (size_t)S.nentries * sizeof(unsigned short), stream));
+    k_window_list<<<grid, 1024, 0, stream>>>(S.view(), d_runs, words, reinterpret_cast<unsigned int *>(bits), pre,
+                                             w.ptr, w.col, w.idx);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(stream));
+    return w;
+  }
+
+  // What of a CTA's rows a resident pressure kernel keeps in shared memory next to `fixed` bytes of its
+  // own and `reserved` static ones: the row data if they fit; the window with every entry's position if
+  // they fit too, then values of as many entries as there is room for; otherwise columns.
+  CgResidentArgs resident_caps(int64_t fixed, int64_t reserved) const {
+    CgResidentArgs r{};
+    r.nslices = s1.nslices;
+    r.bpc_sell = cg_res_bpc_sell;
+    r.bpc_nat = cg_res_bpc_nat;
+    r.W = win1.view();
+    const int64_t avail = smem_optin - reserved - fixed - 16;  // 16: alignment
+    const auto bytes = [](int rows, int win, int ent, int val) { return (int64_t)resident_rows_bytes(rows, win, ent, val); };
+    const int rows = cg_res_bpc_sell * kBlock;
+    if (bytes(rows, 0, 0, 0) <= avail) r.row_cap = rows;
+    if (win1.longest > 0 && bytes(r.row_cap, win1.longest, cg_res_entries, 0) <= avail) {
+      r.win_cap = win1.longest;
+      r.ent_cap = cg_res_entries;
+      r.val_cap = (int)std::min<int64_t>(cg_res_entries, (avail - bytes(r.row_cap, r.win_cap, r.ent_cap, 0)) / (int64_t)sizeof(double));
+    } else {
+      r.ent_cap = (int)std::min<int64_t>(cg_res_entries, std::max<int64_t>(0, avail - bytes(r.row_cap, 0, 0, 0)) / (int64_t)sizeof(int));
+    }
+    return r;
   }
 
   void build_pattern(bool p2, int nrows, std::vector<int> &h_rp, int *&d_rp, int *&d_ci,
@@ -498,7 +573,7 @@ struct cfsa_ns {
     p = dalloc<double>(nv);
     pc = dalloc<double>(nv);
     for (double **w : {&wb, &wr, &wr0, &wp, &wv, &ws, &wt}) *w = dalloc<double>(n3);
-    for (double **w : {&pb, &pr, &pz, &pp, &pq, &ps, &pt, &pv, &pu}) *w = dalloc<double>(nv);
+    for (double **w : {&pb, &pr, &pz, &pp, &pq, &ps, &pt, &pv}) *w = dalloc<double>(nv);
     ct = dalloc<double>((size_t)nt * 3);
     divt = dalloc<double>(nt);
     stash = dalloc<double>(1);
@@ -539,7 +614,7 @@ struct cfsa_ns {
     CK(cudaMemsetAsync(ms, 0, sizeof(MixedState), stream));
     Ls32 = dalloc<float>((size_t)s1.nentries);
     CK(cudaMemsetAsync(Ls32, 0, (size_t)s1.nentries * sizeof(float), stream));
-    for (float **w : {&invL32, &px32, &pp32, &pu32, &pr32[0], &pr32[1], &pw32[0], &pw32[1], &ps32[0], &ps32[1]})
+    for (float **w : {&invL32, &px32, &pp32, &pr32[0], &pr32[1], &pw32[0], &pw32[1], &ps32[0], &ps32[1]})
       *w = dalloc<float>((size_t)nv);
     cs_in = dalloc<CgState>(1);
     pmx = dalloc<PMixState>(1);
@@ -548,7 +623,6 @@ struct cfsa_ns {
     CK(cudaMallocHost(&h_pmx, sizeof(PMixState)));
     if (const char *e = std::getenv("CFSA_MIXED_P_TOL_IN")) mixed_p_tol_in = std::atof(e);
     if (const char *e = std::getenv("CFSA_MIXED_DELTA")) mixed_delta = std::atof(e);
-    if (const char *e = std::getenv("CFSA_CG2L_SPLIT")) cg2l_split = std::atoi(e) != 0;
 
     bs_prof = dalloc<BicgState>(1);
     cs_prof = dalloc<CgState>(1);
@@ -618,38 +692,27 @@ struct cfsa_ns {
       for (double *&v : cg1_vec) v = dalloc<double>((size_t)nv);
       if (cg_grid < 1) cg_persistent = false;
       // resident variant: blocks split into contiguous runs, one run per SM
-      int optin = 0;
-      CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-      const int grid = std::max(1, std::min(nsm, std::max(nblk_sell, nblk_nat)));
-      const int bpc_s = (nblk_sell + grid - 1) / grid, bpc_n = (nblk_nat + grid - 1) / grid;
-      int max_entries = 0;
-      for (int c = 0; c < grid; ++c) {
-        const int b0 = std::min(nblk_sell, c * bpc_s), b1 = std::min(nblk_sell, b0 + bpc_s);
-        if (b1 > b0)
-          max_entries = std::max(max_entries, s1.h_sptr[std::min(8 * b1, s1.nslices)] - s1.h_sptr[8 * b0]);
-      }
-      const int64_t row_bytes = (int64_t)3 * bpc_s * kBlock * (int64_t)sizeof(int);
-      const int64_t avail = (int64_t)optin - 2048 - row_bytes;  // 2 KiB for static shared memory
-      if (avail > 0) {
-        cg_res_col_cap = (int)std::min<int64_t>(max_entries, avail / (int64_t)sizeof(int));
-        cg_res_smem = (size_t)(row_bytes + (int64_t)cg_res_col_cap * (int64_t)sizeof(int));
-        int per_sm_res = 0;
-        int per_sm_res1 = 0;
-        if (cudaFuncSetAttribute(k_cg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cg_res_smem) == cudaSuccess &&
-            cudaFuncSetAttribute(k_cg1_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cg_res_smem) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_res, k_cg_resident, kCgResThreads,
-                                                          cg_res_smem) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_res1, k_cg1_resident, kCgResThreads,
-                                                          cg_res_smem) == cudaSuccess &&
-            per_sm_res >= 1 && per_sm_res1 >= 1) {
-          cg_resident = true;
-          cg_res_grid = grid;
-          cg_res_bpc_sell = bpc_s;
-          cg_res_bpc_nat = bpc_n;
-        }
-        cudaGetLastError();
+      CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+      cg_res_grid = std::max(1, std::min(nsm, std::max(nblk_sell, nblk_nat)));
+      cg_res_bpc_sell = (nblk_sell + cg_res_grid - 1) / cg_res_grid;
+      cg_res_bpc_nat = (nblk_nat + cg_res_grid - 1) / cg_res_grid;
+      std::vector<int> runs(2 * (cg_res_grid + 1), s1.nslices);  // one range per CTA, no second one
+      for (int c = 0; c <= cg_res_grid; ++c) runs[c] = std::min(s1.nslices, kSlicesPerBlock * c * cg_res_bpc_sell);
+      for (int c = 0; c < cg_res_grid; ++c)
+        cg_res_entries = std::max(cg_res_entries, s1.h_sptr[runs[c + 1]] - s1.h_sptr[runs[c]]);
+      // CFSA_NO_WINDOWS=1: gather from global memory, as on meshes whose windows do not fit
+      const char *no_win = std::getenv("CFSA_NO_WINDOWS");
+      if (!no_win || std::atoi(no_win) == 0) win1 = build_windows(s1, runs, cg_res_grid, (int)nv);
+      const CgResidentArgs caps = resident_caps(0, 2048);  // 2 KiB for static shared memory
+      cg_res_smem = resident_rows_bytes(caps.row_cap, caps.win_cap, caps.ent_cap, caps.val_cap);
+      cg_resident = caps.row_cap > 0;
+      for (const void *fn : {(const void *)k_cg_resident<true>, (const void *)k_cg_resident<false>,
+                             (const void *)k_cg1_resident<true>, (const void *)k_cg1_resident<false>,
+                             (const void *)k_bicg_resident<true>, (const void *)k_bicg_resident<false>}) {
+        int o = 0;
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_res_smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kCgResThreads, cg_res_smem));
+        if (o < 1) throw CudaError{"resident pressure solver does not fit on an SM"};
       }
     }
     if (const char *e = std::getenv("CFSA_CG_LOOP")) cg_persistent = cg_persistent && (std::atoi(e) == 0);
@@ -918,35 +981,26 @@ struct cfsa_ns {
     V.need = cupload(need);
     V.gacc = cupload(std::vector<unsigned long long>((size_t)27 * std::max(nc, 1), 0ull));
     V.npos_max = npos_max;
-    // shared memory: coarse arrays, row staging, then as many column indices as fit
-    int optin = 0;
-    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    cudaFuncAttributes fa{};
-    CK(cudaFuncGetAttributes(&fa, k_cg2l_resident<double, false>));
-    const int64_t coarse_bytes = (int64_t)(6 * nc + 2 + 2 * npos_max) * (int64_t)sizeof(double);
-    const int64_t row_bytes = (int64_t)3 * cg_res_bpc_sell * kBlock * (int64_t)sizeof(int);
-    const int64_t avail = (int64_t)optin - (int64_t)fa.sharedSizeBytes - coarse_bytes - row_bytes;
-    if (avail < 0) throw CudaError{"two-level pressure preconditioner: coarse space too large for shared memory"};
-    int max_entries = 0;
-    for (int c = 0; c < cg_res_grid; ++c) {
-      const int b0 = std::min(nblk_sell, c * cg_res_bpc_sell), b1 = std::min(nblk_sell, b0 + cg_res_bpc_sell);
-      if (b1 > b0) max_entries = std::max(max_entries, s1.h_sptr[std::min(8 * b1, s1.nslices)] - s1.h_sptr[8 * b0]);
+    // shared memory: coarse arrays, then the rows
+    const void *const kernels[] = {(const void *)k_cg2l_resident<double, true>, (const void *)k_cg2l_resident<double, false>,
+                                   (const void *)k_cg2l_resident<float, true>, (const void *)k_cg2l_resident<float, false>};
+    size_t fixed_smem = 0;
+    for (const void *fn : kernels) {
+      cudaFuncAttributes fa{};
+      CK(cudaFuncGetAttributes(&fa, fn));
+      fixed_smem = std::max(fixed_smem, fa.sharedSizeBytes);
     }
-    cg2l_col_cap = (int)std::min<int64_t>(max_entries, avail / (int64_t)sizeof(int));
-    cg2l_smem = (size_t)(coarse_bytes + row_bytes + (int64_t)cg2l_col_cap * (int64_t)sizeof(int));
-    int per_sm = 1;
-    for (const void *fn : {(const void *)k_cg2l_resident<double, false>, (const void *)k_cg2l_resident<float, false>,
-                           (const void *)k_cg2l_resident<double, true>, (const void *)k_cg2l_resident<float, true>}) {
-      cudaFuncAttributes fb{};
-      CK(cudaFuncGetAttributes(&fb, fn));
-      if (fb.sharedSizeBytes > fa.sharedSizeBytes)
-        throw CudaError{"two-level pressure preconditioner: float form needs more static shared memory"};
+    const int64_t coarse_bytes = (int64_t)(4 * nc + 2 + 2 * npos_max) * (int64_t)sizeof(double);
+    cg2l_caps = resident_caps(coarse_bytes, (int64_t)fixed_smem);
+    if (!cg2l_caps.row_cap) throw CudaError{"two-level pressure preconditioner: coarse space too large for shared memory"};
+    cg2l_smem = (size_t)coarse_bytes +
+                resident_rows_bytes(cg2l_caps.row_cap, cg2l_caps.win_cap, cg2l_caps.ent_cap, cg2l_caps.val_cap);
+    for (const void *fn : kernels) {
       CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg2l_smem));
       int o = 0;
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kCgResThreads, cg2l_smem));
-      per_sm = std::min(per_sm, o);
+      if (o < 1) throw CudaError{"two-level pressure preconditioner: kernel does not fit on an SM"};
     }
-    if (per_sm < 1) throw CudaError{"two-level pressure preconditioner: kernel does not fit on an SM"};
     CK(cudaStreamSynchronize(stream));
     coarse_view = V;
     coarse_nc = nc;
@@ -1275,12 +1329,8 @@ struct cfsa_ns {
     c.st = s_out;
     c.bar = GridBarrier{bar_count, bar_err, bar_spin_limit};
     c.scaled = (conv_norm == CFSA_NORM_JACOBI) ? 1 : 0;
-    CgResidentArgs rz{};
+    CgResidentArgs rz = cg2l_caps;
     rz.P = c;
-    rz.nslices = s1.nslices;
-    rz.bpc_sell = cg_res_bpc_sell;
-    rz.bpc_nat = cg_res_bpc_nat;
-    rz.col_cap = cg2l_col_cap;
     Cg2lArgs c2{};
     c2.R = rz;
     c2.V = coarse_view;
@@ -1295,8 +1345,6 @@ struct cfsa_ns {
     c2.invL32 = invL32;
     c2.x32 = px32;
     c2.p32 = pp32;
-    c2.u = pu;
-    c2.u32 = pu32;
     for (int q = 0; q < 2; ++q) {
       c2.r32[q] = pr32[q];
       c2.w32[q] = pw32[q];
@@ -1321,10 +1369,11 @@ struct cfsa_ns {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    const bool win = c2.R.win_cap > 0;
     if (f32)
-      CK(cudaLaunchKernelEx(&cfg, cg2l_split ? k_cg2l_resident<float, true> : k_cg2l_resident<float, false>, c2));
+      CK(cudaLaunchKernelEx(&cfg, win ? k_cg2l_resident<float, true> : k_cg2l_resident<float, false>, c2));
     else
-      CK(cudaLaunchKernelEx(&cfg, cg2l_split ? k_cg2l_resident<double, true> : k_cg2l_resident<double, false>, c2));
+      CK(cudaLaunchKernelEx(&cfg, win ? k_cg2l_resident<double, true> : k_cg2l_resident<double, false>, c2));
   }
 
   // Mixed-precision pressure solve (ns_mixed.cuh): FP64 defect correction around the float
@@ -1378,6 +1427,33 @@ struct cfsa_ns {
     return h_pmx->active != 0;
   }
 
+  // The whole pressure BiCGSTAB in one cooperative launch.
+  void launch_pressure_bicg(const BicgArgs &b) {
+    PBicgArgs a{};
+    a.B = b;
+    a.R = resident_caps(0, 2048);
+    a.R.P.S = s1.view();
+    a.R.P.nblk_sell = (int)blocks_for(s1.nrows_pad);
+    a.R.P.nblk_nat = (int)blocks_for(nv);
+    a.R.P.part_a = cg_part_a;
+    a.R.P.part_b = cg_part_b;
+    a.R.P.bar = GridBarrier{bar_count, bar_err, kBarrierSpinLimit};
+    a.p2 = pp2;
+    a.v2 = pv2;
+    clear_barrier(stream);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned int)cg_res_grid);
+    cfg.blockDim = dim3(kCgResThreads);
+    cfg.dynamicSmemBytes = cg_res_smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, a.R.win_cap ? k_bicg_resident<true> : k_bicg_resident<false>, a));
+  }
+
   // Pressure Krylov solve (state set up by k_pressure_rhs) into x; failures and iteration
   // counts go to `s_out`. Mixed precision applies to the two-level CG (the other methods solve
   // in FP64 in both precisions).
@@ -1406,7 +1482,7 @@ struct cfsa_ns {
       b.st = s_out;
       b.slot = 1;
       b.cw = (conv_norm == CFSA_NORM_JACOBI) ? invL : nullptr;
-      CFSA_RESIDENT(k_bicg_solve1, (PBicgArgs{b, pp2, pv2}), s1, stream);
+      launch_pressure_bicg(b);
       k_check_bicg<<<1, 1, 0, stream>>>(bs_p, 1, 1, s_out, bar_err);
     } else if (cg_persistent || krylov == CFSA_KRYLOV_CG1 || krylov == CFSA_KRYLOV_CG2L) {
       CgPersistentArgs c{};
@@ -1443,12 +1519,8 @@ struct cfsa_ns {
         CK(cudaMemsetAsync(ps, 0, (size_t)nv * sizeof(double), stream));
         launch_cg2l(cg2l_args(x, s_out, cs), false, stream);
       } else if (krylov == CFSA_KRYLOV_CG1) {
-        CgResidentArgs rz{};
+        CgResidentArgs rz = resident_caps(0, 2048);
         rz.P = c;
-        rz.nslices = s1.nslices;
-        rz.bpc_sell = cg_res_bpc_sell;
-        rz.bpc_nat = cg_res_bpc_nat;
-        rz.col_cap = cg_res_col_cap;
         Cg1Args c1{};
         c1.R = rz;
         c1.r[0] = pr;
@@ -1464,18 +1536,14 @@ struct cfsa_ns {
         cfg.gridDim = dim3((unsigned int)cg_res_grid);
         cfg.blockDim = dim3(kCgResThreads);
         cfg.dynamicSmemBytes = cg_res_smem;
-        CK(cudaLaunchKernelEx(&cfg, k_cg1_resident, c1));
+        CK(cudaLaunchKernelEx(&cfg, rz.win_cap ? k_cg1_resident<true> : k_cg1_resident<false>, c1));
       } else if (cg_resident) {
-        CgResidentArgs rz{};
+        CgResidentArgs rz = resident_caps(0, 2048);
         rz.P = c;
-        rz.nslices = s1.nslices;
-        rz.bpc_sell = cg_res_bpc_sell;
-        rz.bpc_nat = cg_res_bpc_nat;
-        rz.col_cap = cg_res_col_cap;
         cfg.gridDim = dim3((unsigned int)cg_res_grid);
         cfg.blockDim = dim3(kCgResThreads);
         cfg.dynamicSmemBytes = cg_res_smem;
-        CK(cudaLaunchKernelEx(&cfg, k_cg_resident, rz));
+        CK(cudaLaunchKernelEx(&cfg, rz.win_cap ? k_cg_resident<true> : k_cg_resident<false>, rz));
       } else {
         CK(cudaLaunchKernelEx(&cfg, k_cg_persistent, c));
       }
@@ -1561,7 +1629,7 @@ struct cfsa_ns {
     b.st = st;
     b.slot = 1;
     b.cw = nullptr;
-    CFSA_RESIDENT(k_bicg_solve1, (PBicgArgs{b, pp2, pv2}), s1, stream);
+    launch_pressure_bicg(b);
     k_check_bicg<<<1, 1, 0, stream>>>(bs_p, 1, 1, st, bar_err);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(x_host, d_x, (size_t)nv * sizeof(double), cudaMemcpyDeviceToHost, stream));

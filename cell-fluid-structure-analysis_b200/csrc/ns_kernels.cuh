@@ -979,6 +979,74 @@ __global__ void k_cg_p(CgArgs A) {
 }
 
 // ------------------------------------------------------------------------------------------
+// Windows: the distinct columns of the rows that one CTA of a resident solve owns, in ascending order,
+// and every entry's position in its CTA's list. A product then reads each needed vector entry once per
+// CTA from L2 into shared memory and gathers from there. Built once per pattern from a bitmap per CTA:
+// mark the columns, count the bits before each word, list the marked columns. `runs`: the slice ranges
+// of the CTAs in the format of SellView::rfirst.
+struct WindowView {
+  const int *ptr;             // [G+1] list of CTA c: col[ptr[c]] .. col[ptr[c+1]]
+  const int *col;
+  const unsigned short *idx;  // [nentries] position in the owner's list, SELL layout; nullptr: no windows
+};
+
+template <class F>
+__device__ __forceinline__ void each_run_entry(const SellView &S, const int *runs, F &&f) {
+  const int *r = runs + blockIdx.x, *r2 = r + gridDim.x + 1;
+  const int na = r[1] - r[0], n = na + r2[1] - r2[0], lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < n; q += blockDim.x >> 5) {
+    const int sl = (q < na) ? r[0] + q : r2[0] + q - na;
+    const int base = S.sptr[sl] + lane, len = S.len[sl * kSellC + lane];
+    for (int k = 0; k < len; ++k) f(base + k * kSellC);
+  }
+}
+
+__global__ void k_window_mark(SellView S, const int *__restrict__ runs, int words, unsigned int *bits) {
+  unsigned int *b = bits + (size_t)blockIdx.x * words;
+  each_run_entry(S, runs, [&](int pos) {
+    const int j = S.col[pos];
+    const unsigned int m = 1u << (j & 31);
+    if (!(*(volatile unsigned int *)(b + (j >> 5)) & m)) atomicOr(b + (j >> 5), m);
+  });
+}
+
+// pre[w]: marked columns before word w; count[c]: all of CTA c's. One warp per 32-word chunk would need a
+// second pass; one warp walks the words 32 at a time (set-up only, a few thousand words).
+__global__ void k_window_scan(int words, const unsigned int *__restrict__ bits, int *__restrict__ pre,
+                              int *__restrict__ count) {
+  const unsigned int *b = bits + (size_t)blockIdx.x * words;
+  int *p = pre + (size_t)blockIdx.x * words;
+  int total = 0;
+  for (int w0 = 0; w0 < words; w0 += 32) {
+    const int w = w0 + (int)threadIdx.x, n = (w < words) ? __popc(b[w]) : 0;
+    int s = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, s, o);
+      if ((int)threadIdx.x >= o) s += v;
+    }
+    if (w < words) p[w] = total + s - n;
+    total += __shfl_sync(0xffffffffu, s, 31);
+  }
+  if (threadIdx.x == 0) count[blockIdx.x] = total;
+}
+
+__global__ void k_window_list(SellView S, const int *__restrict__ runs, int words,
+                              const unsigned int *__restrict__ bits, const int *__restrict__ pre,
+                              const int *__restrict__ ptr, int *__restrict__ col, unsigned short *__restrict__ idx) {
+  const unsigned int *b = bits + (size_t)blockIdx.x * words;
+  const int *p = pre + (size_t)blockIdx.x * words;
+  for (int w = threadIdx.x; w < words; w += blockDim.x) {
+    int o = ptr[blockIdx.x] + p[w];
+    for (unsigned int m = b[w]; m; m &= m - 1) col[o++] = 32 * w + __ffs(m) - 1;
+  }
+  each_run_entry(S, runs, [&](int pos) {
+    const int j = S.col[pos], w = j >> 5;
+    idx[pos] = (unsigned short)(p[w] + __popc(b[w] & ((1u << (j & 31)) - 1u)));
+  });
+}
+
+// ------------------------------------------------------------------------------------------
 // Persistent CG: the whole pressure solve in one cooperative launch. Per iteration:
 //   A  (SELL blocks)    p_new = z + beta p (on the fly, double-buffered), q = L p_new, p.q partials
 //   -- grid barrier --
@@ -1230,22 +1298,27 @@ __global__ void __launch_bounds__(kBlock, 4) k_cg_persistent(CgPersistentArgs A)
 }
 
 // ------------------------------------------------------------------------------------------
-// SMEM-resident persistent CG: one CTA of 1024 threads per SM for the whole solve. Each CTA owns
-// a contiguous run of 256-position blocks (SELL blocks for the product, natural blocks for the
-// vector updates) and keeps, in shared memory for the whole solve, the row id, length and entry
-// base of each of its SELL positions and the column indices of as many of its slices as fit
-// (the rest are read from global memory). Inside an iteration the column indices then cost a
-// shared-memory read instead of an L2 round trip before the gathers can be issued. The
-// arithmetic, the per-block partial sums and the 256-accumulator tree are those of
-// k_cg_persistent, so both kernels produce the same bits.
-constexpr int kCgResThreads = 1024;
+// Resident pressure solvers: one CTA per SM for the whole solve. Each CTA owns a contiguous run of
+// 256-position blocks (SELL blocks for the product, natural blocks for the vector updates) and keeps in
+// shared memory what it needs of its rows in every iteration (ResidentRows). The arithmetic, the
+// per-block partial sums and the 256-accumulator tree are those of k_cg_persistent, so both kernels
+// produce the same bits.
+// 512 threads per CTA: 128 registers per thread leave room for every load of a row in flight, and the
+// block-wide steps of an iteration (half a dozen) cost less with 16 warps than with 32. Two-level CG, us per
+// iteration with 1024 / 768 / 512 threads: 16.1 / 12.9 / 11.7 at 30k tets, 14.9 / 13.8 / 11.8 at 250k,
+// 24.7 / 20.8 / 19.0 at 1M.
+constexpr int kCgResThreads = 512;
 constexpr int kCgResGroups = kCgResThreads / kBlock;  // 256-thread groups per CTA
 
 struct CgResidentArgs {
   CgPersistentArgs P;
   int nslices;
   int bpc_sell, bpc_nat;  // blocks per CTA
-  int col_cap;            // column indices that fit in shared memory per CTA
+  WindowView W;
+  int row_cap;  // positions per CTA whose row data fit in shared memory (all or 0)
+  int win_cap;  // longest window (0: no windows, the products gather from global memory)
+  int ent_cap;  // entries per CTA whose indices fit in shared memory (window positions: all; or columns)
+  int val_cap;  // entries per CTA whose values fit too (windows only)
 };
 
 __device__ __forceinline__ void group_sync(int g) {
@@ -1275,49 +1348,188 @@ __device__ __forceinline__ void group_partial(double (&v)[NV], double *__restric
   group_sync(g);
 }
 
-// tree_total for a 1024-thread CTA: the 256-thread quarter j forms the 256 accumulators of value
-// j (same sums in the same order as tree_total), so the values are reduced side by side with eight
-// loads in flight per thread instead of one value after another.
+// tree_total for a resident CTA: the accumulators of all values are formed side by side, eight loads in
+// flight per thread (same sums in the same order as tree_total). Calls are a grid barrier apart, which
+// keeps sm from being rewritten while it is read.
 template <int NV>
 __device__ __forceinline__ void tree_total_cta(const double *__restrict__ partials, int nblk,
                                                double (&out)[NV], double (*sm)[kBlock / 32]) {
-  static_assert(NV * kBlock <= kCgResThreads, "one 256-thread quarter per value");
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = threadIdx.x / kBlock, t = threadIdx.x & (kBlock - 1);
-  if (j < NV) {
-    // accumulator t of value j: blocks t, t + 256, ... in order, eight loads in flight
+  for (int a = threadIdx.x; a < NV * kBlock; a += kCgResThreads) {
+    // accumulator t of value j: blocks t, t + 256, ... in order
+    const int j = a / kBlock, t = a & (kBlock - 1);
     constexpr int kB = 8;
     double s = 0.0;
-    int b = t;
-    for (; b + (kB - 1) * kBlock < nblk; b += kB * kBlock) {
+    for (int b = t; b < nblk; b += kB * kBlock) {
       double v[kB];
 #pragma unroll
-      for (int q = 0; q < kB; ++q) v[q] = __ldcg(&partials[(size_t)(b + q * kBlock) * kMaxRed + j]);
+      for (int q = 0; q < kB; ++q)
+        v[q] = (b + q * kBlock < nblk) ? __ldcg(&partials[(size_t)(b + q * kBlock) * kMaxRed + j]) : 0.0;
 #pragma unroll
-      for (int q = 0; q < kB; ++q) s += v[q];
+      for (int q = 0; q < kB; ++q)
+        if (b + q * kBlock < nblk) s += v[q];
     }
-    double v[kB];
-#pragma unroll
-    for (int q = 0; q < kB; ++q)
-      v[q] = (b + q * kBlock < nblk) ? __ldcg(&partials[(size_t)(b + q * kBlock) * kMaxRed + j]) : 0.0;
-#pragma unroll
-    for (int q = 0; q < kB; ++q)
-      if (b + q * kBlock < nblk) s += v[q];
     s = warp_sum(s);
-    if (lane == 0) sm[j][warp & (kBlock / 32 - 1)] = s;
+    if ((threadIdx.x & 31) == 0) sm[j][t >> 5] = s;
   }
   __syncthreads();
 #pragma unroll
-  for (int j2 = 0; j2 < NV; ++j2) {
+  for (int j = 0; j < NV; ++j) {
     double s = 0.0;
-    for (int w = 0; w < kBlock / 32; ++w) s += sm[j2][w];
-    out[j2] = s;
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) s += sm[j][w];
+    out[j] = s;
   }
-  __syncthreads();
 }
 
+// Shared memory of ResidentRows: window and staged values (doubles at most), row data, window columns,
+// then window positions (or, without windows, columns) of the staged entries.
+inline size_t resident_rows_bytes(int rows, int win, int ent, int nval) {
+  return ((size_t)win + nval) * sizeof(double) + ((size_t)rows * 3 + win) * sizeof(int) +
+         (size_t)ent * (win ? sizeof(unsigned short) : sizeof(int));
+}
+
+// A CTA's SELL rows in shared memory for the whole solve (row id, length and entry base of each
+// position, as many indices and then values as fit), and products with a vector that is given as a
+// function of the column.
+//
+// With a window, fill() evaluates the function once per distinct column of the CTA (all of its loads in
+// flight together) and the rows then read shared memory only; without one (the window, or its 16-bit
+// positions, do not fit: meshes numbered without locality, or above ~3M tets) every entry of every row
+// evaluates it from global memory. The expression and the order of each row's sum are the same, so the
+// bits are. The pass over the rows of a two-level CG iteration at 1M tets took 12.7 us with gathers from
+// L2, bound by ten dependent round trips per pair of rows. Shared memory serves a warp's 32 scattered
+// doubles in about 6 cycles of the SM, so a window product is bound by that: 15 entries x (6 + 3) cycles
+// x 38 warps = 2.7 us at 1M tets.
+template <class TS, bool WIN>
+struct ResidentRows {
+  const CgResidentArgs &R;
+  const TS *val;
+  int b0, b1, e0, ent_blk, val_blk, nw;  // blocks [b0, ent_blk) have staged indices, [b0, val_blk) values
+  int *row, *len, *base, *col, *wcol;
+  double *win;
+  TS *sval;
+  unsigned short *idx;
+
+  __device__ ResidentRows(const CgResidentArgs &r, const TS *v, char *smem) : R(r), val(v) {
+    const CgPersistentArgs &A = R.P;
+    const SellView &S = A.S;
+    b0 = min(A.nblk_sell, (int)blockIdx.x * R.bpc_sell);
+    b1 = min(A.nblk_sell, b0 + R.bpc_sell);
+    const int rows = R.row_cap;
+    win = reinterpret_cast<double *>(smem);
+    sval = reinterpret_cast<TS *>(win + R.win_cap);
+    row = reinterpret_cast<int *>(smem + ((size_t)R.win_cap * sizeof(double) + (size_t)R.val_cap * sizeof(TS) + 7) / 8 * 8);
+    len = row + rows;
+    base = len + rows;
+    wcol = base + rows;
+    col = wcol;  // without windows
+    idx = reinterpret_cast<unsigned short *>(wcol + R.win_cap);
+    e0 = (b0 < b1) ? S.sptr[8 * b0] : 0;
+    auto end = [&](int b) { return S.sptr[min(8 * b, R.nslices)] - e0; };
+    ent_blk = val_blk = b0;
+    while (ent_blk < b1 && end(ent_blk + 1) <= R.ent_cap) ++ent_blk;
+    const int ne = (ent_blk > b0) ? end(ent_blk) : 0;
+    nw = 0;
+    if constexpr (WIN) {
+      while (val_blk < b1 && end(val_blk + 1) <= R.val_cap) ++val_blk;
+      const int nv = (val_blk > b0) ? end(val_blk) : 0;
+      const int w0 = R.W.ptr[blockIdx.x];
+      nw = R.W.ptr[blockIdx.x + 1] - w0;
+      for (int q = threadIdx.x; q < nw; q += blockDim.x) wcol[q] = R.W.col[w0 + q];
+      for (int e = threadIdx.x; e < ne; e += blockDim.x) idx[e] = R.W.idx[e0 + e];
+      for (int e = threadIdx.x; e < nv; e += blockDim.x) sval[e] = val[e0 + e];
+    } else {
+      for (int e = threadIdx.x; e < ne; e += blockDim.x) col[e] = S.col[e0 + e];
+    }
+    for (int q = threadIdx.x; q < min(rows, (b1 - b0) * kBlock); q += blockDim.x) {
+      const int r = b0 * kBlock + q;
+      const bool in = r < S.nrows_pad;
+      row[q] = in ? S.perm[r] : -1;
+      len[q] = in ? S.len[r] : 0;
+      base[q] = in ? S.sptr[r >> 5] + (r & 31) : 0;
+    }
+    __syncthreads();
+  }
+
+  // Row at position lp of the CTA, -1: padding.
+  __device__ __forceinline__ int row_of(int lp) const {
+    if (R.row_cap) return row[lp];
+    const int r = b0 * kBlock + lp;
+    return (r < R.P.S.nrows_pad) ? R.P.S.perm[r] : -1;
+  }
+
+  // The vector of the next products: f(j) for every column of the window.
+  template <class F>
+  __device__ __forceinline__ void fill(F &&f) {
+    if constexpr (!WIN) return;
+    constexpr int kB = 3;
+    for (int q0 = threadIdx.x; q0 < nw; q0 += kB * (int)blockDim.x) {
+      double v[kB];
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        const int q = q0 + u * (int)blockDim.x;
+        v[u] = (q < nw) ? f(wcol[q]) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        const int q = q0 + u * (int)blockDim.x;
+        if (q < nw) win[q] = v[u];
+      }
+    }
+    __syncthreads();
+  }
+
+  // Row sum of n entries from o on, in ascending column order: U entries at a time, at(pos, a, x) giving
+  // an entry's value and vector element.
+  template <int U, class F>
+  static __device__ __forceinline__ double sum(int o, int n, F &&at) {
+    double acc = 0.0;
+    int k = 0;
+    for (; k + U <= n; k += U) {
+      double a[U], x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) at(o + (k + u) * kSellC, a[u], x[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc += a[u] * x[u];
+    }
+    if (k < n) {  // the last n % U entries as one predicated chunk
+      double a[U], x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k + u < n) at(o + (k + u) * kSellC, a[u], x[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k + u < n) acc += a[u] * x[u];
+    }
+    return acc;
+  }
+
+  // Row sum of position lp of block b. What is staged is the same for a whole block, so the choice is
+  // made once per row and not per entry (a choice per entry cost 3.2 instead of 1.4 us per pass).
+  template <class F>
+  __device__ __forceinline__ double product(int b, int lp, F &&f) const {
+    const int r = b0 * kBlock + lp;
+    const int n = R.row_cap ? len[lp] : R.P.S.len[r];
+    const int o = R.row_cap ? base[lp] : R.P.S.sptr[r >> 5] + (r & 31);
+    if constexpr (WIN) {
+      const TS *v = (b < val_blk) ? sval : val + e0;  // generic loads: shared or global memory
+      return sum<kCgChunk>(o - e0, n, [&](int p, double &a, double &x) {
+        a = (double)v[p];
+        x = win[idx[p]];
+      });
+    } else {
+      const bool staged = b < ent_blk;
+      return sum<kCgChunk>(o, n, [&](int p, double &a, double &x) {
+        a = (double)__ldg(val + p);
+        x = f(staged ? col[p - e0] : __ldg(R.P.S.col + p));
+      });
+    }
+  }
+};
+
+template <bool WIN>
 __global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs R) {
-  extern __shared__ int s_dyn[];
+  extern __shared__ double s_dbl[];
   __shared__ double s_grp[kCgResGroups][3][kBlock / 32];
   __shared__ double s_tree[3][kBlock / 32];
   const CgPersistentArgs &A = R.P;
@@ -1325,28 +1537,10 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs
   if (!A.cs->active) return;
   unsigned int phase = 0;
   const int g = threadIdx.x / kBlock, lt = threadIdx.x & (kBlock - 1);
-  // owned blocks
-  const int b0 = min(A.nblk_sell, (int)blockIdx.x * R.bpc_sell);
-  const int b1 = min(A.nblk_sell, b0 + R.bpc_sell);
+  ResidentRows<double, WIN> rows(R, A.Ls, reinterpret_cast<char *>(s_dbl));
+  // owned blocks of the vector updates
   const int c0 = min(A.nblk_nat, (int)blockIdx.x * R.bpc_nat);
   const int c1 = min(A.nblk_nat, c0 + R.bpc_nat);
-  int *s_row = s_dyn;                          // [bpc_sell * 256]
-  int *s_len = s_row + R.bpc_sell * kBlock;    // [bpc_sell * 256]
-  int *s_base = s_len + R.bpc_sell * kBlock;   // [bpc_sell * 256]
-  int *s_col = s_base + R.bpc_sell * kBlock;   // [col_cap]
-  const int e0 = (b0 < b1) ? A.S.sptr[8 * b0] : 0;
-  int bs = b0;  // blocks [b0, bs) have their column indices in shared memory
-  while (bs < b1 && A.S.sptr[min(8 * (bs + 1), R.nslices)] - e0 <= R.col_cap) ++bs;
-  const int e1 = (bs > b0) ? A.S.sptr[min(8 * bs, R.nslices)] : e0;
-  for (int e = e0 + (int)threadIdx.x; e < e1; e += kCgResThreads) s_col[e - e0] = A.S.col[e];
-  for (int q = threadIdx.x; q < (b1 - b0) * kBlock; q += kCgResThreads) {
-    const int r = b0 * kBlock + q;
-    const bool in = r < A.S.nrows_pad;
-    s_row[q] = in ? A.S.perm[r] : -1;
-    s_len[q] = in ? A.S.len[r] : 0;
-    s_base[q] = in ? A.S.sptr[r >> 5] + (r & 31) : 0;
-  }
-  __syncthreads();
   const double tol2 = A.cs->tol2;
   const int maxit = A.cs->maxit;
   double absnew = A.cs->absnew, beta = 0.0, alpha = 0.0, rr = 0.0;
@@ -1357,53 +1551,15 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs
     const double *pold = A.p[cur];
     double *pnew = A.p[cur ^ 1];
     // phase A: q = L p on the owned SELL blocks, one group per block
-    for (int b = b0 + g; b < b1; b += kCgResGroups) {
-      const int lp = (b - b0) * kBlock + lt;
-      const int i = s_row[lp];
+    const auto pj = [&](int j) { return fly ? __ldcg(A.z + j) + beta * __ldcg(pold + j) : __ldcg(pold + j); };
+    rows.fill(pj);
+    for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+      const int lp = (b - rows.b0) * kBlock + lt;
+      const int i = rows.row_of(lp);
       double v[1] = {0.0};
       if (i >= 0) {
-        const int base = s_base[lp], len = s_len[lp];
-        const bool staged = b < bs;
-        double acc = 0.0;
-        int k = 0;
-        for (; k + kCgChunk <= len; k += kCgChunk) {
-          int jj[kCgChunk];
-          double a[kCgChunk], po[kCgChunk], zz[kCgChunk];
-#pragma unroll
-          for (int u = 0; u < kCgChunk; ++u) {
-            const int pos = base + (k + u) * kSellC;
-            jj[u] = staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-            a[u] = __ldg(A.Ls + pos);
-          }
-#pragma unroll
-          for (int u = 0; u < kCgChunk; ++u) {
-            po[u] = __ldcg(pold + jj[u]);
-            zz[u] = fly ? __ldcg(A.z + jj[u]) : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < kCgChunk; ++u) acc += a[u] * (fly ? zz[u] + beta * po[u] : po[u]);
-        }
-        if (k < len) {  // the last len % kCgChunk entries as one predicated chunk
-          int jj[kCgChunk];
-          double a[kCgChunk], po[kCgChunk], zz[kCgChunk];
-#pragma unroll
-          for (int u = 0; u < kCgChunk; ++u) {
-            const int pos = base + (k + u) * kSellC;
-            const bool in = k + u < len;
-            jj[u] = !in ? 0 : staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-            a[u] = in ? __ldg(A.Ls + pos) : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < kCgChunk; ++u) {
-            const bool in = k + u < len;
-            po[u] = in ? __ldcg(pold + jj[u]) : 0.0;
-            zz[u] = (in && fly) ? __ldcg(A.z + jj[u]) : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < kCgChunk; ++u)
-            if (k + u < len) acc += a[u] * (fly ? zz[u] + beta * po[u] : po[u]);
-        }
-        const double pi = fly ? __ldcg(A.z + i) + beta * __ldcg(pold + i) : __ldcg(pold + i);
+        const double acc = rows.product(b, lp, pj);
+        const double pi = pj(i);
         __stcg(pnew + i, pi);
         __stcg(A.q + i, acc);
         v[0] = pi * acc;
@@ -1483,8 +1639,9 @@ struct Cg1Args {
   double *p;                   // zero on entry
 };
 
+template <bool WIN>
 __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
-  extern __shared__ int s_dyn[];
+  extern __shared__ double s_dbl[];
   __shared__ double s_grp[kCgResGroups][3][kBlock / 32];
   __shared__ double s_tree[3][kBlock / 32];
   const CgResidentArgs &R = C.R;
@@ -1493,44 +1650,21 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
   if (!A.cs->active) return;
   unsigned int phase = 0;
   const int g = threadIdx.x / kBlock, lt = threadIdx.x & (kBlock - 1);
-  const int b0 = min(A.nblk_sell, (int)blockIdx.x * R.bpc_sell);
-  const int b1 = min(A.nblk_sell, b0 + R.bpc_sell);
-  int *s_row = s_dyn;
-  int *s_len = s_row + R.bpc_sell * kBlock;
-  int *s_base = s_len + R.bpc_sell * kBlock;
-  int *s_col = s_base + R.bpc_sell * kBlock;
-  const int e0 = (b0 < b1) ? A.S.sptr[8 * b0] : 0;
-  int bs = b0;
-  while (bs < b1 && A.S.sptr[min(8 * (bs + 1), R.nslices)] - e0 <= R.col_cap) ++bs;
-  const int e1 = (bs > b0) ? A.S.sptr[min(8 * bs, R.nslices)] : e0;
-  for (int e = e0 + (int)threadIdx.x; e < e1; e += kCgResThreads) s_col[e - e0] = A.S.col[e];
-  for (int q = threadIdx.x; q < (b1 - b0) * kBlock; q += kCgResThreads) {
-    const int r = b0 * kBlock + q;
-    const bool in = r < A.S.nrows_pad;
-    s_row[q] = in ? A.S.perm[r] : -1;
-    s_len[q] = in ? A.S.len[r] : 0;
-    s_base[q] = in ? A.S.sptr[r >> 5] + (r & 31) : 0;
-  }
-  __syncthreads();
+  ResidentRows<double, WIN> rows(R, A.Ls, reinterpret_cast<char *>(s_dbl));
   const double tol2 = A.cs->tol2;
   const int maxit = A.cs->maxit;
   double gamma = A.cs->absnew, alpha = 0.0, beta = 0.0, rn2 = A.cs->bnorm2;
   int it = 0, status = KS_RUNNING, cur = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[1] += 1;
   // start: w = A u0, delta = w.u0
-  for (int b = b0 + g; b < b1; b += kCgResGroups) {
-    const int lp = (b - b0) * kBlock + lt;
-    const int i = s_row[lp];
+  const auto u0 = [&](int j) { return __ldcg(C.u0 + j); };
+  rows.fill(u0);
+  for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+    const int lp = (b - rows.b0) * kBlock + lt;
+    const int i = rows.row_of(lp);
     double v[1] = {0.0};
     if (i >= 0) {
-      const int base = s_base[lp], len = s_len[lp];
-      const bool staged = b < bs;
-      double acc = 0.0;
-      for (int k = 0; k < len; ++k) {
-        const int pos = base + k * kSellC;
-        const int jj = staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-        acc += __ldg(A.Ls + pos) * __ldcg(C.u0 + jj);
-      }
+      const double acc = rows.product(b, lp, u0);
       __stcg(C.w[0] + i, acc);
       v[0] = acc * __ldcg(C.u0 + i);
     }
@@ -1551,70 +1685,33 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
     double *part = (it & 1) ? A.part_a : A.part_b;
     const double *ro = C.r[cur], *wo = C.w[cur], *so = C.s[cur];
     double *rn = C.r[cur ^ 1], *wn = C.w[cur ^ 1], *sn = C.s[cur ^ 1];
-    for (int b = b0 + g; b < b1; b += kCgResGroups) {
-      const int lp = (b - b0) * kBlock + lt;
-      const int i = s_row[lp];
+    const auto uj = [&](int j) {
+      const double sj = __ldcg(wo + j) + beta * __ldcg(so + j);
+      const double rj = __ldcg(ro + j) - alpha * sj;
+      return __ldg(A.invL + j) * rj;
+    };
+    int i = -1;
+    double mi = 0.0, roi = 0.0, woi = 0.0, soi = 0.0, poi = 0.0, xoi = 0.0, uoi = 0.0;
+    auto own = [&](int b) {
+      i = (b < rows.b1) ? rows.row_of((b - rows.b0) * kBlock + lt) : -1;
+      if (i < 0) return;
+      roi = __ldcg(ro + i);
+      woi = __ldcg(wo + i);
+      soi = __ldcg(so + i);
+      poi = __ldcg(C.p + i);
+      xoi = __ldcg(A.x + i);
+      mi = __ldg(A.invL + i);
+      uoi = (it == 0) ? __ldcg(C.u0 + i) : mi * roi;
+    };
+    own(rows.b0 + g);
+    rows.fill(uj);
+    for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
       double v[3] = {0.0, 0.0, 0.0};
       if (i >= 0) {
-        const int base = s_base[lp], len = s_len[lp];
-        const bool staged = b < bs;
-        double acc = 0.0;
-        int k = 0;
-        for (; k + kCgChunk <= len; k += kCgChunk) {
-          int jj[kCgChunk];
-          double a[kCgChunk], rr_[kCgChunk], ww[kCgChunk], ss[kCgChunk], mm[kCgChunk];
-#pragma unroll
-          for (int q = 0; q < kCgChunk; ++q) {
-            const int pos = base + (k + q) * kSellC;
-            jj[q] = staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-            a[q] = __ldg(A.Ls + pos);
-          }
-#pragma unroll
-          for (int q = 0; q < kCgChunk; ++q) {
-            rr_[q] = __ldcg(ro + jj[q]);
-            ww[q] = __ldcg(wo + jj[q]);
-            ss[q] = __ldcg(so + jj[q]);
-            mm[q] = __ldg(A.invL + jj[q]);
-          }
-#pragma unroll
-          for (int q = 0; q < kCgChunk; ++q) {
-            const double sj = ww[q] + beta * ss[q];
-            const double rj = rr_[q] - alpha * sj;
-            acc += a[q] * (mm[q] * rj);
-          }
-        }
-        if (k < len) {  // the last len % kCgChunk entries as one predicated chunk
-          int jj[kCgChunk];
-          double a[kCgChunk], rr_[kCgChunk], ww[kCgChunk], ss[kCgChunk], mm[kCgChunk];
-#pragma unroll
-          for (int q = 0; q < kCgChunk; ++q) {
-            const int pos = base + (k + q) * kSellC;
-            const bool in = k + q < len;
-            jj[q] = !in ? 0 : staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-            a[q] = in ? __ldg(A.Ls + pos) : 0.0;
-          }
-#pragma unroll
-          for (int q = 0; q < kCgChunk; ++q) {
-            const bool in = k + q < len;
-            rr_[q] = in ? __ldcg(ro + jj[q]) : 0.0;
-            ww[q] = in ? __ldcg(wo + jj[q]) : 0.0;
-            ss[q] = in ? __ldcg(so + jj[q]) : 0.0;
-            mm[q] = in ? __ldg(A.invL + jj[q]) : 0.0;
-          }
-#pragma unroll
-          for (int q = 0; q < kCgChunk; ++q) {
-            const double sj = ww[q] + beta * ss[q];
-            const double rj = rr_[q] - alpha * sj;
-            if (k + q < len) acc += a[q] * (mm[q] * rj);
-          }
-        }
-        // own row
-        const double mi = __ldg(A.invL + i);
-        const double roi = __ldcg(ro + i);
-        const double uoi = (it == 0) ? __ldcg(C.u0 + i) : mi * roi;
-        const double pi = uoi + beta * __ldcg(C.p + i);
-        const double si = __ldcg(wo + i) + beta * __ldcg(so + i);
-        const double xi = __ldcg(A.x + i) + alpha * pi;
+        const double acc = rows.product(b, (b - rows.b0) * kBlock + lt, uj);
+        const double pi = uoi + beta * poi;
+        const double si = woi + beta * soi;
+        const double xi = xoi + alpha * pi;
         const double ri = roi - alpha * si;
         const double ui = mi * ri;
         __stcg(C.p + i, pi);
@@ -1626,6 +1723,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
         v[1] = acc * ui;
         v[2] = ri * ri;
       }
+      own(b + kCgResGroups);
       group_partial<3>(v, part, b, g, s_grp);
     }
     if (!grid_sync(A.bar, phase)) return;
@@ -1719,10 +1817,6 @@ struct Cg2lArgs {
   // inverse diagonal, solution and the same vectors (r32[0] = b, p32 = s32[0] = 0 on entry)
   const float *Ls32, *invL32;
   float *x32, *r32[2], *w32[2], *s32[2], *p32;
-  // u = D^-1 r + c[agg] of the current residual, stored by the split form (k_cg2l_resident with
-  // SPLIT) between its two passes
-  double *u;
-  float *u32;
 };
 
 // floor(x 2^S) as a two's-complement 128-bit integer (lo, hi); x 2^S is clamped to +-2^100 and a
@@ -1820,16 +1914,11 @@ __device__ __forceinline__ void clear_acc(const CoarseView &V, int buf) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 9 * V.nc; k += gridDim.x * blockDim.x) g[k] = 0ull;
 }
 
-// Aggregate sums of vectors [v0, v0 + NV) from global buffer `buf`.
-template <int NV>
-__device__ __forceinline__ void read_sums(const CoarseView &V, int buf, int v0, double iscale,
-                                          double *const (&dst)[NV]) {
-  for (int idx = threadIdx.x; idx < NV * V.nc; idx += blockDim.x) {
-    const int v = idx / V.nc, m = idx - v * V.nc;
-    unsigned long long lo, hi;
-    words128(V.gacc + 3 * ((size_t)(3 * buf + v0 + v) * V.nc + m), lo, hi);
-    dst[v][m] = unfixed128(lo, hi, iscale);
-  }
+// Sum of vector v over aggregate m in global buffer `buf`.
+__device__ __forceinline__ double sum_value(const CoarseView &V, int buf, int v, int m, double iscale) {
+  unsigned long long lo, hi;
+  words128(V.gacc + 3 * ((size_t)(3 * buf + v) * V.nc + m), lo, hi);
+  return unfixed128(lo, hi, iscale);
 }
 
 // c[m] = Z[m] . t for the aggregates this CTA reads: one warp per aggregate, lane l adding
@@ -1858,17 +1947,13 @@ __device__ __forceinline__ void coarse_values(const CoarseView &V, const double 
   }
 }
 
-// Entries per chunk of the split form's product (one gather per entry, so twice the fused
-// form's chunk fits in the registers).
-constexpr int kCg2lChunk = 8;
-
 // TS: storage type of the operator values, inverse diagonal, solution and Krylov vectors. double:
 // the FP64 solve (bit-identical to the oracle's cg2l); float: the inner solve of the mixed-precision
 // pressure solve (half the bytes per entry). Arithmetic, dot products, aggregate sums and scalars
 // are FP64 in both; in the float form each updated vector entry is rounded to float once and the
 // rounded value is the one used in the dot products and aggregate sums, so they describe the
 // stored vectors.
-template <class TS, bool SPLIT>
+template <class TS, bool WIN>
 __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) {
   extern __shared__ double s_dbl[];
   __shared__ double s_grp[kCgResGroups][4][kBlock / 32];
@@ -1877,14 +1962,14 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
   const CgPersistentArgs &A = R.P;
   const CoarseView &V = C.V;
   constexpr bool f32 = std::is_same<TS, float>::value;
-  constexpr int kZB = f32 ? 8 : 16;  // 16 spills in the float form
+  constexpr int kZB = 16;
   const TS *Lsv, *invLv;
-  TS *xv, *pv, *uv, *rv0, *rv1, *wv0, *wv1, *sv0, *sv1;
+  TS *xv, *pv, *rv0, *rv1, *wv0, *wv1, *sv0, *sv1;
   if constexpr (f32) {
-    Lsv = C.Ls32, invLv = C.invL32, xv = C.x32, pv = C.p32, uv = C.u32;
+    Lsv = C.Ls32, invLv = C.invL32, xv = C.x32, pv = C.p32;
     rv0 = C.r32[0], rv1 = C.r32[1], wv0 = C.w32[0], wv1 = C.w32[1], sv0 = C.s32[0], sv1 = C.s32[1];
   } else {
-    Lsv = A.Ls, invLv = A.invL, xv = A.x, pv = C.p, uv = C.u;
+    Lsv = A.Ls, invLv = A.invL, xv = A.x, pv = C.p;
     rv0 = C.r[0], rv1 = C.r[1], wv0 = C.w[0], wv1 = C.w[1], sv0 = C.s[0], sv1 = C.s[1];
   }
   auto rnd = [](double v) { return (double)(TS)v; };  // storage rounding (identity for double)
@@ -1892,31 +1977,14 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
   if (!A.cs->active) return;
   unsigned int phase = 0;
   const int g = threadIdx.x / kBlock, lt = threadIdx.x & (kBlock - 1);
-  const int b0 = min(A.nblk_sell, (int)blockIdx.x * R.bpc_sell);
-  const int b1 = min(A.nblk_sell, b0 + R.bpc_sell);
   const int nc = V.nc, n = A.n;
-  // shared memory: aggregate sums of r, w, s, the coarse input t, coarse values (two
-  // generations, entry nc = 0 for rows without aggregate), the aggregate-sorted staging of two
-  // row vectors, then the row staging of k_cg1_resident
-  double *cR = s_dbl, *cW = cR + nc, *cS = cW + nc, *ct = cS + nc;
+  // shared memory: aggregate sums of s, the coarse input t, coarse values (two generations, entry
+  // nc = 0 for rows without aggregate), the aggregate-sorted staging of two row vectors, then the rows
+  double *cS = s_dbl, *ct = cS + nc;
   double *cc[2] = {ct + nc, ct + 2 * nc + 1};
   double *s_stage = ct + 3 * nc + 2;
-  int *s_row = reinterpret_cast<int *>(s_stage + 2 * V.npos_max);
-  int *s_len = s_row + R.bpc_sell * kBlock;
-  int *s_base = s_len + R.bpc_sell * kBlock;
-  int *s_col = s_base + R.bpc_sell * kBlock;
-  const int e0 = (b0 < b1) ? A.S.sptr[8 * b0] : 0;
-  int bs = b0;
-  while (bs < b1 && A.S.sptr[min(8 * (bs + 1), R.nslices)] - e0 <= R.col_cap) ++bs;
-  const int e1 = (bs > b0) ? A.S.sptr[min(8 * bs, R.nslices)] : e0;
-  for (int e = e0 + (int)threadIdx.x; e < e1; e += kCgResThreads) s_col[e - e0] = A.S.col[e];
-  for (int q = threadIdx.x; q < (b1 - b0) * kBlock; q += kCgResThreads) {
-    const int r = b0 * kBlock + q;
-    const bool in = r < A.S.nrows_pad;
-    s_row[q] = in ? A.S.perm[r] : -1;
-    s_len[q] = in ? A.S.len[r] : 0;
-    s_base[q] = in ? A.S.sptr[r >> 5] + (r & 31) : 0;
-  }
+  ResidentRows<TS, WIN> rows(R, Lsv, reinterpret_cast<char *>(s_stage + 2 * V.npos_max));
+  const int b0 = rows.b0, b1 = rows.b1;
   for (int m = threadIdx.x; m <= nc; m += kCgResThreads) {
     cc[0][m] = 0.0;
     cc[1][m] = 0.0;
@@ -1939,6 +2007,12 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
   int it = 0, status = KS_RUNNING, cur = 0, pc = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[1] += 1;
   const TS *bvec = rv0;
+  // T(r) of the next residual, from T(r) and T(w) of the last one (T(s) by recurrence)
+  auto coarse_input = [&](int m, double r_m, double w_m) {
+    const double sm = w_m + beta * cS[m];
+    cS[m] = sm;
+    ct[m] = r_m - alpha * sm;
+  };
   const int v_r[1] = {0}, v_w[1] = {1}, v_rw[2] = {0, 1};
   // start: c0 = Z T(b) (phase 0, buffer 0)
   if (nc > 0) {
@@ -1949,27 +2023,22 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     __syncthreads();
     seg_sums<1>(V, s_stage, 0, v_r, scale);
     if (!grid_sync(A.bar, phase)) return;
-    double *const dR[1] = {cR};
-    read_sums<1>(V, 0, 0, iscale, dR);
+    for (int m = threadIdx.x; m < nc; m += kCgResThreads) ct[m] = sum_value(V, 0, 0, m, iscale);
     __syncthreads();
-    coarse_values<kZB>(V, cR, cc[0]);
+    coarse_values<kZB>(V, ct, cc[0]);
     __syncthreads();
   }
   // phase 1 (buffer 1): w0 = A u0 with u0 = D^-1 b + c0[agg]; delta0 = w0.u0, gamma0 = b.u0
+  const auto u0 = [&](int j) {
+    return (double)__ldg(invLv + j) * (double)__ldcg(bvec + j) + cc[0][__ldg(V.agg + j)];
+  };
+  rows.fill(u0);
   for (int b = b0 + g; b < b1; b += kCgResGroups) {
     const int lp = (b - b0) * kBlock + lt;
-    const int i = s_row[lp];
+    const int i = rows.row_of(lp);
     double v[2] = {0.0, 0.0};
     if (i >= 0) {
-      const int base = s_base[lp], len = s_len[lp];
-      const bool staged = b < bs;
-      double acc = 0.0;
-      for (int k = 0; k < len; ++k) {
-        const int pos = base + k * kSellC;
-        const int jj = staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-        const double uj = (double)__ldg(invLv + jj) * (double)__ldcg(bvec + jj) + cc[0][__ldg(V.agg + jj)];
-        acc += (double)__ldg(Lsv + pos) * uj;
-      }
+      double acc = rows.product(b, lp, u0);
       acc = rnd(acc);
       const double bi = (double)__ldcg(bvec + i);
       const double ui = (double)__ldg(invLv + i) * bi + cc[0][__ldg(V.agg + i)];
@@ -1996,204 +2065,69 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     else
       alpha = d0[1] / d0[0];
     gamma = d0[1];
-    if (nc > 0) {
-      double *const dW[1] = {cW};
-      read_sums<1>(V, 1, 1, iscale, dW);
-      __syncthreads();
-    }
+    for (int m = threadIdx.x; m < nc; m += kCgResThreads) coarse_input(m, ct[m], sum_value(V, 1, 1, m, iscale));
   }
   while (status == KS_RUNNING) {
     double *part = (it & 1) ? A.part_a : A.part_b;
     const int buf = (it + 2) % 3;  // phase it + 2
     const TS *ro = cur ? rv1 : rv0, *wo = cur ? wv1 : wv0, *so = cur ? sv1 : sv0;
     TS *rn = cur ? rv0 : rv1, *wn = cur ? wv0 : wv1, *sn = cur ? sv0 : sv1;
-    // coarse input of the new residual and its coarse values
+    // coarse values of the new residual
     if (nc > 0) {
       clear_acc(V, (it + 3) % 3);  // buffer of the next phase; last read before the previous barrier
-      for (int m = threadIdx.x; m < nc; m += kCgResThreads) {
-        const double sm = cW[m] + beta * cS[m];  // T(s) of the new s, by recurrence
-        cS[m] = sm;
-        ct[m] = cR[m] - alpha * sm;
-      }
       __syncthreads();
       coarse_values<kZB>(V, ct, cc[pc ^ 1]);
       __syncthreads();
     }
     const double *cold = cc[pc], *cnew = cc[pc ^ 1];
-    if constexpr (SPLIT) {
-      // pass 1: own-row updates and u = D^-1 r_new + c_new[agg]; slots 0-2 take r.u, r.r, r.D^-1 r
-      for (int b = b0 + g; b < b1; b += kCgResGroups) {
-        const int lp = (b - b0) * kBlock + lt;
-        const int i = s_row[lp];
-        double v[3] = {0.0, 0.0, 0.0};
-        if (i >= 0) {
-          const int ai = __ldg(V.agg + i);
-          const double mi = (double)__ldg(invLv + i);
-          const double roi = (double)__ldcg(ro + i);
-          const double woi = (double)__ldcg(wo + i), soi = (double)__ldcg(so + i);
-          const double poi = (double)__ldcg(pv + i), xoi = (double)__ldcg(xv + i);
-          const double uoi = mi * roi + cold[ai];
-          const double pi = rnd(uoi + beta * poi);
-          const double si = rnd(woi + beta * soi);
-          const double xi = xoi + alpha * pi;
-          const double ri = rnd(roi - alpha * si);
-          const double ui = rnd(mi * ri + cnew[ai]);
-          __stcg(pv + i, (TS)pi);
-          __stcg(sn + i, (TS)si);
-          __stcg(xv + i, (TS)xi);
-          __stcg(rn + i, (TS)ri);
-          __stcg(uv + i, (TS)ui);
-          v[0] = ri * ui;
-          v[1] = ri * ri;
-          v[2] = ri * (mi * ri);
-          if (nc > 0) {
-            const int ps = __ldg(V.row_pos + i);
-            if (ps >= 0) s_stage[ps] = ri;
-          }
+    const auto uj = [&](int j) {
+      const double sj = (double)__ldcg(wo + j) + beta * (double)__ldcg(so + j);
+      const double rj = (double)__ldcg(ro + j) - alpha * sj;
+      return (double)__ldg(invLv + j) * rj + cnew[__ldg(V.agg + j)];
+    };
+    // the own row's entries are requested ahead of the window's, so that they arrive with it
+    int i = -1, ai = 0, ps = -1;
+    double mi = 0.0, roi = 0.0, woi = 0.0, soi = 0.0, poi = 0.0, xoi = 0.0;
+    auto own = [&](int b) {
+      i = (b < b1) ? rows.row_of((b - b0) * kBlock + lt) : -1;
+      if (i < 0) return;
+      roi = (double)__ldcg(ro + i);
+      woi = (double)__ldcg(wo + i);
+      soi = (double)__ldcg(so + i);
+      poi = (double)__ldcg(pv + i);
+      xoi = (double)__ldcg(xv + i);
+      mi = (double)__ldg(invLv + i);
+      ai = __ldg(V.agg + i);
+      if (nc > 0) ps = __ldg(V.row_pos + i);
+    };
+    own(b0 + g);
+    rows.fill(uj);
+    for (int b = b0 + g; b < b1; b += kCgResGroups) {
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+      if (i >= 0) {
+        const double acc = rnd(rows.product(b, (b - b0) * kBlock + lt, uj));
+        const double uoi = mi * roi + cold[ai];
+        const double pi = rnd(uoi + beta * poi);
+        const double si = rnd(woi + beta * soi);
+        const double xi = xoi + alpha * pi;
+        const double ri = rnd(roi - alpha * si);
+        const double ui = mi * ri + cnew[ai];
+        __stcg(pv + i, (TS)pi);
+        __stcg(sn + i, (TS)si);
+        __stcg(xv + i, (TS)xi);
+        __stcg(rn + i, (TS)ri);
+        __stcg(wn + i, (TS)acc);
+        v[0] = ri * ui;
+        v[1] = acc * ui;
+        v[2] = ri * ri;
+        v[3] = ri * (mi * ri);
+        if (ps >= 0) {
+          s_stage[ps] = ri;
+          s_stage[V.npos_max + ps] = acc;
         }
-        group_partial<3>(v, part, b, g, s_grp);
       }
-      if (!grid_sync(A.bar, phase)) return;
-      // pass 2: w = A u (one gather per entry); slot 3 takes w.u
-      for (int b = b0 + g; b < b1; b += kCgResGroups) {
-        const int lp = (b - b0) * kBlock + lt;
-        const int i = s_row[lp];
-        double v[1] = {0.0};
-        if (i >= 0) {
-          const int base = s_base[lp], len = s_len[lp];
-          const bool staged = b < bs;
-          double acc = 0.0;
-          int k = 0;
-          for (; k + kCg2lChunk <= len; k += kCg2lChunk) {
-            int jj[kCg2lChunk];
-            double a[kCg2lChunk], uu[kCg2lChunk];
-#pragma unroll
-            for (int q = 0; q < kCg2lChunk; ++q) {
-              const int pos = base + (k + q) * kSellC;
-              jj[q] = staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-              a[q] = (double)__ldg(Lsv + pos);
-            }
-#pragma unroll
-            for (int q = 0; q < kCg2lChunk; ++q) uu[q] = (double)__ldcg(uv + jj[q]);
-#pragma unroll
-            for (int q = 0; q < kCg2lChunk; ++q) acc += a[q] * uu[q];
-          }
-          if (k < len) {  // the last len % kCg2lChunk entries as one predicated chunk
-            int jj[kCg2lChunk];
-            double a[kCg2lChunk], uu[kCg2lChunk];
-#pragma unroll
-            for (int q = 0; q < kCg2lChunk; ++q) {
-              const int pos = base + (k + q) * kSellC;
-              const bool in = k + q < len;
-              jj[q] = !in ? 0 : staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-              a[q] = in ? (double)__ldg(Lsv + pos) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < kCg2lChunk; ++q) uu[q] = (k + q < len) ? (double)__ldcg(uv + jj[q]) : 0.0;
-#pragma unroll
-            for (int q = 0; q < kCg2lChunk; ++q)
-              if (k + q < len) acc += a[q] * uu[q];
-          }
-          acc = rnd(acc);
-          __stcg(wn + i, (TS)acc);
-          v[0] = acc * (double)__ldcg(uv + i);
-          if (nc > 0) {
-            const int ps = __ldg(V.row_pos + i);
-            if (ps >= 0) s_stage[V.npos_max + ps] = acc;
-          }
-        }
-        group_partial<1>(v, part, b, g, s_grp, 3);
-      }
-    } else {
-      for (int b = b0 + g; b < b1; b += kCgResGroups) {
-        const int lp = (b - b0) * kBlock + lt;
-        const int i = s_row[lp];
-        double v[4] = {0.0, 0.0, 0.0, 0.0};
-        if (i >= 0) {
-          const int base = s_base[lp], len = s_len[lp];
-          const bool staged = b < bs;
-          double acc = 0.0;
-          int k = 0;
-          for (; k + kCgChunk <= len; k += kCgChunk) {
-            int jj[kCgChunk], aj[kCgChunk];
-            double a[kCgChunk], rr_[kCgChunk], ww[kCgChunk], ss[kCgChunk], mm[kCgChunk];
-  #pragma unroll
-            for (int q = 0; q < kCgChunk; ++q) {
-              const int pos = base + (k + q) * kSellC;
-              jj[q] = staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-              a[q] = (double)__ldg(Lsv + pos);
-            }
-  #pragma unroll
-            for (int q = 0; q < kCgChunk; ++q) {
-              rr_[q] = (double)__ldcg(ro + jj[q]);
-              ww[q] = (double)__ldcg(wo + jj[q]);
-              ss[q] = (double)__ldcg(so + jj[q]);
-              mm[q] = (double)__ldg(invLv + jj[q]);
-              aj[q] = __ldg(V.agg + jj[q]);
-            }
-  #pragma unroll
-            for (int q = 0; q < kCgChunk; ++q) {
-              const double sj = ww[q] + beta * ss[q];
-              const double rj = rr_[q] - alpha * sj;
-              acc += a[q] * (mm[q] * rj + cnew[aj[q]]);
-            }
-          }
-          if (k < len) {  // the last len % kCgChunk entries as one predicated chunk
-            int jj[kCgChunk], aj[kCgChunk];
-            double a[kCgChunk], rr_[kCgChunk], ww[kCgChunk], ss[kCgChunk], mm[kCgChunk];
-  #pragma unroll
-            for (int q = 0; q < kCgChunk; ++q) {
-              const int pos = base + (k + q) * kSellC;
-              const bool in = k + q < len;
-              jj[q] = !in ? 0 : staged ? s_col[pos - e0] : __ldg(A.S.col + pos);
-              a[q] = in ? (double)__ldg(Lsv + pos) : 0.0;
-            }
-  #pragma unroll
-            for (int q = 0; q < kCgChunk; ++q) {
-              const bool in = k + q < len;
-              rr_[q] = in ? (double)__ldcg(ro + jj[q]) : 0.0;
-              ww[q] = in ? (double)__ldcg(wo + jj[q]) : 0.0;
-              ss[q] = in ? (double)__ldcg(so + jj[q]) : 0.0;
-              mm[q] = in ? (double)__ldg(invLv + jj[q]) : 0.0;
-              aj[q] = in ? __ldg(V.agg + jj[q]) : 0;
-            }
-  #pragma unroll
-            for (int q = 0; q < kCgChunk; ++q) {
-              const double sj = ww[q] + beta * ss[q];
-              const double rj = rr_[q] - alpha * sj;
-              if (k + q < len) acc += a[q] * (mm[q] * rj + cnew[aj[q]]);
-            }
-          }
-          acc = rnd(acc);
-          // own row
-          const int ai = __ldg(V.agg + i);
-          const double mi = (double)__ldg(invLv + i);
-          const double roi = (double)__ldcg(ro + i);
-          const double uoi = mi * roi + cold[ai];
-          const double pi = rnd(uoi + beta * (double)__ldcg(pv + i));
-          const double si = rnd((double)__ldcg(wo + i) + beta * (double)__ldcg(so + i));
-          const double xi = (double)__ldcg(xv + i) + alpha * pi;
-          const double ri = rnd(roi - alpha * si);
-          const double ui = mi * ri + cnew[ai];
-          __stcg(pv + i, (TS)pi);
-          __stcg(sn + i, (TS)si);
-          __stcg(xv + i, (TS)xi);
-          __stcg(rn + i, (TS)ri);
-          __stcg(wn + i, (TS)acc);
-          v[0] = ri * ui;
-          v[1] = acc * ui;
-          v[2] = ri * ri;
-          v[3] = ri * (mi * ri);
-          if (nc > 0) {
-            const int ps = __ldg(V.row_pos + i);
-            if (ps >= 0) {
-              s_stage[ps] = ri;
-              s_stage[V.npos_max + ps] = acc;
-            }
-          }
-        }
-        group_partial<4>(v, part, b, g, s_grp);
-      }
+      own(b + kCgResGroups);
+      group_partial<4>(v, part, b, g, s_grp);
     }
     if (nc > 0) {
       __syncthreads();
@@ -2202,17 +2136,6 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     if (!grid_sync(A.bar, phase)) return;
     double t[4];
     tree_total_cta<4>(part, A.nblk_sell, t, s_tree);
-    if constexpr (SPLIT) {  // slots r.u, r.r, r.D^-1 r, w.u -> r.u, w.u, r.r, r.D^-1 r
-      const double wu = t[3];
-      t[3] = t[2];
-      t[2] = t[1];
-      t[1] = wu;
-    }
-    if (nc > 0) {
-      double *const d2[2] = {cR, cW};
-      read_sums<2>(V, buf, 0, iscale, d2);
-      __syncthreads();
-    }
     ++it;
     pc ^= 1;
     rn2 = A.scaled ? t[3] : t[2];
@@ -2238,6 +2161,8 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     alpha = t[0] / den;
     beta = beta_new;
     gamma = t[0];
+    for (int m = threadIdx.x; m < nc; m += kCgResThreads)
+      coarse_input(m, sum_value(V, buf, 0, m, iscale), sum_value(V, buf, 1, m, iscale));
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     CgState *c = A.cs;

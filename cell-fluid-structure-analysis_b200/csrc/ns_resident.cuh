@@ -574,35 +574,51 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve3(BicgArgs A, ResidentArgs R
   if (blockIdx.x == 0 && threadIdx.x == 0) *A.bs = s;
 }
 
-// Pressure BiCGSTAB, one right-hand side. The operator and the vectors are L2-resident and an SM owns
-// only a few rows per thread, so a barrier costs more than extra gathers: p and s are not stored before
-// the products, each gathering thread forms them from r, p, v (r, v) with the owner's expression, which
-// leaves three barriers per iteration. p and v are double-buffered, since neighbours still read the old
-// ones while a row writes its new ones.
+// Pressure BiCGSTAB, one right-hand side, on the rows and windows of the resident CG kernels. The
+// operator and the vectors are L2-resident and an SM owns only a few rows per thread, so a barrier costs
+// more than reading a vector twice: p and s are not stored before the products but formed from r, p, v
+// (r, v) where a product reads them, with the owner's expression, which leaves three barriers per
+// iteration. p and v are double-buffered, since neighbours still read the old ones while a row writes
+// its new ones; the block partials alternate between two buffers.
 struct PBicgArgs {
   BicgArgs B;
+  CgResidentArgs R;
   double *p2, *v2;  // second buffers of p and v
 };
 
-template <int T, int U>
-__global__ void __launch_bounds__(T, 1) k_bicg_solve1(PBicgArgs P, ResidentArgs R) {
-  extern __shared__ double s_slots[];
+template <bool WIN>
+__global__ void __launch_bounds__(kCgResThreads, 1) k_bicg_resident(PBicgArgs P) {
+  extern __shared__ double s_dbl[];
+  __shared__ double s_grp[kCgResGroups][2][kBlock / 32];
+  __shared__ double s_tree[2][kBlock / 32];
   __shared__ BicgState s;
   const BicgArgs &A = P.B;
+  const CgPersistentArgs &C = P.R.P;
   if (A.st && A.st->halt) return;
   if (threadIdx.x == 0) s = *A.bs;
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.st) A.st->body_runs[A.slot] += 1;
   __syncthreads();
-  Resident<T> G(R, s_slots);
+  if (!s.active) return;
+  unsigned int phase = 0, nred = 0;
+  const int g = threadIdx.x / kBlock, lt = threadIdx.x & (kBlock - 1);
+  ResidentRows<double, WIN> rows(P.R, A.At, reinterpret_cast<char *>(s_dbl));
+  const int c0 = min(C.nblk_nat, (int)blockIdx.x * P.R.bpc_nat), c1 = min(C.nblk_nat, c0 + P.R.bpc_nat);
   int active = s.active, cur = 0;
   while (active) {
     const double *po = cur ? P.p2 : A.pk, *vo = cur ? P.v2 : A.v;
     double *pn = cur ? A.pk : P.p2, *vn = cur ? A.v : P.v2;
     const bool restart = s.restart != 0;
     if (restart) {
-      G.template rows<1>(A.S, [&](int r, int i, double (&part)[1]) { part[0] = bicg_restart_row(A, pn, 0, r, i); });
+      double *part = (nred++ & 1) ? C.part_b : C.part_a;
+      for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+        const int lp = (b - rows.b0) * kBlock + lt, i = rows.row_of(lp);
+        double v[1] = {0.0};
+        if (i >= 0) v[0] = bicg_restart_row(A, pn, 0, rows.b0 * kBlock + lp, i);
+        group_partial<1>(v, part, b, g, s_grp);
+      }
+      if (!grid_sync(C.bar, phase)) return;
       double t[1];
-      if (!G.template reduce<1>(t)) return;
+      tree_total_cta<1>(part, C.nblk_sell, t, s_tree);
       if (threadIdx.x == 0) {
         s.rho[0] = s.r0norm2[0] = t[0];
         s.restart = 0;
@@ -611,58 +627,72 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve1(PBicgArgs P, ResidentArgs 
     }
     // p = r + beta (p - omega v), v = At p, alpha = rho / (r0 . v)
     const double be = s.beta[0], om0 = s.omega[0];
-    if (restart) {
-      G.template products<1, 1, 2 * U, 1>(A.S, A.At, double(), [&](int, int j) { return pn[j]; },
-                                          [&](int, int i) { return A.r0[i]; },
-                                          [&](int i, const double *acc, const double *own, double (&part)[1]) {
-        vn[i] = acc[0];
-        part[0] = own[0] * acc[0];
-      });
-    } else {
-      const auto pj = [&](int, int j) { return A.r[j] + be * (po[j] - om0 * vo[j]); };
-      G.template products<1, 1, U, 1>(A.S, A.At, double(), pj, pj,
-                                      [&](int i, const double *acc, const double *own, double (&part)[1]) {
-        pn[i] = own[0];
-        vn[i] = acc[0];
-        part[0] = A.r0[i] * acc[0];
-      });
-    }
     {
+      double *part = (nred++ & 1) ? C.part_b : C.part_a;
+      const auto pj = [&](int j) { return restart ? pn[j] : A.r[j] + be * (po[j] - om0 * vo[j]); };
+      rows.fill(pj);
+      for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+        const int lp = (b - rows.b0) * kBlock + lt, i = rows.row_of(lp);
+        double v[1] = {0.0};
+        if (i >= 0) {
+          const double acc = rows.product(b, lp, pj);
+          if (!restart) pn[i] = pj(i);
+          vn[i] = acc;
+          v[0] = A.r0[i] * acc;
+        }
+        group_partial<1>(v, part, b, g, s_grp);
+      }
+      if (!grid_sync(C.bar, phase)) return;
       double t[1];
-      if (!G.template reduce<1>(t)) return;
+      tree_total_cta<1>(part, C.nblk_sell, t, s_tree);
       active = each_component<1>(active, &s.active, [&](int) { return bicg_after_v(s, 0, t[0]); });
     }
     if (!active) break;
     // s = r - alpha v, t = At s, omega = (t . s) / (t . t)
     const double al = s.alpha[0];
-    const auto sj = [&](int, int j) { return A.r[j] - al * vn[j]; };
-    G.template products<2, 1, 2 * U, 1>(A.S, A.At, double(), sj, sj,
-                                        [&](int i, const double *acc, const double *own, double (&part)[2]) {
-      A.t[i] = acc[0];
-      part[0] = acc[0] * acc[0];
-      part[1] = acc[0] * own[0];
-    });
     {
+      double *part = (nred++ & 1) ? C.part_b : C.part_a;
+      const auto sj = [&](int j) { return A.r[j] - al * vn[j]; };
+      rows.fill(sj);
+      for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+        const int lp = (b - rows.b0) * kBlock + lt, i = rows.row_of(lp);
+        double v[2] = {0.0, 0.0};
+        if (i >= 0) {
+          const double acc = rows.product(b, lp, sj);
+          A.t[i] = acc;
+          v[0] = acc * acc;
+          v[1] = acc * sj(i);
+        }
+        group_partial<2>(v, part, b, g, s_grp);
+      }
+      if (!grid_sync(C.bar, phase)) return;
       double t[2];
-      if (!G.template reduce<2>(t)) return;
+      tree_total_cta<2>(part, C.nblk_sell, t, s_tree);
       each_component<1>(active, &s.active, [&](int) { return bicg_after_t(s, 0, t[0], t[1]); });
     }
     // x += alpha D^-1 p + omega D^-1 s, r = s - omega t; convergence test and next beta
     const double om = s.omega[0];
-    G.template entries<2>(A.n, [&](int i, double (&part)[2]) {
-      const double dinv = A.invA[i];
-      const double w = A.cw ? A.cw[i] : 1.0;
-      const double si = A.r[i] - al * vn[i];
-      const double y = dinv * pn[i];
-      const double z = dinv * si;
-      A.x[i] = A.x[i] + (al * y + om * z);
-      const double ri = si - om * A.t[i];
-      A.r[i] = ri;
-      part[0] = (ri * ri) * w;
-      part[1] = A.r0[i] * ri;
-    });
+    double *part = (nred++ & 1) ? C.part_b : C.part_a;
+    for (int b = c0 + g; b < c1; b += kCgResGroups) {
+      const int i = b * kBlock + lt;
+      double v[2] = {0.0, 0.0};
+      if (i < A.n) {
+        const double dinv = A.invA[i];
+        const double w = A.cw ? A.cw[i] : 1.0;
+        const double si = A.r[i] - al * vn[i];
+        const double y = dinv * pn[i];
+        const double z = dinv * si;
+        A.x[i] = A.x[i] + (al * y + om * z);
+        const double ri = si - om * A.t[i];
+        A.r[i] = ri;
+        v[0] = (ri * ri) * w;
+        v[1] = A.r0[i] * ri;
+      }
+      group_partial<2>(v, part, b, g, s_grp);
+    }
+    if (!grid_sync(C.bar, phase)) return;
     double t[2];
-    if (!G.template reduce<2>(t)) return;
+    tree_total_cta<2>(part, C.nblk_nat, t, s_tree);
     active = each_component<1>(active, &s.active, [&](int) { return bicg_after_xr(s, 0, t[0], t[1]); });
     cur ^= 1;
   }

@@ -1,0 +1,62 @@
+"""Resident Krylov solves at the sizes where their partitions can go wrong, bit for bit against the
+oracle (same sums in the same order), and the pressure solvers with and without column windows."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+RHO, NU = 1060.0, 0.004
+
+
+def solver(cf, m, momentum, pressure, tol=1e-11):
+    s = cf.NavierStokesSolver()
+    s.setKrylovTolerances(tol, tol)
+    s.setMaxIterations(5000, 20000)
+    s.setMomentumSolver(momentum)
+    s.setPressureSolver(pressure)
+    s.setDt(0.01)
+    s.initialize(m, cf.Fluid(RHO, NU))
+    s.setMeanInletVelocity([0.5, 0.0, 0.0])
+    return s
+
+
+def mesh(cf, shape):
+    m = cf.Mesh.cylinder(30.0, 2.0, *shape) if len(shape) == 2 else cf.Mesh.structuredRectangularPrism(6.0, 2.0, 1.5, *shape)
+    m.setupBoundaryConditions((1.0, 0.0, 0.0), 1.0)
+    return m
+
+
+# rows of the momentum operator: below one 256-row block, on both sides of the one-CTA line (768
+# rows), few blocks, more blocks than SMs with a ragged last slice
+@pytest.mark.parametrize("shape", [(1, 2), (2, 5), (2, 6), (5, 3, 2), (9, 7, 3), (6, 40), (29, 17, 13)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("momentum", [0, 1], ids=["cg", "bicgstab"])
+def test_resident_solves_match_oracle(cf, po, shape, momentum):
+    m = mesh(cf, shape)
+    s = solver(cf, m, momentum, cf.KRYLOV_BICGSTAB)
+    o = po.Oracle(m.vertices(), m.tets())
+    o.set_fluid(RHO, NU)
+    o.set_params(dt=0.01, tol_mom=1e-11, tol_p=1e-11, maxit_mom=5000, maxit_p=20000, pressure_solver=0)
+    o.set_momentum_solver(1 if momentum == cf.KRYLOV_CG else 0)
+    o.initialize()
+    inlet = np.zeros((o.N2, 3))
+    inlet[:, 0] = 0.5
+    o.set_inlet(inlet)
+    for _ in range(2):
+        assert s.pisoStep() and o.piso_step() == 0
+    ref = o.state()
+    assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
+
+
+@pytest.mark.parametrize("shape", [(1, 2), (4, 9), (11, 9, 7), (8, 60)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("pressure", [0, 1, 2, 3], ids=["cg", "bicgstab", "cg1", "cg2l"])
+def test_windows_do_not_change_the_bits(cf, monkeypatch, shape, pressure):
+    m = mesh(cf, shape)
+    got = []
+    for off in ("0", "1"):
+        monkeypatch.setenv("CFSA_NO_WINDOWS", off)
+        s = solver(cf, m, cf.KRYLOV_CG, pressure)
+        assert s.pisoSteps(2) == (True, 2)
+        got.append((s.getVelocity(), s.getPressure(), s.stats()["pressure_iters"]))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    assert got[0][2] == got[1][2] > 0
