@@ -6,6 +6,7 @@
 // loop continues, so a step (or a batch of steps) runs with no host round trip.
 #include "cfsa_ns.h"
 #include "ns_adjoint.cuh"
+#include "ns_coarse.cuh"
 #include "ns_kernels.cuh"
 #include "ns_mixed.cuh"
 #include "ns_resident.cuh"
@@ -114,6 +115,25 @@ struct PinnedSet {
   }
 };
 
+// Device buffers of the two-level coarse space; they only grow.
+struct CoarseBuffers {
+  unsigned long long *key = nullptr, *gacc = nullptr;
+  int *first = nullptr, *id = nullptr, *slot = nullptr, *agg = nullptr, *rows = nullptr, *row_pos = nullptr,
+      *scal = nullptr, *list = nullptr, *cnt = nullptr, *ptr = nullptr, *npieces = nullptr, *need = nullptr,
+      *nneed = nullptr;
+  double *bounds = nullptr, *A = nullptr, *T = nullptr, *Z = nullptr;
+  int4 *pieces = nullptr;
+  size_t cap_key = 0, cap_gacc = 0, cap_first = 0, cap_id = 0, cap_slot = 0, cap_agg = 0, cap_rows = 0, cap_pos = 0,
+         cap_scal = 0, cap_list = 0, cap_cnt = 0, cap_ptr = 0, cap_npieces = 0, cap_need = 0, cap_nneed = 0,
+         cap_bounds = 0, cap_A = 0, cap_T = 0, cap_Z = 0, cap_pieces = 0;
+  ~CoarseBuffers() {
+    for (void *p : {(void *)key, (void *)gacc, (void *)first, (void *)id, (void *)slot, (void *)agg, (void *)rows,
+                    (void *)row_pos, (void *)scal, (void *)list, (void *)cnt, (void *)ptr, (void *)npieces,
+                    (void *)need, (void *)nneed, (void *)bounds, (void *)A, (void *)T, (void *)Z, (void *)pieces})
+      cudaFree(p);
+  }
+};
+
 }  // namespace
 
 struct cfsa_ns {
@@ -215,7 +235,7 @@ struct cfsa_ns {
   int coarse_target = 256;
   bool coarse_dirty = true;
   int coarse_nc = 0;
-  std::vector<void *> coarse_allocs;
+  CoarseBuffers coarse_buf;
   CoarseView coarse_view{};
   CgResidentArgs cg2l_caps{};
   size_t cg2l_smem = 0;
@@ -302,7 +322,6 @@ struct cfsa_ns {
       if (e) cudaEventDestroy(e);
     if (adj_exec) cudaGraphExecDestroy(adj_exec);
     for (void *ptr : rec_allocs) cudaFree(ptr);
-    for (void *ptr : coarse_allocs) cudaFree(ptr);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (graph) cudaGraphDestroy(graph);
     for (void *ptr : allocs) cudaFree(ptr);
@@ -764,66 +783,83 @@ struct cfsa_ns {
   }
 
   // ------------------------------------------------------------------ two-level preconditioner
-  // Coarse space of k_cg2l_resident: geometric aggregates over the vertices without a penalty
-  // row, Z = (P^T L P)^-1 by Cholesky, and the index lists of the aggregate sums. Every step of
-  // the construction is fixed in order (the oracle's build_coarse follows the same steps), so the
-  // device and oracle solves agree bit for bit.
+  // Coarse space of k_cg2l_resident (ns_coarse.cuh): geometric aggregates over the vertices without a
+  // penalty row, Z = (P^T L P)^-1 by Cholesky, and the lists of the aggregate sums.
   //   box edge h_k = e c^k, e the largest extent of the bounding box of the unpenalised vertices,
   //   c = 2^-1/4, k in [0, 64] the smallest exponent (bisection) with >= coarse_target occupied
   //   boxes; boxes numbered by first vertex; an A_c that is not SPD disables the coarse part.
+  // The buffers stay with the handle and only grow, so a rebuild of the same size keeps the captured
+  // step graph.
   template <class T>
-  T *cupload(const std::vector<T> &h) {
-    void *ptr = nullptr;
-    CK(cudaMalloc(&ptr, std::max<size_t>(h.size(), 1) * sizeof(T)));
-    coarse_allocs.push_back(ptr);
-    if (!h.empty()) CK(cudaMemcpyAsync(ptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
-    return static_cast<T *>(ptr);
+  void coarse_grow(T *&p, size_t &cap, size_t n) {
+    if (n <= cap) return;
+    CK(cudaStreamSynchronize(stream));
+    if (p) {
+      CK(cudaFree(p));
+      p = nullptr;
+      cap = 0;
+    }
+    CK(cudaMalloc(&p, n * sizeof(T)));
+    cap = n;
   }
 
-  static int count_boxes(const std::vector<double> &xyz, const std::vector<char> &pen, int64_t n,
-                         double h, const double lo[3], std::vector<int64_t> *keys_out) {
-    std::vector<int64_t> keys;
-    keys.reserve(n);
-    for (int64_t i = 0; i < n; ++i) {
-      if (pen[i]) continue;
-      const int64_t ix = (int64_t)std::floor((xyz[3 * i] - lo[0]) / h);
-      const int64_t iy = (int64_t)std::floor((xyz[3 * i + 1] - lo[1]) / h);
-      const int64_t iz = (int64_t)std::floor((xyz[3 * i + 2] - lo[2]) / h);
-      keys.push_back((ix * 2097152 + iy) * 2097152 + iz);
-    }
-    if (keys_out) *keys_out = keys;
-    std::sort(keys.begin(), keys.end());
-    return (int)(std::unique(keys.begin(), keys.end()) - keys.begin());
+  // Enters the boxes of edge h into the hash table and returns their number.
+  int occupied_boxes(BoxArgs &a, double h) {
+    a.h = h;
+    CK(cudaMemsetAsync(a.key, 0xff, (size_t)(a.mask + 1) * sizeof(unsigned long long), stream));
+    CK(cudaMemsetAsync(a.first, 0x7f, (size_t)(a.mask + 1) * sizeof(int), stream));
+    CK(cudaMemsetAsync(a.count, 0, sizeof(int), stream));
+    k_box_insert<<<blocks_for(nv), kBlock, 0, stream>>>(a);
+    CK(cudaGetLastError());
+    int n = 0;
+    CK(cudaMemcpyAsync(&n, a.count, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    return n;
   }
 
   void build_coarse() {
     NvtxRange nvtx_("cfsa two-level coarse space");
+    const int n = (int)nv;
+    CoarseBuffers &B = coarse_buf;
+    unsigned int table = 64;
+    while (table < 2 * (unsigned int)n) table *= 2;
+    coarse_grow(B.key, B.cap_key, table);
+    coarse_grow(B.first, B.cap_first, table);
+    coarse_grow(B.id, B.cap_id, table);
+    for (auto &v : {std::make_pair(&B.slot, &B.cap_slot), std::make_pair(&B.agg, &B.cap_agg),
+                    std::make_pair(&B.rows, &B.cap_rows), std::make_pair(&B.row_pos, &B.cap_pos)})
+      coarse_grow(*v.first, *v.second, (size_t)n);
+    coarse_grow(B.scal, B.cap_scal, (size_t)4);
+    const int nb = 64;
+    coarse_grow(B.bounds, B.cap_bounds, (size_t)6 * nb);
+    BoxArgs a{};
+    a.n = n;
+    a.outlet_type = outlet_type;
+    a.ref_node = ref_node;
+    a.xyz = xyz;
+    a.bc = bc;
+    a.key = B.key;
+    a.mask = table - 1;
+    a.first = B.first;
+    a.slot = B.slot;
+    a.count = B.scal;
+    k_box_bounds<<<nb, kBlock, 0, stream>>>(a, B.bounds);
+    CK(cudaGetLastError());
+    std::vector<double> bb((size_t)6 * nb);
+    CK(cudaMemcpyAsync(bb.data(), B.bounds, bb.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    for (void *q : coarse_allocs) CK(cudaFree(q));
-    coarse_allocs.clear();
-    const int64_t n = nv;
-    std::vector<char> pen(n, 0);
-    if (outlet_type == CFSA_OUTLET_NEUMANN) {
-      if (ref_node >= 0 && ref_node < n) pen[ref_node] = 1;
-    } else if (outlet_type == CFSA_OUTLET_DIRICHLET) {
-      for (int64_t i = 0; i < n; ++i) pen[i] = h_bc[i] == BC_OUTLET;
-    }
-    std::vector<int> agg(n, 0);
-    int nc = 0;
-    double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-    bool any = false;
-    for (int64_t i = 0; i < n; ++i) {
-      if (pen[i]) continue;
-      for (int d = 0; d < 3; ++d) {
-        const double x = h_xyz[3 * i + d];
-        if (!any) lo[d] = hi[d] = x;
-        lo[d] = std::min(lo[d], x);
-        hi[d] = std::max(hi[d], x);
+    double hi[3];
+    for (int d = 0; d < 3; ++d) {
+      a.lo[d] = bb[d];
+      hi[d] = bb[3 + d];
+      for (int q = 1; q < nb; ++q) {
+        a.lo[d] = std::min(a.lo[d], bb[6 * q + d]);
+        hi[d] = std::max(hi[d], bb[6 * q + 3 + d]);
       }
-      any = true;
     }
-    const double e = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
-    if (any && e > 0.0 && coarse_target >= 1) {
+    const double e = std::max(hi[0] - a.lo[0], std::max(hi[1] - a.lo[1], hi[2] - a.lo[2]));
+    int nc = 0;
+    if (e > 0.0 && coarse_target >= 1) {  // e < 0: no unpenalised vertex
       auto h_of = [&](int k) {
         double h = e;
         for (int q = 0; q < k; ++q) h = h * 0.8408964152537145;  // 2^-1/4
@@ -832,154 +868,86 @@ struct cfsa_ns {
       int klo = 0, khi = 64;
       while (klo < khi) {
         const int km = (klo + khi) / 2;
-        if (count_boxes(h_xyz, pen, n, h_of(km), lo, nullptr) >= coarse_target)
+        if (occupied_boxes(a, h_of(km)) >= coarse_target)
           khi = km;
         else
           klo = km + 1;
       }
-      std::vector<int64_t> keys;
-      count_boxes(h_xyz, pen, n, h_of(klo), lo, &keys);
-      // number the boxes by their first vertex
-      std::vector<std::pair<int64_t, int>> kv(keys.size());
-      for (size_t q = 0; q < keys.size(); ++q) kv[q] = {keys[q], (int)q};
-      std::stable_sort(kv.begin(), kv.end(), [](const std::pair<int64_t, int> &a, const std::pair<int64_t, int> &b) {
-        return a.first < b.first;
-      });
-      std::vector<std::pair<int, int>> firsts;  // (first vertex rank, start in kv)
-      for (size_t q = 0; q < kv.size();) {
-        size_t r = q;
-        while (r < kv.size() && kv[r].first == kv[q].first) ++r;
-        firsts.push_back({kv[q].second, (int)q});
-        q = r;
-      }
-      std::sort(firsts.begin(), firsts.end());
-      std::vector<int> id_sorted(kv.size()), id_of(keys.size());
-      for (size_t gq = 0; gq < firsts.size(); ++gq) {
-        size_t q = firsts[gq].second;
-        const int64_t key = kv[q].first;
-        while (q < kv.size() && kv[q].first == key) id_sorted[q++] = (int)gq;
-      }
-      for (size_t q = 0; q < kv.size(); ++q) id_of[kv[q].second] = id_sorted[q];
-      nc = (int)firsts.size();
-      size_t q = 0;
-      for (int64_t i = 0; i < n; ++i) agg[i] = pen[i] ? nc : id_of[q++];
+      nc = occupied_boxes(a, h_of(klo));
     }
-    std::vector<double> Z;
+    const int pieces_max = cg_res_bpc_sell * kBlock / kSegPiece + std::min(nc, cg_res_bpc_sell * kBlock);
     if (nc > 0) {
-      // A_c = P^T L P over the unpenalised rows (the penalties sit on penalised rows only)
-      std::vector<int> ci((size_t)nnz1);
-      std::vector<double> lv((size_t)nnz1);
-      CK(cudaMemcpyAsync(ci.data(), ci1, (size_t)nnz1 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-      CK(cudaMemcpyAsync(lv.data(), Lv, (size_t)nnz1 * sizeof(double), cudaMemcpyDeviceToHost, stream));
+      const size_t nn = (size_t)nc * nc;
+      coarse_grow(B.list, B.cap_list, (size_t)nc);
+      coarse_grow(B.cnt, B.cap_cnt, (size_t)nc);
+      coarse_grow(B.ptr, B.cap_ptr, (size_t)nc + 1);
+      coarse_grow(B.A, B.cap_A, nn);
+      coarse_grow(B.T, B.cap_T, nn);
+      coarse_grow(B.Z, B.cap_Z, nn);
+      coarse_grow(B.gacc, B.cap_gacc, (size_t)27 * nc);
+      coarse_grow(B.pieces, B.cap_pieces, (size_t)cg_res_grid * pieces_max);
+      coarse_grow(B.npieces, B.cap_npieces, (size_t)cg_res_grid);
+      coarse_grow(B.need, B.cap_need, (size_t)cg_res_grid * nc);
+      coarse_grow(B.nneed, B.cap_nneed, (size_t)cg_res_grid);
+      CK(cudaMemsetAsync(B.scal + 1, 0, sizeof(int), stream));
+      CK(cudaMemsetAsync(B.scal + 2, 1, sizeof(int), stream));
+      CK(cudaMemsetAsync(B.cnt, 0, (size_t)nc * sizeof(int), stream));
+      k_box_collect<<<blocks_for(n), kBlock, 0, stream>>>(n, B.slot, B.first, B.scal + 1, B.list);
+      k_box_number<<<blocks_for(nc), kBlock, 0, stream>>>(nc, B.list, B.slot, B.id);
+      k_box_assign<<<blocks_for(n), kBlock, 0, stream>>>(n, nc, B.slot, B.id, B.agg, B.cnt);
+      k_prefix<<<1, 32, 0, stream>>>(nc, B.cnt, B.ptr);
+      k_agg_rows<<<nc, kBlock, 0, stream>>>(n, B.agg, B.ptr, B.rows);
+      k_coarse_matrix<<<nc, 512, 0, stream>>>(nc, B.ptr, B.rows, rp1, ci1, Lv, B.agg, B.A);
+      for (int j0 = 0; j0 < nc; j0 += kPanel) {
+        const unsigned int g = (unsigned int)((nc - j0 + kPanel - 1) / kPanel);
+        if (j0 > 0) k_chol_update<<<g, 1024, 0, stream>>>(nc, j0, B.A);
+        k_chol_panel<<<g, 32, 0, stream>>>(nc, j0, B.A, B.scal + 2);
+      }
+      CK(cudaGetLastError());
+      int spd = 0;
+      CK(cudaMemcpyAsync(&spd, B.scal + 2, sizeof(int), cudaMemcpyDeviceToHost, stream));
+      const dim3 tiles((nc + 31) / 32, (nc + 31) / 32);
+      k_transpose<<<tiles, kBlock, 0, stream>>>(nc, B.A, B.T);
+      CK(cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nc * sizeof(double))));
+      k_coarse_inverse<<<nc, 512, nc * sizeof(double), stream>>>(nc, B.T, B.A);
+      k_coarse_z<<<dim3((nc + 31) / 32, (nc + 7) / 8), kBlock, 0, stream>>>(nc, B.A, B.Z);
+      CoarseListArgs l{};
+      l.n = n;
+      l.nc = nc;
+      l.bpc = cg_res_bpc_sell;
+      l.rp = rp1;
+      l.ci = ci1;
+      l.agg = B.agg;
+      l.row_pos = B.row_pos;
+      l.pieces = B.pieces;
+      l.npieces = B.npieces;
+      l.piece_stride = pieces_max;
+      l.need = B.need;
+      l.nneed = B.nneed;
+      l.need_stride = nc;
+      const size_t list_smem = ((size_t)cg_res_bpc_sell * kBlock + 2 * (size_t)nc + (nc + 31) / 32) * sizeof(int);
+      CK(cudaFuncSetAttribute(k_coarse_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem));
+      k_coarse_lists<<<cg_res_grid, 1024, list_smem, stream>>>(l);
+      CK(cudaGetLastError());
       CK(cudaStreamSynchronize(stream));
-      std::vector<double> Ac((size_t)nc * nc, 0.0), G((size_t)nc * nc, 0.0), Gi((size_t)nc * nc, 0.0);
-      for (int64_t i = 0; i < n; ++i) {
-        if (agg[i] >= nc) continue;
-        for (int k = h_rp1[i]; k < h_rp1[i + 1]; ++k) {
-          const int j = ci[k];
-          if (agg[j] >= nc) continue;
-          double &a = Ac[(size_t)agg[i] * nc + agg[j]];
-          a = a + lv[k];
-        }
-      }
-      bool spd = true;
-      for (int i = 0; i < nc && spd; ++i)
-        for (int j = 0; j <= i; ++j) {
-          double sum = Ac[(size_t)i * nc + j];
-          for (int k = 0; k < j; ++k) sum = sum - G[(size_t)i * nc + k] * G[(size_t)j * nc + k];
-          if (i == j) {
-            if (!(sum > 0.0)) {
-              spd = false;
-              break;
-            }
-            G[(size_t)i * nc + i] = std::sqrt(sum);
-          } else {
-            G[(size_t)i * nc + j] = sum / G[(size_t)j * nc + j];
-          }
-        }
-      if (!spd) {
-        nc = 0;
-        std::fill(agg.begin(), agg.end(), 0);
-      } else {
-        for (int j = 0; j < nc; ++j) {
-          Gi[(size_t)j * nc + j] = 1.0 / G[(size_t)j * nc + j];
-          for (int i = j + 1; i < nc; ++i) {
-            double sum = 0.0;
-            for (int k = j; k < i; ++k) sum = sum - G[(size_t)i * nc + k] * Gi[(size_t)k * nc + j];
-            Gi[(size_t)i * nc + j] = sum / G[(size_t)i * nc + i];
-          }
-        }
-        Z.assign((size_t)nc * nc, 0.0);
-        for (int m = 0; m < nc; ++m)
-          for (int k = 0; k < nc; ++k) {
-            double sum = 0.0;
-            for (int q = std::max(m, k); q < nc; ++q) sum = sum + Gi[(size_t)q * nc + m] * Gi[(size_t)q * nc + k];
-            Z[(size_t)m * nc + k] = sum;
-          }
-      }
+      if (!spd) nc = 0;
     }
-    // per CTA: its rows sorted by aggregate (staging positions, one segment per aggregate) and
-    // the aggregates of its rows' columns (coarse values it reads)
-    const int nblk_sell = (int)blocks_for(s1.nrows_pad);
-    std::vector<int> row_pos(n, -1), own_ptr(cg_res_grid + 1, 0), own, seg_lo, seg_hi,
-        need_ptr(cg_res_grid + 1, 0), need;
-    int npos_max = 0;
-    if (nc > 0) {
-      std::vector<int> ci((size_t)nnz1);
-      CK(cudaMemcpyAsync(ci.data(), ci1, (size_t)nnz1 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-      CK(cudaStreamSynchronize(stream));
-      for (int c = 0; c < cg_res_grid; ++c) {
-        const int b0 = std::min(nblk_sell, c * cg_res_bpc_sell), b1 = std::min(nblk_sell, b0 + cg_res_bpc_sell);
-        const int64_t r0 = (int64_t)kBlock * b0, r1 = std::min<int64_t>(n, (int64_t)kBlock * b1);
-        std::vector<std::pair<int, int>> rows;  // (aggregate, row)
-        std::vector<int> mn;
-        for (int64_t i = r0; i < r1; ++i) {
-          if (agg[i] < nc) rows.push_back({agg[i], (int)i});
-          for (int k = h_rp1[i]; k < h_rp1[i + 1]; ++k)
-            if (agg[ci[k]] < nc) mn.push_back(agg[ci[k]]);
-        }
-        std::sort(rows.begin(), rows.end());
-        for (size_t q = 0; q < rows.size(); ++q) {
-          row_pos[rows[q].second] = (int)q;
-          if (q == 0 || rows[q].first != rows[q - 1].first) {
-            own.push_back(rows[q].first);
-            seg_lo.push_back((int)q);
-            seg_hi.push_back((int)q);
-            mn.push_back(rows[q].first);
-          }
-          seg_hi.back() = (int)q + 1;
-        }
-        own_ptr[c + 1] = (int)own.size();
-        std::sort(mn.begin(), mn.end());
-        mn.erase(std::unique(mn.begin(), mn.end()), mn.end());
-        need.insert(need.end(), mn.begin(), mn.end());
-        need_ptr[c + 1] = (int)need.size();
-        npos_max = std::max(npos_max, (int)rows.size());
-      }
-    }
-    // pieces of kSegPiece staging positions per segment, in segment order (seg_sums)
-    std::vector<int> own_pfirst(own.size() + 1, 0);
-    std::vector<int4> pieces;
-    for (size_t q = 0; q < own.size(); ++q) {
-      own_pfirst[q] = (int)pieces.size();
-      for (int a0 = seg_lo[q]; a0 < seg_hi[q]; a0 += kSegPiece)
-        pieces.push_back(make_int4(a0, std::min(seg_hi[q], a0 + kSegPiece), own[q], 0));
-    }
-    own_pfirst[own.size()] = (int)pieces.size();
+    if (nc == 0) CK(cudaMemsetAsync(B.agg, 0, (size_t)n * sizeof(int), stream));
     CoarseView V{};
     V.nc = nc;
-    V.agg = cupload(agg);
-    V.Z = cupload(Z);
-    V.row_pos = cupload(row_pos);
-    V.own_ptr = cupload(own_ptr);
-    V.own = cupload(own);
-    V.seg_lo = cupload(seg_lo);
-    V.seg_hi = cupload(seg_hi);
-    V.own_pfirst = cupload(own_pfirst);
-    V.pieces = cupload(pieces);
-    V.need_ptr = cupload(need_ptr);
-    V.need = cupload(need);
-    V.gacc = cupload(std::vector<unsigned long long>((size_t)27 * std::max(nc, 1), 0ull));
+    V.agg = B.agg;
+    if (nc > 0) {
+      V.Z = B.Z;
+      V.row_pos = B.row_pos;
+      V.pieces = B.pieces;
+      V.npieces = B.npieces;
+      V.piece_stride = pieces_max;
+      V.need = B.need;
+      V.nneed = B.nneed;
+      V.need_stride = nc;
+      V.gacc = B.gacc;
+    }
+    const int npos_max = nc > 0 ? cg_res_bpc_sell * kBlock : 0;
     V.npos_max = npos_max;
     // shared memory: coarse arrays, then the rows
     const void *const kernels[] = {(const void *)k_cg2l_resident<double, true>, (const void *)k_cg2l_resident<double, false>,
@@ -1001,11 +969,11 @@ struct cfsa_ns {
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kCgResThreads, cg2l_smem));
       if (o < 1) throw CudaError{"two-level pressure preconditioner: kernel does not fit on an SM"};
     }
-    CK(cudaStreamSynchronize(stream));
+    // the view is a captured launch argument; the shared-memory layout follows from it
+    if (std::memcmp(&V, &coarse_view, sizeof(V)) != 0) graph_dirty = true;
     coarse_view = V;
     coarse_nc = nc;
     coarse_dirty = false;
-    graph_dirty = true;
   }
 
   // ------------------------------------------------------------------ Krylov loops

@@ -1799,11 +1799,10 @@ struct CoarseView {
   const double *Z;              // [nc*nc] (P^T A P)^-1, symmetric
   const int *row_pos;           // [n] position of the row in its CTA's aggregate-sorted staging
                                 // order, -1 for rows without aggregate
-  const int *own_ptr, *own;     // aggregates of each CTA's rows (ascending)
-  const int *seg_lo, *seg_hi;   // staging positions of each own aggregate's rows
-  const int *own_pfirst;        // [own entries + 1] first piece of each own aggregate's segment
-  const int4 *pieces;           // (first, end staging position, aggregate, 0) per piece
-  const int *need_ptr, *need;   // aggregates whose coarse value each CTA reads
+  const int4 *pieces;           // per CTA piece_stride of (first, end staging position, aggregate, 0):
+  const int *npieces;           // the segments of its rows' aggregates in pieces of kSegPiece positions
+  const int *need, *nneed;      // per CTA need_stride aggregates whose coarse value it reads (ascending)
+  int piece_stride, need_stride;
   unsigned long long *gacc;     // [3 buffers][3 vectors][nc][3 words] fixed-point sums (red128)
   int npos_max;                 // largest staging list (shared-memory doubles per vector)
 };
@@ -1865,8 +1864,8 @@ __device__ __forceinline__ double unfixed128(unsigned long long lo, unsigned lon
 }
 
 // Sums of this CTA's staged values per own aggregate into global buffer `buf`. Each own
-// aggregate's segment of the staging is cut into pieces of kSegPiece positions (listed per CTA
-// on the host) and the warps take the CTA's pieces round robin, so a CTA whose rows fall into a
+// aggregate's segment of the staging is cut into pieces of kSegPiece positions (k_coarse_lists) and the
+// warps take the CTA's pieces round robin, so a CTA whose rows fall into a
 // few large aggregates still spreads the work over all its warps. In a piece each lane adds its
 // values exactly as 128-bit integers offset by 2^100 (so that they are non-negative); the lane sums
 // are cut into five 26-bit limbs, each limb summed by a warp reduction (32 x 2^26 < 2^32), and
@@ -1876,10 +1875,9 @@ template <int NV>
 __device__ __forceinline__ void seg_sums(const CoarseView &V, const double *__restrict__ stage,
                                          int buf, const int (&vi)[NV], double scale) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int g0 = __ldg(V.own_pfirst + __ldg(V.own_ptr + blockIdx.x));
-  const int g1 = __ldg(V.own_pfirst + __ldg(V.own_ptr + blockIdx.x + 1));
-  for (int gp = g0 + warp; gp < g1; gp += nw) {
-    const int4 pc = __ldg(V.pieces + gp);  // x = first, y = end position, z = aggregate
+  const int np = __ldg(V.npieces + blockIdx.x);
+  for (int gp = warp; gp < np; gp += nw) {
+    const int4 pc = __ldg(V.pieces + (size_t)blockIdx.x * V.piece_stride + gp);  // x = first, y = end position, z = aggregate
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       const double *sv = stage + (size_t)v * V.npos_max;
@@ -1928,10 +1926,10 @@ template <int ZB>
 __device__ __forceinline__ void coarse_values(const CoarseView &V, const double *__restrict__ t,
                                               double *__restrict__ c) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int q0 = __ldg(V.need_ptr + blockIdx.x), q1 = __ldg(V.need_ptr + blockIdx.x + 1);
+  const int nq = __ldg(V.nneed + blockIdx.x);
   const int nc = V.nc;
-  for (int q = q0 + warp; q < q1; q += nw) {
-    const int m = __ldg(V.need + q);
+  for (int q = warp; q < nq; q += nw) {
+    const int m = __ldg(V.need + (size_t)blockIdx.x * V.need_stride + q);
     const double *zr = V.Z + (size_t)m * nc;
     double sum = 0.0;
     for (int k0 = lane; k0 < nc; k0 += 32 * ZB) {

@@ -60,3 +60,35 @@ def test_windows_do_not_change_the_bits(cf, monkeypatch, shape, pressure):
         got.append((s.getVelocity(), s.getPressure(), s.stats()["pressure_iters"]))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
     assert got[0][2] == got[1][2] > 0
+
+
+# aggregates: one, a partial panel, several 32-column panels, more than one CTA's worth of columns,
+# more boxes asked for than there are vertices
+@pytest.mark.parametrize("target", [1, 31, 100, 700])
+@pytest.mark.parametrize("shape", [(2, 3), (6, 30)], ids=lambda s: "x".join(map(str, s)))
+def test_coarse_space_matches_oracle(cf, po, shape, target):
+    m = mesh(cf, shape)
+    s = solver(cf, m, cf.KRYLOV_CG, cf.KRYLOV_CG2L)
+    s.setCoarseTarget(target)
+    o = po.Oracle(m.vertices(), m.tets())
+    o.set_fluid(RHO, NU)
+    o.set_params(dt=0.01, tol_mom=1e-11, tol_p=1e-11, maxit_mom=5000, maxit_p=20000, pressure_solver=3)
+    o.set_momentum_solver(1)
+    o.set_coarse_target(target)
+    o.initialize()
+    inlet = np.zeros((o.N2, 3))
+    inlet[:, 0] = 0.5
+    o.set_inlet(inlet)
+    assert s.pisoStep() and o.piso_step() == 0
+    ref = o.state()
+    assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
+    # a rebuild on moved vertices and back leaves the same coarse space
+    x = m.vertices()
+    u, p = s.getVelocity().copy(), s.getPressure().copy()
+    s.updateVertices(x * [1.0, 1.01, 0.99])
+    s.coarseSize()
+    s.updateVertices(x)
+    s.setFields(u, p)
+    assert s.pisoStep() and o.piso_step() == 0
+    ref = o.state()
+    assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
