@@ -1068,18 +1068,20 @@ struct cfsa_ns {
     const int nblk = (int)blocks_for(S.nrows);
     return std::max(S.max_run, kSlicesPerBlock * ((nblk + S.nruns - 1) / S.nruns));
   }
-  // Two forms of each kernel: many threads with short chunks of a row in flight, or fewer threads with
-  // longer chunks. Rows to spare per thread hide the chunk's latency in the first form, a short run of
-  // rows wants it paid less often. Measured per momentum iteration, CG / BiCGSTAB, FP64, us:
-  //   rows        1024 threads, 4 entries   640 threads, 5 entries
-  //   144,499     48.8 /  84.6              37.4 /  74.8
-  //   355,395     66.2 / 119                59.9 / 121
-  //   696,987     110.5 / 213               108 / 228
+  // Three forms of each kernel, fewer threads with longer chunks of a row in flight the fewer rows there
+  // are: rows to spare per thread hide a chunk's latency, a short run of rows wants it paid less often.
+  // Measured per momentum iteration, CG / BiCGSTAB, FP64, us:
+  //   rows        1024 threads, 4 entries   640 threads, 5 entries   256 threads, 8 entries
+  //   45,347      38.8 /  67.9              29.1 /  58.4             24.9 /  45.1
+  //   144,499     48.8 /  84.6              37.4 /  74.8             42.1 /  77.9
+  //   355,395     66.2 / 119                59.9 / 121               79.0 / 147
+  //   696,987     110.5 / 213               108 / 228                151 / 304
   //   1,378,515   182 (CG)                  193 (CG)
-  static constexpr int kFewRows = 450000;
+  static constexpr int kFewRows = 90000, kManyRows = 450000;
 #define CFSA_RESIDENT(kernel, args, S, s, ...)                                                              \
-  ((S).nrows < kFewRows ? launch_resident(kernel<640, 5 __VA_OPT__(, 6)>, 640, args, S, s)                 \
-                        : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
+  ((S).nrows < kFewRows    ? launch_resident(kernel<256, 8 __VA_OPT__(, 8)>, 256, args, S, s)              \
+   : (S).nrows < kManyRows ? launch_resident(kernel<640, 5 __VA_OPT__(, 6)>, 640, args, S, s)              \
+                           : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
   template <class Args>
   void launch_resident(void (*kernel)(Args, ResidentArgs), int threads, const Args &a, const Sell &S, cudaStream_t s) {
     const int chunks = resident_chunks(S);

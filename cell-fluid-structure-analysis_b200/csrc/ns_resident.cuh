@@ -163,26 +163,62 @@ struct Resident {
     rev = !rev;
   }
 
-  // f(i, part) for every entry i < n of the CTA's natural blocks (NV = 0: f(i), no sums).
-  template <int NV, class F>
-  __device__ __forceinline__ void entries(int n, F &&f) {
+  // The CTA's natural blocks.
+  __device__ __forceinline__ void begin_entries(int n) {
     nchunk = (n + 31) / 32;
     const int nblk = (n + kBlock - 1) / kBlock;
     a0 = kSlicesPerBlock * (int)((int64_t)nblk * blockIdx.x / gridDim.x);
     na = min(kSlicesPerBlock * (int)((int64_t)nblk * (blockIdx.x + 1) / gridDim.x), nchunk) - a0;
     nc = 0;
+  }
+
+  // f(i, part) for every entry i < n of the CTA's natural blocks.
+  template <int NV, class F>
+  __device__ __forceinline__ void entries(int n, F &&f) {
+    begin_entries(n);
     for (int q = threadIdx.x >> 5; q < na; q += kWarps) {
       int slot;
       const int i = 32 * chunk(q, slot) + (int)(threadIdx.x & 31);
-      if constexpr (NV == 0) {
-        if (i < n) f(i);
-      } else {
-        double part[NV];
+      double part[NV];
 #pragma unroll
-        for (int j = 0; j < NV; ++j) part[j] = 0.0;
-        if (i < n) f(i, part);
-        chunk_sums<NV>(part, slot);
-      }
+      for (int j = 0; j < NV; ++j) part[j] = 0.0;
+      if (i < n) f(i, part);
+      chunk_sums<NV>(part, slot);
+    }
+    rev = !rev;
+  }
+
+  // f(i) for every entry i < n of the CTA's natural blocks.
+  template <class F>
+  __device__ __forceinline__ void each(int n, F &&f) {
+    begin_entries(n);
+    for (int q = threadIdx.x >> 5; q < na; q += kWarps) {
+      int slot;
+      const int i = 32 * chunk(q, slot) + (int)(threadIdx.x & 31);
+      if (i < n) f(i);
+    }
+    rev = !rev;
+  }
+
+  // Vector phase without sums: apply(i, load(i)) for every entry i < n of the CTA's natural blocks; with
+  // registers to spare, the loads of two chunks ahead of the stores of both (which may alias them for all
+  // the compiler knows; at 640 or 1024 threads the second set spills: 12.6 against 11.7 ms per 1M-tet solve).
+  template <class L, class F>
+  __device__ __forceinline__ void update(int n, L &&load, F &&apply) {
+    if constexpr (T > 256) {
+      each(n, [&](int i) { apply(i, load(i)); });
+      return;
+    }
+    begin_entries(n);
+    const int lane = threadIdx.x & 31;
+    for (int q = threadIdx.x >> 5; q < na; q += 2 * kWarps) {
+      int slot;
+      const int i = 32 * chunk(q, slot) + lane;
+      const bool two = q + kWarps < na;
+      const int i2 = two ? 32 * chunk(q + kWarps, slot) + lane : n;
+      const auto v = load(min(i, n - 1)), v2 = load(min(i2, n - 1));
+      if (i < n) apply(i, v);
+      if (i2 < n) apply(i2, v2);
     }
     rev = !rev;
   }
@@ -359,16 +395,24 @@ __global__ void __launch_bounds__(T, 1) k_mcg_solve(BicgArgs A, ResidentArgs R) 
       double be[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) be[c] = s.beta[c];
-      G.template entries<0>(A.n, [&](int i) {
-        const double dinv = A.invA[i];
-        double rv[3], pv[3];
+      struct V {
+        double dinv, r[3], p[3];
+      };
+      G.update(
+          A.n,
+          [&](int i) {
+            V v;
+            v.dinv = A.invA[i];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((active >> c) & 1) rv[c] = A.r[c * n + i], pv[c] = A.pk[c * n + i];
+            for (int c = 0; c < 3; ++c)
+              if ((active >> c) & 1) v.r[c] = A.r[c * n + i], v.p[c] = A.pk[c * n + i];
+            return v;
+          },
+          [&](int i, const V &v) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((active >> c) & 1) A.pk[c * n + i] = dinv * rv[c] + be[c] * pv[c];
-      });
+            for (int c = 0; c < 3; ++c)
+              if ((active >> c) & 1) A.pk[c * n + i] = v.dinv * v.r[c] + be[c] * v.p[c];
+          });
     }
     if (!G.sync()) return;
   }
@@ -456,18 +500,26 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve3(BicgArgs A, ResidentArgs R
 #pragma unroll
       for (int c = 0; c < 3; ++c) be[c] = s.beta[c], om[c] = s.omega[c];
       const int mask = active & ~restart;
-      G.template entries<0>(A.n, [&](int i) {
-        double rv[3], pv[3], vv[3];
+      struct V {
+        double r[3], p[3], v[3];
+      };
+      G.update(
+          A.n,
+          [&](int i) {
+            V x;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((mask >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          rv[c] = A.r[o], pv[c] = A.pk[o], vv[c] = A.v[o];
-        }
+            for (int c = 0; c < 3; ++c) {
+              if (!((mask >> c) & 1)) continue;
+              const int64_t o = c * n + i;
+              x.r[c] = A.r[o], x.p[c] = A.pk[o], x.v[c] = A.v[o];
+            }
+            return x;
+          },
+          [&](int i, const V &x) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((mask >> c) & 1) A.pk[c * n + i] = rv[c] + be[c] * (pv[c] - om[c] * vv[c]);
-      });
+            for (int c = 0; c < 3; ++c)
+              if ((mask >> c) & 1) A.pk[c * n + i] = x.r[c] + be[c] * (x.p[c] - om[c] * x.v[c]);
+          });
     }
     if (restart) {
       G.template rows<3>(A.S, [&](int r, int i, double (&part)[3]) {
@@ -510,15 +562,25 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve3(BicgArgs A, ResidentArgs R
     double al[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) al[c] = s.alpha[c];
-    G.template entries<0>(A.n, [&](int i) {
-      double rv[3], vv[3];
+    {
+      struct V {
+        double r[3], v[3];
+      };
+      G.update(
+          A.n,
+          [&](int i) {
+            V x;
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((active >> c) & 1) rv[c] = A.r[c * n + i], vv[c] = A.v[c * n + i];
+            for (int c = 0; c < 3; ++c)
+              if ((active >> c) & 1) x.r[c] = A.r[c * n + i], x.v[c] = A.v[c * n + i];
+            return x;
+          },
+          [&](int i, const V &x) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((active >> c) & 1) A.s[c * n + i] = rv[c] - al[c] * vv[c];
-    });
+            for (int c = 0; c < 3; ++c)
+              if ((active >> c) & 1) A.s[c * n + i] = x.r[c] - al[c] * x.v[c];
+          });
+    }
     if (!G.sync()) return;
     // t = At s, omega = (t . s) / (t . t)
     with_mask<3>(active, [&](auto mk) {
@@ -794,7 +856,7 @@ __global__ void __launch_bounds__(T, 1) k_mpc_solve(MixedArgs A, ResidentArgs R)
     const int upd = s.upd;
     if (upd) {
       // x += dx (FP64), dx = 0
-      G.template entries<0>(A.n, [&](int i) {
+      G.each(A.n, [&](int i) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           if (!((upd >> c) & 1)) continue;
@@ -862,7 +924,7 @@ __global__ void __launch_bounds__(T, 1) k_mpc_solve(MixedArgs A, ResidentArgs R)
       float be[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) be[c] = (float)s.beta[c];
-      G.template entries<0>(A.n, [&](int i) {
+      G.each(A.n, [&](int i) {
         const float dinv = A.invA32[i];
         float rv[3], pv[3];
 #pragma unroll
@@ -932,7 +994,7 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
         });
         if (threadIdx.x == 0) s.restart_next = 0;
       } else {
-        G.template entries<0>(A.n, [&](int i) {
+        G.each(A.n, [&](int i) {
           double part[3];
           row(i, part);
         });
@@ -976,7 +1038,7 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
     float al[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) al[c] = (float)s.alpha[c];
-    G.template entries<0>(A.n, [&](int i) {
+    G.each(A.n, [&](int i) {
       float rv[3], vv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
@@ -1068,7 +1130,7 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
     const int upd = s.upd, rst = s.restart;
     if (upd) {
       // x += dx (FP64), dx = 0, xs = diag(A) x
-      G.template entries<0>(A.n, [&](int i) {
+      G.each(A.n, [&](int i) {
         const double d = A.diagA[i];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
