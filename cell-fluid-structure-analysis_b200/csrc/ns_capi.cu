@@ -1832,9 +1832,21 @@ struct cfsa_ns {
   // it differs from the value taken at recording time.
   uint64_t adjoint_fingerprint() {
     uint64_t hsh = 1469598103934665603ull;
+    // FNV-1a over 8-byte words in four interleaved lanes (byte by byte, one multiply after another, the
+    // 8.5 MB of a 250k-tet inlet took 11 ms), the tail byte by byte
     auto mix = [&](const void *ptr, size_t nb) {
       const unsigned char *b = static_cast<const unsigned char *>(ptr);
-      for (size_t k = 0; k < nb; ++k) hsh = (hsh ^ b[k]) * 1099511628211ull;
+      uint64_t lane[4] = {hsh, hsh ^ 1, hsh ^ 2, hsh ^ 3};
+      size_t k = 0;
+      for (; k + 32 <= nb; k += 32)
+        for (int q = 0; q < 4; ++q) {
+          uint64_t w;
+          std::memcpy(&w, b + k + 8 * q, 8);
+          lane[q] = (lane[q] ^ w) * 1099511628211ull;
+          lane[q] ^= lane[q] >> 29;
+        }
+      for (int q = 0; q < 4; ++q) hsh = (hsh ^ lane[q]) * 1099511628211ull;
+      for (; k < nb; ++k) hsh = (hsh ^ b[k]) * 1099511628211ull;
     };
     const double d[] = {dt, tol_mom, tol_p, relax_u, relax_p, outlet_pressure, viscosity, density,
                         mixed_delta};
