@@ -1070,17 +1070,16 @@ struct cfsa_ns {
   }
   // Three forms of each kernel, fewer threads with longer chunks of a row in flight the fewer rows there
   // are: rows to spare per thread hide a chunk's latency, a short run of rows wants it paid less often.
-  // Measured per momentum iteration, CG / BiCGSTAB, FP64, us:
-  //   rows        1024 threads, 4 entries   640 threads, 5 entries   256 threads, 8 entries
-  //   45,347      38.8 /  67.9              29.1 /  58.4             24.9 /  45.1
-  //   144,499     48.8 /  84.6              37.4 /  74.8             42.1 /  77.9
-  //   355,395     66.2 / 119                59.9 / 121               79.0 / 147
-  //   696,987     110.5 / 213               108 / 228                151 / 304
-  //   1,378,515   182 (CG)                  193 (CG)
+  // Measured per momentum iteration, CG / BiCGSTAB, FP64, us (threads x entries per chunk):
+  //   rows        1024 x 4       512 x 8       256 x 8
+  //   45,347      38.8 /  67.9   26.7 / 53.1   24.9 /  45.1
+  //   144,499     43.1 /  85.9   32.3 / 61.7   42.1 /  77.9
+  //   355,395     61.3 / 110     56.1 / 106    79.0 / 147
+  //   696,987     104 / 215      112 / 234     151 / 304
   static constexpr int kFewRows = 90000, kManyRows = 450000;
 #define CFSA_RESIDENT(kernel, args, S, s, ...)                                                              \
   ((S).nrows < kFewRows    ? launch_resident(kernel<256, 8 __VA_OPT__(, 8)>, 256, args, S, s)              \
-   : (S).nrows < kManyRows ? launch_resident(kernel<640, 5 __VA_OPT__(, 6)>, 640, args, S, s)              \
+   : (S).nrows < kManyRows ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)             \
                            : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
   template <class Args>
   void launch_resident(void (*kernel)(Args, ResidentArgs), int threads, const Args &a, const Sell &S, cudaStream_t s) {
@@ -1229,11 +1228,11 @@ struct cfsa_ns {
     if (mom_krylov == CFSA_KRYLOV_CG) {
       k_mpc_init<<<strided(k_mpc_init, gp), kBlock, 0, stream>>>(a, tol_mom, maxit_mom, delta);
       CK(cudaGetLastError());
-      CFSA_RESIDENT(k_mpc_solve, a, s2, stream, 4);
+      CFSA_RESIDENT(k_mpc_solve, a, s2, stream, 8);
     } else {
       k_mp_init<<<strided(k_mp_init, gp), kBlock, 0, stream>>>(a, tol_mom, maxit_mom, delta);
       CK(cudaGetLastError());
-      CFSA_RESIDENT(k_mp_solve, a, s2, stream, 4);
+      CFSA_RESIDENT(k_mp_solve, a, s2, stream, 8);
     }
     k_mp_check<<<1, 1, 0, stream>>>(ms, s_out, bar_err);
     CK(cudaGetLastError());
@@ -2283,9 +2282,9 @@ struct cfsa_ns {
       a.p = fs;
       a.r0 = fs;
       a.v = ft;   // scratch output
-      CFSA_RESIDENT(k_mixed_product, (MixedProductArgs{a, 1}), s2, stream, 4);  // warm-up
+      CFSA_RESIDENT(k_mixed_product, (MixedProductArgs{a, 1}), s2, stream, 8);  // warm-up
       CK(cudaEventRecord(ev0, stream));
-      CFSA_RESIDENT(k_mixed_product, (MixedProductArgs{a, iters}), s2, stream, 4);
+      CFSA_RESIDENT(k_mixed_product, (MixedProductArgs{a, iters}), s2, stream, 8);
       CK(cudaEventRecord(ev1, stream));
       *alg_bytes = 8.0 * (double)nnz2 + 8.0 * s2.nrows_pad + 4.0 * (s2.nslices + 1) + 36.0 * (double)N2;
     } else if (which == CFSA_KERNEL_MOMENTUM_SPMV) {

@@ -107,12 +107,18 @@ struct Resident {
 
   // Row products of the CTA's run against NC right-hand sides: finish(i, acc, own, part) for every row
   // i, with acc[c] the row's product, own[c] = own(c, i) and part its NV sums. One thread per row adds
-  // its entries in ascending column order (as sell_spmv_row), in chunks of U: the gathers of a chunk
-  // are issued together with the next chunk's indices and values. load(c, j) reads entry j of x_c with
-  // a plain load, since other CTAs rewrite x between the phases of a launch.
+  // its entries in ascending column order (as sell_spmv_row), in chunks of U: indices and values, then
+  // the gathers, then the sums. Bound: L1 serves the gathers, about six cycles of the SM for 32 lanes
+  // spread over eleven lines (70% of its throughput at 415k tets, DRAM 39%). With one or two FP64
+  // components, and in the form for small meshes, the next chunk's indices and values are requested
+  // along with the gathers; with three, or in FP32, the registers that holds are worth more to longer chunks: three components at 1M tets 118
+  // against 139 us (577 MB, 4.9 TB/s), FP32 81 against 98 us; two components 95 against 100 us.
+  // load(c, j) reads entry j of x_c with a plain load, since other CTAs rewrite x between the phases of
+  // a launch.
   template <int NV, int NC, int U, int MASK, class TV, class TA, class L, class O, class F>
   __device__ __forceinline__ void products(const SellView &S, const TV *val, TA, L &&load, O &&own, F &&finish) {
     int *next = begin_rows(S);
+    constexpr bool kAhead = T <= 256 || (sizeof(TV) == 8 && !(NC == 3 && MASK == 7));
     const int lane = threadIdx.x & 31;
     for (int q = threadIdx.x >> 5; q < na + nc; q = run_next_slice(next)) {
       int slot;
@@ -145,14 +151,18 @@ struct Resident {
               if ((MASK >> c) & 1) xv[u][c] = (k + u < len) ? load(c, j[u]) : TA(0);
           int jn[U];
           TV an[U];
-          fetch(k + U, jn, an);
+          if constexpr (kAhead) fetch(k + U, jn, an);
 #pragma unroll
           for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int c = 0; c < NC; ++c)
               if (((MASK >> c) & 1) && k + u < len) acc[c] += a[u] * xv[u][c];
+          if constexpr (kAhead) {
 #pragma unroll
-          for (int u = 0; u < U; ++u) j[u] = jn[u], a[u] = an[u];
+            for (int u = 0; u < U; ++u) j[u] = jn[u], a[u] = an[u];
+          } else if (k + U < len) {
+            fetch(k + U, j, a);
+          }
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c) ov[c] = ((MASK >> c) & 1) ? own(c, i) : TA(0);
