@@ -748,9 +748,9 @@ struct cfsa_ns {
     NvtxRange nvtx_("cfsa assemble");
     ++geom_gen;
     k_geometry<<<blocks_for(nt), kBlock, 0, stream>>>((int)nt, xyz, tnode, vol, grad);
-    k_assemble_p2<<<blocks_for(N2), kBlock, 0, stream>>>((int)N2, (int)nt, density, 1.0 / viscosity,
+    k_assemble_p2<<<(unsigned int)((N2 + kAsmWarps - 1) / kAsmWarps), 32 * kAsmWarps, 0, stream>>>((int)N2, (int)nt, density, 1.0 / viscosity,
                                                          adj_ptr, adj, tnode, vol, grad, rp2, ci2, Mv, Kv);
-    k_assemble_p1<<<blocks_for(nv), kBlock, 0, stream>>>((int)nv, (int)nt, nnz1, adj_ptr, adj, tnode,
+    k_assemble_p1<<<(unsigned int)((nv + kAsmWarps - 1) / kAsmWarps), 32 * kAsmWarps, 0, stream>>>((int)nv, (int)nt, nnz1, adj_ptr, adj, tnode,
                                                          vol, grad, rp1, ci1, Gv, Lv);
     k_lumped_mass<<<blocks_for(N2), kBlock, 0, stream>>>((int)N2, rp2, Mv, invm);
     CK(cudaGetLastError());
@@ -1239,7 +1239,7 @@ struct cfsa_ns {
   }
 
   void enqueue_pressure_solve(bool capture) {
-    k_tet_div<<<blocks_for(nt), kBlock, 0, stream>>>((int)nt, N2, tnode, grad, ustar, divt, st);
+    k_tet_div<<<blocks_for(nt), kBlock, 0, stream>>>((int)nt, N2, tnode, vol, grad, ustar, divt, st);
     const PressureRhsArgs a = pressure_rhs_args(pc, st);
     k_pressure_rhs<<<blocks_for(nv), kBlock, 0, stream>>>(a);
     CK(cudaGetLastError());
@@ -1250,7 +1250,6 @@ struct cfsa_ns {
     PressureRhsArgs a{};
     a.adj_ptr = adj_ptr;
     a.adj = adj;
-    a.vol = vol;
     a.divt = divt;
     a.bc = bc;
     a.invL = invL;
@@ -2338,7 +2337,7 @@ struct cfsa_ns {
       float total = 0.f;
       int64_t its = 0;
       for (int k = 0; k < iters; ++k) {
-        k_tet_div<<<blocks_for(nt), kBlock, 0, stream>>>((int)nt, N2, tnode, grad, ustar, divt, st_free);
+        k_tet_div<<<blocks_for(nt), kBlock, 0, stream>>>((int)nt, N2, tnode, vol, grad, ustar, divt, st_free);
         const PressureRhsArgs a = pressure_rhs_args(pv, st_free);
         k_pressure_rhs<<<blocks_for(nv), kBlock, 0, stream>>>(a);
         CK(cudaEventRecord(ev0, stream));
@@ -2915,9 +2914,9 @@ int cfsa_ns_compute_divergence(cfsa_ns *h, const double *u, double *div) {
   if (!h || !u || !div) return CFSA_BAD_ARG;
   return guarded(h, [&] {
     h->upload_vec3(u, h->wb);
-    k_tet_div<<<blocks_for(h->nt), kBlock, 0, h->stream>>>((int)h->nt, h->N2, h->tnode, h->grad, h->wb,
+    k_tet_div<<<blocks_for(h->nt), kBlock, 0, h->stream>>>((int)h->nt, h->N2, h->tnode, h->vol, h->grad, h->wb,
                                                            h->divt, h->st_free);
-    k_gather_div<<<blocks_for(h->nv), kBlock, 0, h->stream>>>((int)h->nv, h->adj_ptr, h->adj, h->vol,
+    k_gather_div<<<blocks_for(h->nv), kBlock, 0, h->stream>>>((int)h->nv, h->adj_ptr, h->adj,
                                                               h->divt, h->pb);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(div, h->pb, h->nv * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -3265,9 +3264,9 @@ extern "C" int cfsa_ns_compute_divergence_noalloc(cfsa_ns *h, const double *u_de
   const int code = noalloc_scratch(h, &scratch);
   if (code != CFSA_OK) return code;
   return guarded(h, [&] {
-    k_tet_div<<<blocks_for(h->nt), kBlock, 0, h->stream>>>((int)h->nt, h->N2, h->tnode, h->grad, u_dev,
+    k_tet_div<<<blocks_for(h->nt), kBlock, 0, h->stream>>>((int)h->nt, h->N2, h->tnode, h->vol, h->grad, u_dev,
                                                            scratch, nullptr);
-    k_gather_div<<<blocks_for(h->nv), kBlock, 0, h->stream>>>((int)h->nv, h->adj_ptr, h->adj, h->vol,
+    k_gather_div<<<blocks_for(h->nv), kBlock, 0, h->stream>>>((int)h->nv, h->adj_ptr, h->adj,
                                                               scratch, div_dev);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));

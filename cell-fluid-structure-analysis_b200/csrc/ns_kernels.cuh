@@ -152,80 +152,133 @@ __device__ __forceinline__ void node_grad(const double *__restrict__ grad, int n
   }
 }
 
-// P2 mass and stiffness, one thread per row, incident tets in ascending order
-// (buildMassMatrix NavierStokes.cpp:247-285, buildStiffnessMatrix :159-218).
-__global__ void k_assemble_p2(int nrows, int nt, double density, double mu,
+// Assembly: one warp per row. The warp takes its row's incident tets in ascending order, several at a
+// time; a lane evaluates one (tet, local column) entry, and the tets' entries are then added one tet after
+// another (the columns of one tet are distinct), so every slot sums its tets in ascending order. The row's
+// columns and sums sit in shared memory (rows of more than kAsmRow entries work on global memory). One
+// thread per row walked a vertex row's 24 tets x 10 columns through dependent global reads and writes:
+// P2 4.71 ms and P1 1.85 ms at 1M tets, latency-bound.
+constexpr int kAsmRow = 160, kAsmWarps = 4;
+
+// P2 mass and stiffness (buildMassMatrix NavierStokes.cpp:247-285, buildStiffnessMatrix :159-218).
+__global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p2(int nrows, int nt, double density, double mu,
                               const int *__restrict__ adj_ptr, const int *__restrict__ adj,
                               const int *__restrict__ tnode, const double *__restrict__ vol,
                               const double *__restrict__ grad, const int *__restrict__ rp,
                               const int *__restrict__ ci, double *__restrict__ Mv,
                               double *__restrict__ Kv) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double s_m[kAsmWarps][kAsmRow], s_k[kAsmWarps][kAsmRow];
+  __shared__ int s_c[kAsmWarps][kAsmRow];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * kAsmWarps + warp;
   if (row >= nrows) return;
-  const int beg = rp[row], end = rp[row + 1];
-  for (int k = beg; k < end; ++k) {
-    Mv[k] = 0.0;
-    Kv[k] = 0.0;
+  const int beg = rp[row], len = rp[row + 1] - beg;
+  const bool small = len <= kAsmRow;
+  const int *cols = small ? s_c[warp] : ci + beg;
+  double *am = small ? s_m[warp] : Mv + beg, *ak = small ? s_k[warp] : Kv + beg;
+  for (int k = lane; k < len; k += 32) {
+    if (small) s_c[warp][k] = ci[beg + k];
+    am[k] = 0.0;
+    ak[k] = 0.0;
   }
-  for (int q = adj_ptr[row]; q < adj_ptr[row + 1]; ++q) {
-    const int t = adj[q] >> 4, li = adj[q] & 15;
-    const double V = vol[t];
-    const double mass = density * V;
-    double gi[3];
-    node_grad(grad, nt, t, li, gi);
-    for (int lj = 0; lj < 10; ++lj) {
+  __syncwarp();
+  const int b = lane / 10, lj = lane - 10 * b;  // lanes 0-29: three tets of ten columns
+  const int q1 = adj_ptr[row + 1];
+  for (int q0 = adj_ptr[row]; q0 < q1; q0 += 3) {
+    const bool on = b < 3 && q0 + b < q1;
+    int slot = 0;
+    double m = 0.0, kk = 0.0;
+    if (on) {
+      const int t = adj[q0 + b] >> 4, li = adj[q0 + b] & 15;
       const int col = tnode[(size_t)lj * nt + t];
-      const int slot = find_col(ci, beg, end, col);
-      double m;
-      if (li < 4 && lj < 4)
-        m = (li == lj) ? mass / 10.0 : mass / 20.0;
-      else if (li >= 4 && lj >= 4)
-        m = (li == lj) ? mass / 15.0 : mass / 60.0;
-      else
-        m = mass / 30.0;
-      double gj[3];
+      const double V = vol[t];
+      const double mass = density * V;
+      double gi[3], gj[3];
+      node_grad(grad, nt, t, li, gi);
       node_grad(grad, nt, t, lj, gj);
+      slot = find_col(cols, 0, len, col);
+      // V/10 and V/20 between vertices, V/15 and V/60 between edge nodes, V/30 mixed
+      const bool vi = li < 4, vj = lj < 4;
+      m = mass / (vi != vj ? 30.0 : vi ? (li == lj ? 10.0 : 20.0) : (li == lj ? 15.0 : 60.0));
       const double d = (gi[0] * gj[0] + gi[1] * gj[1]) + gi[2] * gj[2];
-      Mv[slot] += m;
-      Kv[slot] += mu * V * d;
+      kk = mu * V * d;
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      if (on && b == u) {
+        am[slot] += m;
+        ak[slot] += kk;
+      }
+      __syncwarp();
     }
   }
+  if (small)
+    for (int k = lane; k < len; k += 32) {
+      Mv[beg + k] = am[k];
+      Kv[beg + k] = ak[k];
+    }
 }
 
 // P1 gradient and Poisson matrices (buildGradientMatrices NavierStokes.cpp:91-120,
 // buildPoissonMatrix :331-349). G is stored as three consecutive nnz1 blocks (x, y, z).
-__global__ void k_assemble_p1(int nrows, int nt, int64_t nnz1, const int *__restrict__ adj_ptr,
+__global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1(int nrows, int nt, int64_t nnz1, const int *__restrict__ adj_ptr,
                               const int *__restrict__ adj, const int *__restrict__ tnode,
                               const double *__restrict__ vol, const double *__restrict__ grad,
                               const int *__restrict__ rp, const int *__restrict__ ci,
                               double *__restrict__ Gv, double *__restrict__ Lv) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double s_v[kAsmWarps][4][kAsmRow];
+  __shared__ int s_c[kAsmWarps][kAsmRow];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * kAsmWarps + warp;
   if (row >= nrows) return;
-  const int beg = rp[row], end = rp[row + 1];
-  for (int k = beg; k < end; ++k) {
-    Gv[k] = 0.0;
-    Gv[nnz1 + k] = 0.0;
-    Gv[2 * nnz1 + k] = 0.0;
-    Lv[k] = 0.0;
+  const int beg = rp[row], len = rp[row + 1] - beg;
+  const bool small = len <= kAsmRow;
+  const int *cols = small ? s_c[warp] : ci + beg;
+  double *out[4] = {Gv + beg, Gv + nnz1 + beg, Gv + 2 * nnz1 + beg, Lv + beg}, *acc[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[c] = small ? s_v[warp][c] : out[c];
+  for (int k = lane; k < len; k += 32) {
+    if (small) s_c[warp][k] = ci[beg + k];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[c][k] = 0.0;
   }
-  for (int q = adj_ptr[row]; q < adj_ptr[row + 1]; ++q) {
-    const int t = adj[q] >> 4, li = adj[q] & 15;
-    if (li >= 4) continue;
-    const double V = vol[t];
-    double gi[3];
-    node_grad(grad, nt, t, li, gi);
-    for (int lj = 0; lj < 4; ++lj) {
-      const int col = tnode[(size_t)lj * nt + t];
-      const int slot = find_col(ci, beg, end, col);
-      double gj[3];
-      node_grad(grad, nt, t, lj, gj);
-      const double contrib = V / 4.0;
-      Gv[slot] += contrib * gj[0];
-      Gv[nnz1 + slot] += contrib * gj[1];
-      Gv[2 * nnz1 + slot] += contrib * gj[2];
-      Lv[slot] += V * ((gi[0] * gj[0] + gi[1] * gj[1]) + gi[2] * gj[2]);
+  __syncwarp();
+  const int b = lane >> 2, lj = lane & 3;  // eight tets of four columns
+  const int q1 = adj_ptr[row + 1];
+  for (int q0 = adj_ptr[row]; q0 < q1; q0 += 8) {
+    bool on = q0 + b < q1;
+    int slot = 0;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (on) {
+      const int t = adj[q0 + b] >> 4, li = adj[q0 + b] & 15;
+      on = li < 4;
+      if (on) {
+        const int col = tnode[(size_t)lj * nt + t];
+        const double V = vol[t];
+        double gi[3], gj[3];
+        node_grad(grad, nt, t, li, gi);
+        node_grad(grad, nt, t, lj, gj);
+        slot = find_col(cols, 0, len, col);
+        const double contrib = V / 4.0;
+        v[0] = contrib * gj[0];
+        v[1] = contrib * gj[1];
+        v[2] = contrib * gj[2];
+        v[3] = V * ((gi[0] * gj[0] + gi[1] * gj[1]) + gi[2] * gj[2]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (on && b == u) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c][slot] += v[c];
+      }
+      __syncwarp();
     }
   }
+  if (small)
+    for (int k = lane; k < len; k += 32)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) out[c][k] = acc[c][k];
 }
 
 // 1/rowsum(M) with the reference's 1e-14 guard (NavierStokes.cpp:293-306).
@@ -379,9 +432,11 @@ __global__ void k_tet_conv(int nt, int64_t n2, const int *__restrict__ tnode,
 }
 
 // Per-tet divergence tr(grad u) over P1 vertex velocities (computeDivergence
-// NavierStokes.cpp:684-693).
+// NavierStokes.cpp:684-693) times the share V/4 of each vertex, so that the gather reads one value per
+// incident tet instead of two.
 __global__ void k_tet_div(int nt, int64_t n2, const int *__restrict__ tnode,
-                          const double *__restrict__ grad, const double *__restrict__ u,
+                          const double *__restrict__ vol, const double *__restrict__ grad,
+                          const double *__restrict__ u,
                           double *__restrict__ divt, const DevStatus *__restrict__ st) {
   if (st && st->halt) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -393,7 +448,7 @@ __global__ void k_tet_div(int nt, int64_t n2, const int *__restrict__ tnode,
 #pragma unroll
     for (int a = 0; a < 3; ++a) d[a] += u[a * n2 + v] * grad[(size_t)(3 * j + a) * nt + t];
   }
-  divt[t] = (d[0] + d[1]) + d[2];
+  divt[t] = (vol[t] / 4.0) * ((d[0] + d[1]) + d[2]);
 }
 
 // Convection gather: conv_i = -sum_t w_t c_t, w = V/4 (vertex) or V/24 (edge node)
@@ -411,15 +466,23 @@ __device__ __forceinline__ void gather_conv(int i, int nt, const int *__restrict
   }
 }
 
-// Divergence gather onto P1 vertices: div_i = sum_t (V/4) d_t (NavierStokes.cpp:696-698).
+// Divergence gather onto P1 vertices: div_i = sum_t (V/4) d_t (NavierStokes.cpp:696-698), tets ascending,
+// eight incident tets' loads in flight.
 __device__ __forceinline__ double gather_div(int i, const int *__restrict__ adj_ptr,
-                                             const int *__restrict__ adj,
-                                             const double *__restrict__ vol,
-                                             const double *__restrict__ divt) {
+                                             const int *__restrict__ adj, const double *__restrict__ divt) {
+  constexpr int kB = 8;
+  const int q1 = adj_ptr[i + 1];
   double s = 0.0;
-  for (int q = adj_ptr[i]; q < adj_ptr[i + 1]; ++q) {
-    const int t = adj[q] >> 4;
-    s += (vol[t] / 4.0) * divt[t];
+  for (int q = adj_ptr[i]; q < q1; q += kB) {
+    int t[kB];
+    double v[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) t[u] = (q + u < q1) ? adj[q + u] >> 4 : 0;
+#pragma unroll
+    for (int u = 0; u < kB; ++u) v[u] = (q + u < q1) ? divt[t[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kB; ++u)
+      if (q + u < q1) s += v[u];
   }
   return s;
 }
@@ -435,11 +498,10 @@ __global__ void k_gather_conv(int n, int nt, const int *__restrict__ adj_ptr,
 }
 
 __global__ void k_gather_div(int nv, const int *__restrict__ adj_ptr, const int *__restrict__ adj,
-                             const double *__restrict__ vol, const double *__restrict__ divt,
-                             double *__restrict__ out) {
+                             const double *__restrict__ divt, double *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
-  out[i] = gather_div(i, adj_ptr, adj, vol, divt);
+  out[i] = gather_div(i, adj_ptr, adj, divt);
 }
 
 // One SELL row, NC right-hand sides sharing the matrix. Entries are fetched in chunks of U
@@ -794,7 +856,7 @@ __global__ void k_check_cg(const CgState *__restrict__ cs, DevStatus *st, const 
 // (NavierStokes.cpp:590-626), fused with the Krylov initialisation (CG or BiCGSTAB, x0 = 0).
 struct PressureRhsArgs {
   const int *adj_ptr, *adj;
-  const double *vol, *divt;
+  const double *divt;
   const signed char *bc;
   const double *invL;
   double dt, tol, outlet_pressure;
@@ -830,7 +892,7 @@ __global__ void k_pressure_rhs(PressureRhsArgs A) {
               A.adj_q + 2 * (int64_t)A.nv, g);
       b = ((g[0] + g[1]) + g[2]) + A.adj_lpp[i];
     } else {
-      const double d = gather_div(i, A.adj_ptr, A.adj, A.vol, A.divt);
+      const double d = gather_div(i, A.adj_ptr, A.adj, A.divt);
       b = -d / A.dt;
       if (A.outlet_type == 1) {
         if (i == A.ref_node) b += kPoissonPenalty * 0.0;
