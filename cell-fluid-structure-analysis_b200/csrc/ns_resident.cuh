@@ -182,53 +182,82 @@ struct Resident {
     nc = 0;
   }
 
-  // f(i, part) for every entry i < n of the CTA's natural blocks.
-  template <int NV, class F>
-  __device__ __forceinline__ void entries(int n, F &&f) {
-    begin_entries(n);
-    for (int q = threadIdx.x >> 5; q < na; q += kWarps) {
-      int slot;
-      const int i = 32 * chunk(q, slot) + (int)(threadIdx.x & 31);
-      double part[NV];
-#pragma unroll
-      for (int j = 0; j < NV; ++j) part[j] = 0.0;
-      if (i < n) f(i, part);
-      chunk_sums<NV>(part, slot);
-    }
-    rev = !rev;
-  }
-
-  // f(i) for every entry i < n of the CTA's natural blocks.
-  template <class F>
-  __device__ __forceinline__ void each(int n, F &&f) {
-    begin_entries(n);
-    for (int q = threadIdx.x >> 5; q < na; q += kWarps) {
-      int slot;
-      const int i = 32 * chunk(q, slot) + (int)(threadIdx.x & 31);
-      if (i < n) f(i);
-    }
-    rev = !rev;
-  }
-
-  // Vector phase without sums: apply(i, load(i)) for every entry i < n of the CTA's natural blocks; with
-  // registers to spare, the loads of two chunks ahead of the stores of both (which may alias them for all
-  // the compiler knows; at 640 or 1024 threads the second set spills: 12.6 against 11.7 ms per 1M-tet solve).
-  template <class L, class F>
-  __device__ __forceinline__ void update(int n, L &&load, F &&apply) {
-    if constexpr (T > 256) {
-      each(n, [&](int i) { apply(i, load(i)); });
-      return;
-    }
+  // Vector phase: apply(c, i, common(i), load(c, i), scalar(c), part) for every entry i < n of the CTA's
+  // natural blocks and every component c in `mask`, the loads ahead of the stores; value 3 v + c of the phase sums part[v] (NV = 0: no
+  // sums). With 1024 threads the components follow one another and two chunks' loads are in flight, which
+  // fits 64 registers where all components of one entry at a time spill (momentum CG iteration at 1M tets 180
+  // -> 161 us); with fewer threads there is room for all components at once, and short ranges want the
+  // latency paid once (250k tets 54 against 57 us).
+  template <int NV, class S, class C, class L, class F>
+  __device__ __forceinline__ void vector(int n, int mask, S &&scalar, C &&common, L &&load, F &&apply) {
+    using V = decltype(load(0, 0));
+    using W = decltype(common(0));
     begin_entries(n);
     const int lane = threadIdx.x & 31;
-    for (int q = threadIdx.x >> 5; q < na; q += 2 * kWarps) {
-      int slot;
-      const int i = 32 * chunk(q, slot) + lane;
-      const bool two = q + kWarps < na;
-      const int i2 = two ? 32 * chunk(q + kWarps, slot) + lane : n;
-      const auto v = load(min(i, n - 1)), v2 = load(min(i2, n - 1));
-      if (i < n) apply(i, v);
-      if (i2 < n) apply(i2, v2);
+    if constexpr (T >= 1024) {
+      constexpr int K = 2;
+      for (int q = K * (int)(threadIdx.x >> 5); q < na; q += K * kWarps) {
+        W w[K];
+        int slot;
+#pragma unroll
+        for (int u = 0; u < K; ++u) w[u] = common(min(32 * chunk(min(q + u, na - 1), slot) + lane, n - 1));
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {
+          if (!((mask >> c) & 1)) continue;
+          const auto sc = scalar(c);
+          V v[K];
+#pragma unroll
+          for (int u = 0; u < K; ++u) v[u] = load(c, min(32 * chunk(min(q + u, na - 1), slot) + lane, n - 1));
+#pragma unroll
+          for (int u = 0; u < K; ++u) {
+            if (q + u >= na) break;
+            const int i = 32 * chunk(q + u, slot) + lane;
+            double part[NV > 0 ? NV : 1] = {};
+            if (i < n) apply(c, i, w[u], v[u], sc, part);
+            if constexpr (NV > 0) {
+              double *sl = slots() + (size_t)slot * 3 * NV + c;
+#pragma unroll
+              for (int j = 0; j < NV; ++j) {
+                const double t = warp_sum(part[j]);
+                if (lane == 0) sl[3 * j] = t;
+              }
+            }
+          }
+        }
+      }
+    } else {
+      constexpr int K = (T <= 256 && NV == 0) ? 2 : 1;
+      const decltype(scalar(0)) sc[3] = {scalar(0), scalar(1), scalar(2)};
+      for (int q = threadIdx.x >> 5; q < na; q += K * kWarps) {
+        V v[K][3];
+        W w[K];
+        int i[K], slot[K];
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+          const int k = q + u * kWarps;
+          i[u] = (u == 0 || k < na) ? 32 * chunk(k, slot[u]) + lane : n;
+          const int il = min(i[u], n - 1);  // past the end: loads that are not used, no divergence
+          w[u] = common(il);
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            if ((mask >> c) & 1) v[u][c] = load(c, il);
+        }
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+          double sum[NV > 0 ? 3 * NV : 1] = {};
+          if (i[u] < n) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              if (!((mask >> c) & 1)) continue;
+              double part[NV > 0 ? NV : 1] = {};
+              apply(c, i[u], w[u], v[u][c], sc[c], part);
+#pragma unroll
+              for (int j = 0; j < NV; ++j) sum[3 * j + c] = part[j];
+            }
+          }
+          if constexpr (NV > 0) chunk_sums<3 * NV>(sum, slot[u]);
+        }
+      }
     }
     rev = !rev;
   }
@@ -352,30 +381,24 @@ __global__ void __launch_bounds__(T, 1) k_mcg_solve(BicgArgs A, ResidentArgs R) 
     if (!active) break;
     // x += alpha p, r -= alpha q, z = D^-1 r; r.r and r.z; convergence and next beta
     {
-      double al[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) al[c] = s.alpha[c];
-      G.template entries<6>(A.n, [&](int i, double (&part)[6]) {
-        const double dinv = A.invA[i];
-        double xv[3], pv[3], rv[3], qv[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          xv[c] = A.x[o], pv[c] = A.pk[o], rv[c] = A.r[o], qv[c] = A.v[o];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.x[o] = xv[c] + al[c] * pv[c];
-          const double ri = rv[c] - al[c] * qv[c];
-          A.r[o] = ri;
-          const double zi = dinv * ri;
-          part[c] = ri * ri;
-          part[3 + c] = ri * zi;
-        }
-      });
+      struct V {
+        double x, p, r, q;
+      };
+      G.template vector<2>(
+          A.n, active, [&](int c) { return s.alpha[c]; }, [&](int i) { return A.invA[i]; },
+          [&](int c, int i) {
+            const int64_t o = c * n + i;
+            return V{A.x[o], A.pk[o], A.r[o], A.v[o]};
+          },
+          [&](int c, int i, double dinv, const V &v, double al, double (&part)[2]) {
+            const int64_t o = c * n + i;
+            A.x[o] = v.x + al * v.p;
+            const double ri = v.r - al * v.q;
+            A.r[o] = ri;
+            const double zi = dinv * ri;
+            part[0] = ri * ri;
+            part[1] = ri * zi;
+          });
     }
     double t[6];
     if (!G.template reduce<6>(t)) return;
@@ -402,26 +425,14 @@ __global__ void __launch_bounds__(T, 1) k_mcg_solve(BicgArgs A, ResidentArgs R) 
     if (!active) break;
     // p = z + beta p
     {
-      double be[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) be[c] = s.beta[c];
       struct V {
-        double dinv, r[3], p[3];
+        double r, p;
       };
-      G.update(
-          A.n,
-          [&](int i) {
-            V v;
-            v.dinv = A.invA[i];
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-              if ((active >> c) & 1) v.r[c] = A.r[c * n + i], v.p[c] = A.pk[c * n + i];
-            return v;
-          },
-          [&](int i, const V &v) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-              if ((active >> c) & 1) A.pk[c * n + i] = v.dinv * v.r[c] + be[c] * v.p[c];
+      G.template vector<0>(
+          A.n, active, [&](int c) { return s.beta[c]; }, [&](int i) { return A.invA[i]; },
+          [&](int c, int i) { return V{A.r[c * n + i], A.pk[c * n + i]}; },
+          [&](int c, int i, double dinv, const V &v, double be, double (&)[1]) {
+            A.pk[c * n + i] = dinv * v.r + be * v.p;
           });
     }
     if (!G.sync()) return;
@@ -506,29 +517,18 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve3(BicgArgs A, ResidentArgs R
     const int restart = s.restart & active;
     // p = r + beta (p - omega v)
     {
-      double be[3], om[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) be[c] = s.beta[c], om[c] = s.omega[c];
-      const int mask = active & ~restart;
       struct V {
-        double r[3], p[3], v[3];
+        double r, p, v;
       };
-      G.update(
-          A.n,
-          [&](int i) {
-            V x;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              if (!((mask >> c) & 1)) continue;
-              const int64_t o = c * n + i;
-              x.r[c] = A.r[o], x.p[c] = A.pk[o], x.v[c] = A.v[o];
-            }
-            return x;
+      G.template vector<0>(
+          A.n, active & ~restart, [&](int c) { return make_double2(s.beta[c], s.omega[c]); },
+          [](int) { return 0; },
+          [&](int c, int i) {
+            const int64_t o = c * n + i;
+            return V{A.r[o], A.pk[o], A.v[o]};
           },
-          [&](int i, const V &x) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-              if ((mask >> c) & 1) A.pk[c * n + i] = x.r[c] + be[c] * (x.p[c] - om[c] * x.v[c]);
+          [&](int c, int i, int, const V &x, double2 k, double (&)[1]) {  // k: beta, omega
+            A.pk[c * n + i] = x.r + k.x * (x.p - k.y * x.v);
           });
     }
     if (restart) {
@@ -569,27 +569,14 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve3(BicgArgs A, ResidentArgs R
     }
     if (!active) break;
     // s = r - alpha v
-    double al[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) al[c] = s.alpha[c];
     {
       struct V {
-        double r[3], v[3];
+        double r, v;
       };
-      G.update(
-          A.n,
-          [&](int i) {
-            V x;
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-              if ((active >> c) & 1) x.r[c] = A.r[c * n + i], x.v[c] = A.v[c * n + i];
-            return x;
-          },
-          [&](int i, const V &x) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-              if ((active >> c) & 1) A.s[c * n + i] = x.r[c] - al[c] * x.v[c];
-          });
+      G.template vector<0>(
+          A.n, active, [&](int c) { return s.alpha[c]; }, [](int) { return 0; },
+          [&](int c, int i) { return V{A.r[c * n + i], A.v[c * n + i]}; },
+          [&](int c, int i, int, const V &x, double al, double (&)[1]) { A.s[c * n + i] = x.r - al * x.v; });
     }
     if (!G.sync()) return;
     // t = At s, omega = (t . s) / (t . t)
@@ -613,32 +600,28 @@ __global__ void __launch_bounds__(T, 1) k_bicg_solve3(BicgArgs A, ResidentArgs R
       each_component<3>(active, &s.active, [&](int c) { return bicg_after_t(s, c, pick<3>(t, c), pick<3>(t, c, 3)); });
     }
     // x += alpha D^-1 p + omega D^-1 s, r = s - omega t; convergence test and next beta
-    double om[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) om[c] = s.omega[c];
-    G.template entries<6>(A.n, [&](int i, double (&part)[6]) {
-      const double dinv = A.invA[i];
-      const double w = A.cw ? A.cw[i] : 1.0;
-      double pv[3], sv[3], tv[3], xv[3], r0v[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (!((active >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        pv[c] = A.pk[o], sv[c] = A.s[o], tv[c] = A.t[o], xv[c] = A.x[o], r0v[c] = A.r0[o];
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (!((active >> c) & 1)) continue;
-        const int64_t o = c * n + i;
-        const double y = dinv * pv[c];
-        const double z = dinv * sv[c];
-        A.x[o] = xv[c] + (al[c] * y + om[c] * z);
-        const double ri = sv[c] - om[c] * tv[c];
-        A.r[o] = ri;
-        part[c] = (ri * ri) * w;
-        part[3 + c] = r0v[c] * ri;
-      }
-    });
+    {
+      struct V {
+        double p, s, t, x, r0;
+      };
+      G.template vector<2>(
+          A.n, active, [&](int c) { return make_double2(s.alpha[c], s.omega[c]); },
+          [&](int i) { return make_double2(A.invA[i], A.cw ? A.cw[i] : 1.0); },
+          [&](int c, int i) {
+            const int64_t o = c * n + i;
+            return V{A.pk[o], A.s[o], A.t[o], A.x[o], A.r0[o]};
+          },
+          [&](int c, int i, double2 d, const V &v, double2 k, double (&part)[2]) {  // k: alpha, omega
+            const int64_t o = c * n + i;
+            const double y = d.x * v.p;
+            const double z = d.x * v.s;
+            A.x[o] = v.x + (k.x * y + k.y * z);
+            const double ri = v.s - k.y * v.t;
+            A.r[o] = ri;
+            part[0] = (ri * ri) * d.y;
+            part[1] = v.r0 * ri;
+          });
+    }
     double t[6];
     if (!G.template reduce<6>(t)) return;
     active = each_component<3>(active, &s.active, [&](int c) { return bicg_after_xr(s, c, pick<3>(t, c), pick<3>(t, c, 3)); });
@@ -816,31 +799,25 @@ __global__ void __launch_bounds__(T, 1) k_mpc_solve(MixedArgs A, ResidentArgs R)
     // dx += alpha p, r -= alpha q, z = D^-1 r; the iterated residual and r.z; which components take
     // a reliable update, next beta for the others
     {
-      float al[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) al[c] = (float)s.alpha[c];
-      G.template entries<6>(A.n, [&](int i, double (&part)[6]) {
-        const float dinv = A.invA32[i];
-        const double w = A.cw32 ? (double)A.cw32[i] : 1.0;
-        float pv[3], qv[3], rv[3], dxv[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          pv[c] = A.p[o], qv[c] = A.v[o], rv[c] = A.r[o], dxv[c] = A.dx[o];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.dx[o] = dxv[c] + al[c] * pv[c];
-          const float ri = rv[c] - al[c] * qv[c];
-          A.r[o] = ri;
-          const float zi = dinv * ri;
-          part[c] = ((double)ri * (double)ri) * w;
-          part[3 + c] = (double)ri * (double)zi;
-        }
-      });
+      struct V {
+        float p, q, r, dx;
+      };
+      G.template vector<2>(
+          A.n, active, [&](int c) { return (float)s.alpha[c]; },
+          [&](int i) { return make_float2(A.invA32[i], A.cw32 ? A.cw32[i] : 1.f); },
+          [&](int c, int i) {
+            const int64_t o = c * n + i;
+            return V{A.p[o], A.v[o], A.r[o], A.dx[o]};
+          },
+          [&](int c, int i, float2 d, const V &v, float al, double (&part)[2]) {
+            const int64_t o = c * n + i;
+            A.dx[o] = v.dx + al * v.p;
+            const float ri = v.r - al * v.q;
+            A.r[o] = ri;
+            const float zi = d.x * ri;
+            part[0] = ((double)ri * (double)ri) * (double)d.y;
+            part[1] = (double)ri * (double)zi;
+          });
     }
     {
       double t[6];
@@ -866,15 +843,18 @@ __global__ void __launch_bounds__(T, 1) k_mpc_solve(MixedArgs A, ResidentArgs R)
     const int upd = s.upd;
     if (upd) {
       // x += dx (FP64), dx = 0
-      G.each(A.n, [&](int i) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((upd >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.x[o] = A.x[o] + (double)A.dx[o];
-          A.dx[o] = 0.f;
-        }
-      });
+      struct X {
+        double x;
+        float dx;
+      };
+      G.template vector<0>(
+          A.n, upd, [](int) { return 0; }, [](int) { return 0; },
+          [&](int c, int i) { return X{A.x[c * n + i], A.dx[c * n + i]}; },
+          [&](int c, int i, int, const X &v, int, double (&)[1]) {
+            const int64_t o = c * n + i;
+            A.x[o] = v.x + (double)v.dx;
+            A.dx[o] = 0.f;
+          });
       if (!G.sync()) return;
       // r64 = b - A x (FP64 operator), r = (float) r64; convergence on the true residual
       with_mask<3>(upd, [&](auto mk) {
@@ -931,19 +911,15 @@ __global__ void __launch_bounds__(T, 1) k_mpc_solve(MixedArgs A, ResidentArgs R)
     if (!active) break;
     // p = z + beta p with z = D^-1 r
     {
-      float be[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) be[c] = (float)s.beta[c];
-      G.each(A.n, [&](int i) {
-        const float dinv = A.invA32[i];
-        float rv[3], pv[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((active >> c) & 1) rv[c] = A.r[c * n + i], pv[c] = A.p[c * n + i];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((active >> c) & 1) A.p[c * n + i] = dinv * rv[c] + be[c] * pv[c];
-      });
+      struct V {
+        float r, p;
+      };
+      G.template vector<0>(
+          A.n, active, [&](int c) { return (float)s.beta[c]; }, [&](int i) { return A.invA32[i]; },
+          [&](int c, int i) { return V{A.r[c * n + i], A.p[c * n + i]}; },
+          [&](int c, int i, float dinv, const V &v, float be, double (&)[1]) {
+            A.p[c * n + i] = dinv * v.r + be * v.p;
+          });
     }
     if (!G.sync()) return;
   }
@@ -970,29 +946,26 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
     // r0 = p = r and rho = r0 . r
     const int rs = s.restart_next & active;
     {
-      float be[3], om[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) be[c] = (float)s.beta[c], om[c] = (float)s.omega[c];
-      auto row = [&](int i, double (&part)[3]) {
-        float rv[3], pv[3], vv[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((active >> c) & 1) rv[c] = A.r[c * n + i], pv[c] = A.p[c * n + i], vv[c] = A.v[c * n + i];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
+      struct V {
+        float r, p, v;
+      };
+      const auto load = [&](int c, int i) {
+        const int64_t o = c * n + i;
+        return V{A.r[o], A.p[o], A.v[o]};
+      };
+      const auto scalar = [&](int c) { return make_float2((float)s.beta[c], (float)s.omega[c]); };
+      const auto none = [](int) { return 0; };
+      if (rs) {
+        G.template vector<1>(A.n, active, scalar, none, load, [&](int c, int i, int, const V &x, float2 k, double (&part)[1]) {
           const int64_t o = c * n + i;
           if ((rs >> c) & 1) {
-            A.p[o] = rv[c];
-            A.r0[o] = rv[c];
-            part[c] = (double)rv[c] * (double)rv[c];
+            A.p[o] = x.r;
+            A.r0[o] = x.r;
+            part[0] = (double)x.r * (double)x.r;
           } else {
-            A.p[o] = rv[c] + be[c] * (pv[c] - om[c] * vv[c]);
+            A.p[o] = x.r + k.x * (x.p - k.y * x.v);
           }
-        }
-      };
-      if (rs) {
-        G.template entries<3>(A.n, row);
+        });
         double t[3];
         if (!G.template reduce<3>(t)) return;
         each_component<3>(active, &s.active, [&](int c) {
@@ -1004,9 +977,8 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
         });
         if (threadIdx.x == 0) s.restart_next = 0;
       } else {
-        G.each(A.n, [&](int i) {
-          double part[3];
-          row(i, part);
+        G.template vector<0>(A.n, active, scalar, none, load, [&](int c, int i, int, const V &x, float2 k, double (&)[1]) {
+          A.p[c * n + i] = x.r + k.x * (x.p - k.y * x.v);
         });
         if (!G.sync()) return;
       }
@@ -1045,18 +1017,15 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
     }
     if (!active) break;
     // s = r - alpha v
-    float al[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) al[c] = (float)s.alpha[c];
-    G.each(A.n, [&](int i) {
-      float rv[3], vv[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((active >> c) & 1) rv[c] = A.r[c * n + i], vv[c] = A.v[c * n + i];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if ((active >> c) & 1) A.s[c * n + i] = rv[c] - al[c] * vv[c];
-    });
+    {
+      struct V {
+        float r, v;
+      };
+      G.template vector<0>(
+          A.n, active, [&](int c) { return (float)s.alpha[c]; }, [](int) { return 0; },
+          [&](int c, int i) { return V{A.r[c * n + i], A.v[c * n + i]}; },
+          [&](int c, int i, int, const V &x, float al, double (&)[1]) { A.s[c * n + i] = x.r - al * x.v; });
+    }
     if (!G.sync()) return;
     // t = At32 s, omega = (t . s) / (t . t)
     with_mask<3>(active, [&](auto mk) {
@@ -1085,30 +1054,24 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
     // dx += alpha D^-1 p + omega D^-1 s, r = s - omega t; ||r||, r0 . r; which components take a
     // reliable update, next beta for the others
     {
-      float om[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) om[c] = (float)s.omega[c];
-      G.template entries<6>(A.n, [&](int i, double (&part)[6]) {
-        const float dinv = A.invA32[i];
-        const double w = A.cw32 ? (double)A.cw32[i] : 1.0;
-        float pv[3], sv[3], tv[3], dxv[3], r0v[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          pv[c] = A.p[o], sv[c] = A.s[o], tv[c] = A.t[o], dxv[c] = A.dx[o], r0v[c] = A.r0[o];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((active >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          A.dx[o] = dxv[c] + (al[c] * (dinv * pv[c]) + om[c] * (dinv * sv[c]));
-          const float ri = sv[c] - om[c] * tv[c];
-          A.r[o] = ri;
-          part[c] = ((double)ri * (double)ri) * w;
-          part[3 + c] = (double)r0v[c] * (double)ri;
-        }
-      });
+      struct V {
+        float p, s, t, dx, r0;
+      };
+      G.template vector<2>(
+          A.n, active, [&](int c) { return make_float2((float)s.alpha[c], (float)s.omega[c]); },
+          [&](int i) { return make_float2(A.invA32[i], A.cw32 ? A.cw32[i] : 1.f); },
+          [&](int c, int i) {
+            const int64_t o = c * n + i;
+            return V{A.p[o], A.s[o], A.t[o], A.dx[o], A.r0[o]};
+          },
+          [&](int c, int i, float2 d, const V &v, float2 k, double (&part)[2]) {  // k: alpha, omega
+            const int64_t o = c * n + i;
+            A.dx[o] = v.dx + (k.x * (d.x * v.p) + k.y * (d.x * v.s));
+            const float ri = v.s - k.y * v.t;
+            A.r[o] = ri;
+            part[0] = ((double)ri * (double)ri) * (double)d.y;
+            part[1] = (double)v.r0 * (double)ri;
+          });
     }
     {
       double t[6];
@@ -1140,18 +1103,20 @@ __global__ void __launch_bounds__(T, 1) k_mp_solve(MixedArgs A, ResidentArgs R) 
     const int upd = s.upd, rst = s.restart;
     if (upd) {
       // x += dx (FP64), dx = 0, xs = diag(A) x
-      G.each(A.n, [&](int i) {
-        const double d = A.diagA[i];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (!((upd >> c) & 1)) continue;
-          const int64_t o = c * n + i;
-          const double xi = A.x[o] + (double)A.dx[o];
-          A.x[o] = xi;
-          A.dx[o] = 0.f;
-          A.xs[o] = d * xi;
-        }
-      });
+      struct X {
+        double x;
+        float dx;
+      };
+      G.template vector<0>(
+          A.n, upd, [](int) { return 0; }, [&](int i) { return A.diagA[i]; },
+          [&](int c, int i) { return X{A.x[c * n + i], A.dx[c * n + i]}; },
+          [&](int c, int i, double d, const X &v, int, double (&)[1]) {
+            const int64_t o = c * n + i;
+            const double xi = v.x + (double)v.dx;
+            A.x[o] = xi;
+            A.dx[o] = 0.f;
+            A.xs[o] = d * xi;
+          });
       if (!G.sync()) return;
       // r64 = b - At64 (D x), r = (float) r64 (and r0 = r for a restart); convergence on the true
       // residual, next beta from the replaced one
