@@ -784,7 +784,7 @@ def main():
                 "unit": "GB/s", "frac": dom["achieved_gbs"] / peak, "peak_kind": peak_kind,
                 "traffic": dom["traffic"],
                 "traffic_note": "scaled, not measured on this workload: ncu dram__bytes_read.sum + write.sum of "
-                                "the momentum product captured at 414,720 tets (k_mcg_q<3>), times the ratio of "
+                                "the momentum product captured at 414,720 tets (k_momentum_product), times the ratio of "
                                 "algorithmic bytes per launch (profiles/dram_traffic.json)"}
 
     # accuracy of the headline itself: the timed steps again from the same state with the Krylov

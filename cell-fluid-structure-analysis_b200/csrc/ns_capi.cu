@@ -1,9 +1,9 @@
 // Host side of the C ABI declared in include/cfsa_ns.h: device memory, set-up (adjacency,
 // patterns, SELL layout, assembly), the step sequence and its CUDA-graph capture.
 //
-// One PISO step is captured once into a CUDA graph whose two Krylov loops are conditional
-// WHILE nodes: the last reduction kernel of each iteration decides on the device whether the
-// loop continues, so a step (or a batch of steps) runs with no host round trip.
+// One PISO step is captured once into a CUDA graph: every Krylov solve is one resident kernel that decides
+// on the device when it is done (the float pressure sweeps and the multi-kernel CG are conditional WHILE
+// nodes), so a step (or a batch of steps) runs with no host round trip.
 #include "cfsa_ns.h"
 #include "ns_adjoint.cuh"
 #include "ns_coarse.cuh"
@@ -56,7 +56,7 @@ struct Sell {
   int nrows = 0, nrows_pad = 0, nslices = 0;
   int64_t nentries = 0;
   std::vector<int> h_sptr;  // host copy of sptr
-  int *rfirst = nullptr;    // slice runs of the run-walking kernels (one per SM)
+  int *rfirst = nullptr;    // slice runs of the resident solves' CTAs (SellView::rfirst)
   int nruns = 0, max_run = 0;  // CTAs, most slices of one CTA
   SellView view() const { return SellView{sptr, col, len, perm, nrows_pad, rfirst}; }
 };
@@ -138,7 +138,7 @@ struct CoarseBuffers {
 
 struct cfsa_ns {
   int device = 0;
-  cudaStream_t stream = nullptr, body_stream = nullptr, body_stream2 = nullptr;
+  cudaStream_t stream = nullptr, body_stream = nullptr;
   // stream-ordered field read-back (cfsa_ns_get_*_async): device staging copies of u (node-major)
   // and p taken on `stream`, copied to the caller's host arrays on copy_stream
   cudaStream_t copy_stream = nullptr;
@@ -213,7 +213,7 @@ struct cfsa_ns {
   bool cg_persistent = true;
   int cg_grid = 0;
   std::map<const void *, int> stride_ctas_of;  // one resident wave of each grid-stride kernel
-  // SMEM-resident variant of the persistent CG (k_cg_resident): one 1024-thread CTA per SM
+  // resident pressure solvers: one kCgResThreads CTA per SM
   bool cg_resident = false;
   double *cg1_vec[3] = {nullptr, nullptr, nullptr};  // second r, w, s buffers of k_cg1_resident
   int cg_res_grid = 0, cg_res_bpc_sell = 0, cg_res_bpc_nat = 0, cg_res_entries = 0;  // entries: most of one CTA
@@ -336,7 +336,6 @@ struct cfsa_ns {
     for (cudaEvent_t e : ph)
       if (e) cudaEventDestroy(e);
     if (body_stream) cudaStreamDestroy(body_stream);
-    if (body_stream2) cudaStreamDestroy(body_stream2);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -495,7 +494,6 @@ struct cfsa_ns {
     CK(cudaGetDevice(&device));
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&body_stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&body_stream2, cudaStreamNonBlocking));
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
     for (cudaEvent_t &e : ph) CK(cudaEventCreate(&e));
@@ -977,60 +975,30 @@ struct cfsa_ns {
   }
 
   // ------------------------------------------------------------------ Krylov loops
-  // Appends a WHILE conditional node to the graph being captured on `stream`; its body (one
-  // Krylov iteration) is captured from `body` on body_stream. Returns the handle.
+  // Appends a WHILE conditional node to the graph being captured on `stream`; its body (one sweep or
+  // iteration) is captured on body_stream.
   template <class Body>
   void capture_while(Body body) {
-    capture_while_on(stream, body_stream, body);
-  }
-
-  // WHILE node appended to the graph being captured on `cap`; the body is captured on `sub`.
-  template <class Body>
-  void capture_while_on(cudaStream_t cap, cudaStream_t sub, Body body) {
-    capture_while_with(cap, sub, new_cond_handle(cap), body);
-  }
-
-  // Handle of a conditional node of the graph being captured on `cap`. Its default is applied
-  // when the top-level graph is launched; a node nested in a loop body must be set by a kernel
-  // upstream of it in the same body (k_mp_xr sets the reliable-update IF node every iteration).
-  cudaGraphConditionalHandle new_cond_handle(cudaStream_t cap, unsigned int dflt = 1) {
-    cudaStreamCaptureStatus cst;
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamGetCaptureInfo(cap, &cst, nullptr, &g, nullptr, nullptr));
-    if (cst != cudaStreamCaptureStatusActive) throw CudaError{"stream is not capturing"};
-    cudaGraphConditionalHandle h;
-    CK(cudaGraphConditionalHandleCreate(&h, g, dflt, cudaGraphCondAssignDefault));
-    return h;
-  }
-
-  template <class Body>
-  void capture_while_with(cudaStream_t cap, cudaStream_t sub, cudaGraphConditionalHandle h, Body body) {
-    capture_cond_with(cap, sub, h, cudaGraphCondTypeWhile, body);
-  }
-
-  // Conditional node (WHILE or IF) appended to the graph being captured on `cap`; its body is
-  // captured from `body` on `sub`.
-  template <class Body>
-  void capture_cond_with(cudaStream_t cap, cudaStream_t sub, cudaGraphConditionalHandle h,
-                         cudaGraphConditionalNodeType type, Body body) {
     cudaStreamCaptureStatus cst;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t *deps = nullptr;
     size_t ndeps = 0;
-    CK(cudaStreamGetCaptureInfo(cap, &cst, nullptr, &g, &deps, &ndeps));
+    CK(cudaStreamGetCaptureInfo(stream, &cst, nullptr, &g, &deps, &ndeps));
     if (cst != cudaStreamCaptureStatusActive) throw CudaError{"stream is not capturing"};
+    cudaGraphConditionalHandle h;
+    CK(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
     cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
     cp.conditional.handle = h;
-    cp.conditional.type = type;
+    cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
     cudaGraphNode_t node;
     CK(cudaGraphAddNode(&node, g, deps, ndeps, &cp));
-    CK(cudaStreamUpdateCaptureDependencies(cap, &node, 1, cudaStreamSetCaptureDependencies));
+    CK(cudaStreamUpdateCaptureDependencies(stream, &node, 1, cudaStreamSetCaptureDependencies));
     cudaGraph_t bodyg = cp.conditional.phGraph_out[0];
-    CK(cudaStreamBeginCaptureToGraph(sub, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    body(sub, h, 1);
+    CK(cudaStreamBeginCaptureToGraph(body_stream, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+    body(body_stream, h, 1);
     cudaGraph_t out = nullptr;
-    CK(cudaStreamEndCapture(sub, &out));
+    CK(cudaStreamEndCapture(body_stream, &out));
   }
 
   // Eager loop: enqueue iterations in growing chunks and poll the active flag in between.
@@ -1045,11 +1013,8 @@ struct cfsa_ns {
     }
   }
 
-  // Grid of a grid-stride reduction kernel over nblk blocks of 256 positions. The FP32 mixed-
-  // precision x/r update and the FP64 x/r update run one resident wave of CTAs that each visit
-  // several blocks (fewer CTA-wide barriers and tickets: 325 vs 355 us per FP32 inner iteration,
-  // 438 vs 448 us per FP64 iteration at 1M tets). The SELL products of the Krylov loops are
-  // run-walking kernels instead (one kRunThreads CTA per SM over a contiguous run of slices).
+  // Grid of a grid-stride reduction kernel over nblk blocks of 256 positions: one resident wave of CTAs
+  // that each visit several blocks (fewer CTA-wide barriers and tickets than one CTA per block).
   template <class K>
   unsigned int strided(K kernel, unsigned int nblk) const {
     auto it = stride_ctas_of.find((const void *)kernel);
@@ -2647,7 +2612,7 @@ int cfsa_ns_update_boundary_tags(cfsa_ns *h, const int8_t *p1_bc, const int8_t *
 // Message of a failed stepping call (status from the device status word).
 static std::string step_failure(int code) {
   std::string m = "step failed with status " + std::to_string(code);
-  if (code == CFSA_CUDA_ERROR) m += ": the pressure solve gave up waiting at a grid barrier";
+  if (code == CFSA_CUDA_ERROR) m += ": a Krylov solve gave up waiting at a grid barrier";
   return m;
 }
 

@@ -318,12 +318,6 @@ __global__ void k_sell_fill(int nrows_pad, const int *__restrict__ sptr, const i
   }
 }
 
-__global__ void k_scatter_vals(int64_t nnz, const int *__restrict__ posmap,
-                               const double *__restrict__ src, double *__restrict__ dst) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nnz) dst[posmap[k]] = src[k];
-}
-
 // Momentum operator A = M/dt + K + 1e10 on Inlet/Wall diagonals (NavierStokes.cpp:460-495).
 __global__ void k_momentum_diag(int n, double dt, const int *__restrict__ dpos,
                                 const double *__restrict__ Mv, const double *__restrict__ Kv,
@@ -587,9 +581,6 @@ __device__ __forceinline__ void with_mask(int mask, F &&f) {
   }
 }
 
-// Entries per chunk of a row in the FP64 Krylov products (4 measured faster than 8 on the
-// 1M-tet momentum operator: 135.8 vs 142.9 us; 12 or 16 with fewer threads per SM were slower).
-constexpr int kU64 = 4;
 
 // Row i of the transposed P1 operators G_a^T (a = 0..2) applied to x_a. The P1 pattern is
 // structurally symmetric: the entry (i, j) of G_a^T is G_a(j, i), stored at the transposed slot
@@ -1832,7 +1823,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
 // Two-level single-reduction CG (CFSA_KRYLOV_CG2L): the recurrences of k_cg1_resident with the
 // preconditioner M r = D^-1 r + P Z P^T r, where P is the indicator matrix of geometric aggregates
 // (boxes of a uniform grid over the vertices, rows without a penalty only) and Z = (P^T A P)^-1 is
-// a dense nc x nc matrix built on the host. The coarse correction removes the smooth error
+// a dense nc x nc matrix (ns_coarse.cuh). The coarse correction removes the smooth error
 // components that make Jacobi-CG slow on the Poisson operator (681 -> 127 iterations on the
 // 1M-tet cylinder with ~256 aggregates requested).
 //
@@ -1840,8 +1831,8 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
 // formed after the barrier from the previous iteration's aggregate sums of r and w and the
 // aggregate-level recurrence for s,
 //   T(s) <- T(w) + beta T(s),   t = T(r) - alpha T(s),   c = Z t,
-// and each neighbour's new u = D^-1 r_new + c[agg] is then formed on the fly in the fused product,
-// as k_cg1_resident does for the Jacobi part.
+// and each neighbour's new u = D^-1 r_new + c[agg] is then formed where the product needs it (in the
+// window, or per entry), as k_cg1_resident does for the Jacobi part.
 //
 // Aggregate sums are exact fixed-point sums, so their order does not matter and they cost a few
 // atomics instead of a reduction tree: each value x becomes the 128-bit integer floor(x 2^S)

@@ -3,7 +3,7 @@
 // Comput. 22(5), 2000; group-wise solution updates: Sleijpen & van der Vorst, Computing 56, 1996;
 // their mixed-precision GPU form: Clark et al., Comput. Phys. Commun. 181, 2010).
 //
-//   FP64: b, x (solution), r64 (true residual), xs = diag(A) x
+//   FP64: b, x (solution), xs = diag(A) x; the true residual is formed and rounded to r in one pass
 //   FP32: r, r0, p, v, s, t (Krylov vectors), dx (correction accumulated since the last update)
 //   every iteration (FP32 operator At32 = FP32 copy of A D^-1, FP64 dot products and scalars):
 //     p = r + beta (p - omega v); v = At32 p; alpha = rho / (r0.v); s = r - alpha v;
@@ -13,9 +13,9 @@
 //   breakdown:  x += dx; dx = 0; r64 = b - A x (FP64 operator); r = (float) r64
 // The Krylov space is kept across updates (p, r0 and the scalars carry on), so the iteration
 // count stays that of the FP64 solve instead of restarting with every correction. Convergence is
-// decided on the FP64 true residual only, with the FP64 solve's criterion. In a CUDA graph the
-// update is a conditional IF node inside the iteration's WHILE body, so iterations without an
-// update launch nothing extra. The penalty rows (diagonal 1e10) have unit diagonal in A D^-1, so
+// decided on the FP64 true residual only, with the FP64 solve's criterion. The iterations and
+// updates run in k_mp_solve (ns_resident.cuh); this file holds the state, the initialisation and the
+// check. The penalty rows (diagonal 1e10) have unit diagonal in A D^-1, so
 // FP32 holds them without overflow or loss. Components are independent (per-component scalars,
 // masks and updates).
 #pragma once

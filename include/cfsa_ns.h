@@ -125,7 +125,7 @@ typedef struct {
 } cfsa_ns_stats;
 
 /* kernel ids for cfsa_ns_profile_kernel */
-#define CFSA_KERNEL_MOMENTUM_SPMV 0 /* 3-right-hand-side SELL product of the momentum BiCGSTAB */
+#define CFSA_KERNEL_MOMENTUM_SPMV 0 /* 3-right-hand-side SELL product of the momentum solve */
 #define CFSA_KERNEL_PRESSURE_SPMV 1 /* SELL product of the pressure CG */
 /* the whole resident pressure solve (CFSA_KRYLOV_CG2L or _CG1) on the last step's system, fused
  * product and vector updates inside one kernel: avg_ms per solve, alg_bytes = iterations x bytes
@@ -165,12 +165,12 @@ int cfsa_ns_set_pressure_solver(cfsa_ns *h, int krylov);                   /* ne
 int cfsa_ns_set_momentum_solver(cfsa_ns *h, int krylov);
 /* new: aggregate count the CFSA_KRYLOV_CG2L coarse space aims for (default 256, 1..1024, others
  * are rejected with CFSA_BAD_ARG). The aggregates are boxes of a uniform grid, so the number
- * actually occupied can exceed the target (256 requested gives 432 on the 1M-tet cylinder); the
- * host Cholesky of the coarse matrix grows with the cube of the occupied count (~0.1 s at 432 on
- * that mesh). The coarse space is rebuilt with the Poisson operator. Its per-aggregate arrays (6 doubles each) share
- * the solve kernel's shared memory with the row staging: a coarse space that does not fit (very
- * large targets on very large meshes) fails the next step with CFSA_CUDA_ERROR and says so in
- * cfsa_ns_last_error. */
+ * actually occupied can exceed the target (256 requested gives 432 on the 1M-tet cylinder). The coarse
+ * space is rebuilt on the device with the Poisson operator (2.5 ms at 432 on that mesh, about half of it
+ * the Cholesky and inverse of the coarse matrix, which grow with the occupied count). Its per-aggregate
+ * arrays (4 doubles each) share the solve kernel's shared memory with the row staging: a coarse space
+ * that does not fit (very large targets on very large meshes) fails the next step with CFSA_CUDA_ERROR
+ * and says so in cfsa_ns_last_error. */
 int cfsa_ns_set_coarse_target(cfsa_ns *h, int target);
 /* new: aggregates of the current CFSA_KRYLOV_CG2L coarse space (built on demand; 0 for the other
  * methods or when the coarse operator was not SPD) */
@@ -250,15 +250,16 @@ int cfsa_ns_get_matrix(cfsa_ns *h, int which, int64_t *rowptr, int32_t *cols, do
 int cfsa_ns_get_inv_lumped_mass(cfsa_ns *h, double *out /*[N2]*/);
 
 /* ---- diagnostics (no counterpart in the reference) ---- */
-/* Times `iters` back-to-back launches of one step kernel on the handle's stream with CUDA events,
- * on the current device data, without touching the solver state. avg_ms: mean duration of one
- * launch; alg_bytes: algorithmic bytes one launch must move (matrix values and column indices,
- * row metadata, each vector element read or written once). */
+/* Times `iters` back-to-back runs of one step kernel on the handle's stream with CUDA events, on the
+ * current device data, without touching the solver state. A momentum product is a phase of the resident
+ * momentum solve; it runs `iters` times inside one launch, with its dot product's barrier and totals.
+ * avg_ms: mean duration of one run; alg_bytes: algorithmic bytes one run must move (matrix values and
+ * column indices, row metadata, each vector element read or written once). */
 int cfsa_ns_profile_kernel(cfsa_ns *h, int which, int iters, double *avg_ms, double *alg_bytes);
 /* Bound on the polls a CTA of the resident pressure solvers (CG, CFSA_KRYLOV_CG1, CG2L) makes at
  * a grid barrier before it gives up: the solve then stops, the step fails with CFSA_CUDA_ERROR
  * ("gave up waiting at a grid barrier"), time does not advance, and the handle stays usable.
- * polls < 0 restores the default (2^25 polls, over a second); 0 gives up at the first wait, which
+ * polls < 0 restores the default (2^22 polls, over two seconds; the bound of the other resident solves); 0 gives up at the first wait, which
  * tests use to exercise the failure path. */
 int cfsa_ns_set_barrier_spin_limit(cfsa_ns *h, int64_t polls);
 
