@@ -452,11 +452,27 @@ __device__ __forceinline__ void gather_conv(int i, int nt, const int *__restrict
                                             const double *__restrict__ vol,
                                             const double *__restrict__ ct, double acc[3]) {
   acc[0] = acc[1] = acc[2] = 0.0;
-  for (int q = adj_ptr[i]; q < adj_ptr[i + 1]; ++q) {
-    const int t = adj[q] >> 4, l = adj[q] & 15;
-    const double w = (l < 4) ? vol[t] / 4.0 : vol[t] / 24.0;
+  constexpr int kB = 4;  // incident tets in flight
+  const int q1 = adj_ptr[i + 1];
+  for (int q = adj_ptr[i]; q < q1; q += kB) {
+    int e[kB];
+    double w[kB], v[kB][3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] = acc[c] - w * ct[(size_t)c * nt + t];
+    for (int u = 0; u < kB; ++u) e[u] = (q + u < q1) ? adj[q + u] : 0;
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const int t = e[u] >> 4;
+      w[u] = (q + u < q1) ? vol[t] : 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[u][c] = (q + u < q1) ? ct[(size_t)c * nt + t] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      if (q + u >= q1) break;
+      const double wu = ((e[u] & 15) < 4) ? w[u] / 4.0 : w[u] / 24.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) acc[c] = acc[c] - wu * v[u][c];
+    }
   }
 }
 
@@ -602,6 +618,33 @@ __device__ __forceinline__ void gt_row3(int i, const int *__restrict__ rp, const
   out[2] = s2;
 }
 
+// Row i of G_a p (a = 0..2), columns ascending, four entries in flight.
+__device__ __forceinline__ void grad_row(int i, const CsrView &G, const double *__restrict__ Gv, int64_t nnz1,
+                                         const double *__restrict__ p, double g[3]) {
+  constexpr int kB = 4;
+  g[0] = g[1] = g[2] = 0.0;
+  const int k1 = G.rp[i + 1];
+  for (int k = G.rp[i]; k < k1; k += kB) {
+    int j[kB];
+    double a[kB][3], x[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const bool in = k + u < k1;
+      j[u] = in ? G.ci[k + u] : 0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a[u][c] = in ? Gv[c * nnz1 + k + u] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u) x[u] = (k + u < k1) ? p[j[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      if (k + u >= k1) break;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) g[c] += a[u][c] * x[u];
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // Momentum right-hand side (NavierStokes.cpp:429-495) for the three components, fused with the
 // initialisation of the batched BiCGSTAB (x0 = 0, r = r0 = b, p = v = 0).
@@ -655,17 +698,12 @@ __global__ void k_momentum_rhs(MomentumRhsArgs A) {
         }
       } else {
       double mu[3];
-      sell_spmv_row<3>(A.S, A.Ms, A.u, n, r, mu);
+      sell_spmv_row<3, 4>(A.S, A.Ms, A.u, n, r, mu);
 #pragma unroll
       for (int c = 0; c < 3; ++c) b[c] = 0.0 + mu[c] / A.dt;
       if (i < A.nv) {
-        double gp[3] = {0.0, 0.0, 0.0};
-        for (int k = A.G.rp[i]; k < A.G.rp[i + 1]; ++k) {
-          const double pj = A.p[A.G.ci[k]];
-          gp[0] += A.Gv[k] * pj;
-          gp[1] += A.Gv[A.nnz1 + k] * pj;
-          gp[2] += A.Gv[2 * A.nnz1 + k] * pj;
-        }
+        double gp[3];
+        grad_row(i, A.G, A.Gv, A.nnz1, A.p, gp);
 #pragma unroll
         for (int c = 0; c < 3; ++c) b[c] -= gp[c];
       }
@@ -2297,13 +2335,8 @@ __global__ void k_correct_velocity(CorrectArgs A) {
   } else if (bcv == BC_WALL) {
     out[0] = out[1] = out[2] = 0.0;
   } else if (i < A.nv && A.invm[i] > 1e-14) {
-    double g[3] = {0.0, 0.0, 0.0};
-    for (int k = A.G.rp[i]; k < A.G.rp[i + 1]; ++k) {
-      const double pj = A.pc[A.G.ci[k]];
-      g[0] += A.Gv[k] * pj;
-      g[1] += A.Gv[A.nnz1 + k] * pj;
-      g[2] += A.Gv[2 * A.nnz1 + k] * pj;
-    }
+    double g[3];
+    grad_row(i, A.G, A.Gv, A.nnz1, A.pc, g);
     const double f = -A.dt * A.invm[i];
     for (int c = 0; c < 3; ++c) out[c] = A.ustar[c * n + i] + A.relax_u * (f * g[c]);
   } else {
