@@ -213,7 +213,7 @@ struct cfsa_ns {
   bool cg_persistent = true;
   int cg_grid = 0;
   std::map<const void *, int> stride_ctas_of;  // one resident wave of each grid-stride kernel
-  // resident pressure solvers: one kCgResThreads CTA per SM
+  // resident pressure solvers: one kCgResThreads<windows> CTA per SM
   bool cg_resident = false;
   double *cg1_vec[3] = {nullptr, nullptr, nullptr};  // second r, w, s buffers of k_cg1_resident
   int cg_res_grid = 0, cg_res_bpc_sell = 0, cg_res_bpc_nat = 0, cg_res_entries = 0;  // entries: most of one CTA
@@ -723,12 +723,14 @@ struct cfsa_ns {
       const CgResidentArgs caps = resident_caps(0, 2048);  // 2 KiB for static shared memory
       cg_res_smem = resident_rows_bytes(caps.row_cap, caps.win_cap, caps.ent_cap, caps.val_cap);
       cg_resident = caps.row_cap > 0;
-      for (const void *fn : {(const void *)k_cg_resident<true>, (const void *)k_cg_resident<false>,
-                             (const void *)k_cg1_resident<true>, (const void *)k_cg1_resident<false>,
-                             (const void *)k_bicg_resident<true>, (const void *)k_bicg_resident<false>}) {
+      const std::pair<const void *, int> kernels[] = {
+          {(const void *)k_cg_resident<true>, kCgResThreads<true>},    {(const void *)k_cg_resident<false>, kCgResThreads<false>},
+          {(const void *)k_cg1_resident<true>, kCgResThreads<true>},   {(const void *)k_cg1_resident<false>, kCgResThreads<false>},
+          {(const void *)k_bicg_resident<true>, kCgResThreads<true>},  {(const void *)k_bicg_resident<false>, kCgResThreads<false>}};
+      for (const auto &[fn, threads] : kernels) {
         int o = 0;
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_res_smem));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kCgResThreads, cg_res_smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, threads, cg_res_smem));
         if (o < 1) throw CudaError{"resident pressure solver does not fit on an SM"};
       }
     }
@@ -948,10 +950,13 @@ struct cfsa_ns {
     const int npos_max = nc > 0 ? cg_res_bpc_sell * kBlock : 0;
     V.npos_max = npos_max;
     // shared memory: coarse arrays, then the rows
-    const void *const kernels[] = {(const void *)k_cg2l_resident<double, true>, (const void *)k_cg2l_resident<double, false>,
-                                   (const void *)k_cg2l_resident<float, true>, (const void *)k_cg2l_resident<float, false>};
+    const std::pair<const void *, int> kernels[] = {
+        {(const void *)k_cg2l_resident<double, true>, kCgResThreads<true>},
+        {(const void *)k_cg2l_resident<double, false>, kCgResThreads<false>},
+        {(const void *)k_cg2l_resident<float, true>, kCgResThreads<true>},
+        {(const void *)k_cg2l_resident<float, false>, kCgResThreads<false>}};
     size_t fixed_smem = 0;
-    for (const void *fn : kernels) {
+    for (const auto &[fn, threads] : kernels) {
       cudaFuncAttributes fa{};
       CK(cudaFuncGetAttributes(&fa, fn));
       fixed_smem = std::max(fixed_smem, fa.sharedSizeBytes);
@@ -961,10 +966,10 @@ struct cfsa_ns {
     if (!cg2l_caps.row_cap) throw CudaError{"two-level pressure preconditioner: coarse space too large for shared memory"};
     cg2l_smem = (size_t)coarse_bytes +
                 resident_rows_bytes(cg2l_caps.row_cap, cg2l_caps.win_cap, cg2l_caps.ent_cap, cg2l_caps.val_cap);
-    for (const void *fn : kernels) {
+    for (const auto &[fn, threads] : kernels) {
       CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg2l_smem));
       int o = 0;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kCgResThreads, cg2l_smem));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, threads, cg2l_smem));
       if (o < 1) throw CudaError{"two-level pressure preconditioner: kernel does not fit on an SM"};
     }
     // the view is a captured launch argument; the shared-memory layout follows from it
@@ -1294,7 +1299,7 @@ struct cfsa_ns {
       CK(cudaMemsetAsync(coarse_view.gacc, 0, (size_t)27 * coarse_view.nc * sizeof(unsigned long long), s));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned int)cg_res_grid);
-    cfg.blockDim = dim3(kCgResThreads);
+    cfg.blockDim = dim3(c2.R.win_cap ? kCgResThreads<true> : kCgResThreads<false>);
     cfg.dynamicSmemBytes = cg2l_smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -1376,7 +1381,7 @@ struct cfsa_ns {
     clear_barrier(stream);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned int)cg_res_grid);
-    cfg.blockDim = dim3(kCgResThreads);
+    cfg.blockDim = dim3(a.R.win_cap ? kCgResThreads<true> : kCgResThreads<false>);
     cfg.dynamicSmemBytes = cg_res_smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1467,14 +1472,14 @@ struct cfsa_ns {
         CK(cudaMemsetAsync(pp, 0, (size_t)nv * sizeof(double), stream));
         CK(cudaMemsetAsync(ps, 0, (size_t)nv * sizeof(double), stream));
         cfg.gridDim = dim3((unsigned int)cg_res_grid);
-        cfg.blockDim = dim3(kCgResThreads);
+        cfg.blockDim = dim3(rz.win_cap ? kCgResThreads<true> : kCgResThreads<false>);
         cfg.dynamicSmemBytes = cg_res_smem;
         CK(cudaLaunchKernelEx(&cfg, rz.win_cap ? k_cg1_resident<true> : k_cg1_resident<false>, c1));
       } else if (cg_resident) {
         CgResidentArgs rz = resident_caps(0, 2048);
         rz.P = c;
         cfg.gridDim = dim3((unsigned int)cg_res_grid);
-        cfg.blockDim = dim3(kCgResThreads);
+        cfg.blockDim = dim3(rz.win_cap ? kCgResThreads<true> : kCgResThreads<false>);
         cfg.dynamicSmemBytes = cg_res_smem;
         CK(cudaLaunchKernelEx(&cfg, rz.win_cap ? k_cg_resident<true> : k_cg_resident<false>, rz));
       } else {

@@ -1394,12 +1394,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_cg_persistent(CgPersistentArgs A)
 // shared memory what it needs of its rows in every iteration (ResidentRows). The arithmetic, the
 // per-block partial sums and the 256-accumulator tree are those of k_cg_persistent, so both kernels
 // produce the same bits.
-// 512 threads per CTA: 128 registers per thread leave room for every load of a row in flight, and the
+// With windows 512 threads per CTA: 128 registers per thread leave room for every load of a row in flight, and the
 // block-wide steps of an iteration (half a dozen) cost less with 16 warps than with 32. Two-level CG, us per
 // iteration with 1024 / 768 / 512 threads: 16.1 / 12.9 / 11.7 at 30k tets, 14.9 / 13.8 / 11.8 at 250k,
-// 24.7 / 20.8 / 19.0 at 1M.
-constexpr int kCgResThreads = 512;
-constexpr int kCgResGroups = kCgResThreads / kBlock;  // 256-thread groups per CTA
+// 24.7 / 20.8 / 19.0 at 1M. Without windows 1024: the gathers from L2 and HBM want warps in flight; CG on a
+// 4M-tet bifurcation takes 104 us per iteration with 512 threads and 79 with 1024.
+template <bool WIN>
+constexpr int kCgResThreads = WIN ? 512 : 1024;
+template <bool WIN>
+constexpr int kCgResGroups = kCgResThreads<WIN> / kBlock;  // 256-thread groups per CTA
 
 struct CgResidentArgs {
   CgPersistentArgs P;
@@ -1442,10 +1445,10 @@ __device__ __forceinline__ void group_partial(double (&v)[NV], double *__restric
 // tree_total for a resident CTA: the accumulators of all values are formed side by side, eight loads in
 // flight per thread (same sums in the same order as tree_total). Calls are a grid barrier apart, which
 // keeps sm from being rewritten while it is read.
-template <int NV>
+template <int NV, bool WIN>
 __device__ __forceinline__ void tree_total_cta(const double *__restrict__ partials, int nblk,
                                                double (&out)[NV], double (*sm)[kBlock / 32]) {
-  for (int a = threadIdx.x; a < NV * kBlock; a += kCgResThreads) {
+  for (int a = threadIdx.x; a < NV * kBlock; a += kCgResThreads<WIN>) {
     // accumulator t of value j: blocks t, t + 256, ... in order
     const int j = a / kBlock, t = a & (kBlock - 1);
     constexpr int kB = 8;
@@ -1595,6 +1598,43 @@ struct ResidentRows {
     return acc;
   }
 
+  // The same without a window: a chunk's columns and values, then its gathers.
+  template <class J, class F>
+  __device__ __forceinline__ double gather(int o, int n, J &&column, F &&f) const {
+    double acc = 0.0;
+    int k = 0;
+    for (; k + kCgChunk <= n; k += kCgChunk) {
+      int j[kCgChunk];
+      double a[kCgChunk], x[kCgChunk];
+#pragma unroll
+      for (int u = 0; u < kCgChunk; ++u) {
+        const int p = o + (k + u) * kSellC;
+        j[u] = column(p);
+        a[u] = (double)__ldg(val + p);
+      }
+#pragma unroll
+      for (int u = 0; u < kCgChunk; ++u) x[u] = f(j[u]);
+#pragma unroll
+      for (int u = 0; u < kCgChunk; ++u) acc += a[u] * x[u];
+    }
+    if (k < n) {
+      int j[kCgChunk];
+      double a[kCgChunk], x[kCgChunk];
+#pragma unroll
+      for (int u = 0; u < kCgChunk; ++u) {
+        const int p = o + min(k + u, n - 1) * kSellC;
+        j[u] = column(p);
+        a[u] = (double)__ldg(val + p);
+      }
+#pragma unroll
+      for (int u = 0; u < kCgChunk; ++u) x[u] = f(j[u]);
+#pragma unroll
+      for (int u = 0; u < kCgChunk; ++u)
+        if (k + u < n) acc += a[u] * x[u];
+    }
+    return acc;
+  }
+
   // Row sum of position lp of block b. What is staged is the same for a whole block, so the choice is
   // made once per row and not per entry (a choice per entry cost 3.2 instead of 1.4 us per pass).
   template <class F>
@@ -1609,19 +1649,16 @@ struct ResidentRows {
         x = win[idx[p]];
       });
     } else {
-      const bool staged = b < ent_blk;
-      return sum<kCgChunk>(o, n, [&](int p, double &a, double &x) {
-        a = (double)__ldg(val + p);
-        x = f(staged ? col[p - e0] : __ldg(R.P.S.col + p));
-      });
+      if (b < ent_blk) return gather(o, n, [&](int p) { return col[p - e0]; }, f);
+      return gather(o, n, [&](int p) { return __ldg(R.P.S.col + p); }, f);
     }
   }
 };
 
 template <bool WIN>
-__global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs R) {
+__global__ void __launch_bounds__(kCgResThreads<WIN>, 1) k_cg_resident(CgResidentArgs R) {
   extern __shared__ double s_dbl[];
-  __shared__ double s_grp[kCgResGroups][3][kBlock / 32];
+  __shared__ double s_grp[kCgResGroups<WIN>][3][kBlock / 32];
   __shared__ double s_tree[3][kBlock / 32];
   const CgPersistentArgs &A = R.P;
   if (A.st && A.st->halt) return;
@@ -1644,7 +1681,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs
     // phase A: q = L p on the owned SELL blocks, one group per block
     const auto pj = [&](int j) { return fly ? __ldcg(A.z + j) + beta * __ldcg(pold + j) : __ldcg(pold + j); };
     rows.fill(pj);
-    for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+    for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups<WIN>) {
       const int lp = (b - rows.b0) * kBlock + lt;
       const int i = rows.row_of(lp);
       double v[1] = {0.0};
@@ -1659,14 +1696,14 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs
     }
     if (!grid_sync(A.bar, phase)) return;
     double pq[1];
-    tree_total_cta<1>(A.part_a, A.nblk_sell, pq, s_tree);
+    tree_total_cta<1, WIN>(A.part_a, A.nblk_sell, pq, s_tree);
     if (pq[0] == 0.0) {
       status = KS_BREAKDOWN;
       break;
     }
     alpha = absnew / pq[0];
     // phase B: vector updates on the owned natural blocks
-    for (int b = c0 + g; b < c1; b += kCgResGroups) {
+    for (int b = c0 + g; b < c1; b += kCgResGroups<WIN>) {
       const int i = b * kBlock + lt;
       double v[2] = {0.0, 0.0};
       if (i < A.n) {
@@ -1683,7 +1720,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg_resident(CgResidentArgs
     }
     if (!grid_sync(A.bar, phase)) return;
     double tb[2];
-    tree_total_cta<2>(A.part_b, A.nblk_nat, tb, s_tree);
+    tree_total_cta<2, WIN>(A.part_b, A.nblk_nat, tb, s_tree);
     ++it;
     rr = A.scaled ? tb[1] : tb[0];
     if (isnan(tb[0]) || isnan(tb[1])) {
@@ -1731,9 +1768,9 @@ struct Cg1Args {
 };
 
 template <bool WIN>
-__global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
+__global__ void __launch_bounds__(kCgResThreads<WIN>, 1) k_cg1_resident(Cg1Args C) {
   extern __shared__ double s_dbl[];
-  __shared__ double s_grp[kCgResGroups][3][kBlock / 32];
+  __shared__ double s_grp[kCgResGroups<WIN>][3][kBlock / 32];
   __shared__ double s_tree[3][kBlock / 32];
   const CgResidentArgs &R = C.R;
   const CgPersistentArgs &A = R.P;
@@ -1750,7 +1787,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
   // start: w = A u0, delta = w.u0
   const auto u0 = [&](int j) { return __ldcg(C.u0 + j); };
   rows.fill(u0);
-  for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+  for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups<WIN>) {
     const int lp = (b - rows.b0) * kBlock + lt;
     const int i = rows.row_of(lp);
     double v[1] = {0.0};
@@ -1764,7 +1801,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
   if (!grid_sync(A.bar, phase)) return;
   {
     double d0[1];
-    tree_total_cta<1>(A.part_a, A.nblk_sell, d0, s_tree);
+    tree_total_cta<1, WIN>(A.part_a, A.nblk_sell, d0, s_tree);
     if (d0[0] == 0.0)
       status = KS_BREAKDOWN;
     else
@@ -1796,7 +1833,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
     };
     own(rows.b0 + g);
     rows.fill(uj);
-    for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups) {
+    for (int b = rows.b0 + g; b < rows.b1; b += kCgResGroups<WIN>) {
       double v[3] = {0.0, 0.0, 0.0};
       if (i >= 0) {
         const double acc = rows.product(b, (b - rows.b0) * kBlock + lt, uj);
@@ -1814,12 +1851,12 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg1_resident(Cg1Args C) {
         v[1] = acc * ui;
         v[2] = ri * ri;
       }
-      own(b + kCgResGroups);
+      own(b + kCgResGroups<WIN>);
       group_partial<3>(v, part, b, g, s_grp);
     }
     if (!grid_sync(A.bar, phase)) return;
     double t[3];
-    tree_total_cta<3>(part, A.nblk_sell, t, s_tree);
+    tree_total_cta<3, WIN>(part, A.nblk_sell, t, s_tree);
     ++it;
     rn2 = A.scaled ? t[0] : t[2];
     cur ^= 1;
@@ -2043,9 +2080,9 @@ __device__ __forceinline__ void coarse_values(const CoarseView &V, const double 
 // rounded value is the one used in the dot products and aggregate sums, so they describe the
 // stored vectors.
 template <class TS, bool WIN>
-__global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) {
+__global__ void __launch_bounds__(kCgResThreads<WIN>, 1) k_cg2l_resident(Cg2lArgs C) {
   extern __shared__ double s_dbl[];
-  __shared__ double s_grp[kCgResGroups][4][kBlock / 32];
+  __shared__ double s_grp[kCgResGroups<WIN>][4][kBlock / 32];
   __shared__ double s_tree[4][kBlock / 32];
   const CgResidentArgs &R = C.R;
   const CgPersistentArgs &A = R.P;
@@ -2074,7 +2111,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
   double *s_stage = ct + 3 * nc + 2;
   ResidentRows<TS, WIN> rows(R, Lsv, reinterpret_cast<char *>(s_stage + 2 * V.npos_max));
   const int b0 = rows.b0, b1 = rows.b1;
-  for (int m = threadIdx.x; m <= nc; m += kCgResThreads) {
+  for (int m = threadIdx.x; m <= nc; m += kCgResThreads<WIN>) {
     cc[0][m] = 0.0;
     cc[1][m] = 0.0;
     if (m < nc) cS[m] = 0.0;
@@ -2105,14 +2142,14 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
   const int v_r[1] = {0}, v_w[1] = {1}, v_rw[2] = {0, 1};
   // start: c0 = Z T(b) (phase 0, buffer 0)
   if (nc > 0) {
-    for (int i = b0 * kBlock + (int)threadIdx.x; i < min(n, b1 * kBlock); i += kCgResThreads) {
+    for (int i = b0 * kBlock + (int)threadIdx.x; i < min(n, b1 * kBlock); i += kCgResThreads<WIN>) {
       const int ps = __ldg(V.row_pos + i);
       if (ps >= 0) s_stage[ps] = (double)__ldcg(bvec + i);
     }
     __syncthreads();
     seg_sums<1>(V, s_stage, 0, v_r, scale);
     if (!grid_sync(A.bar, phase)) return;
-    for (int m = threadIdx.x; m < nc; m += kCgResThreads) ct[m] = sum_value(V, 0, 0, m, iscale);
+    for (int m = threadIdx.x; m < nc; m += kCgResThreads<WIN>) ct[m] = sum_value(V, 0, 0, m, iscale);
     __syncthreads();
     coarse_values<kZB>(V, ct, cc[0]);
     __syncthreads();
@@ -2122,7 +2159,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     return (double)__ldg(invLv + j) * (double)__ldcg(bvec + j) + cc[0][__ldg(V.agg + j)];
   };
   rows.fill(u0);
-  for (int b = b0 + g; b < b1; b += kCgResGroups) {
+  for (int b = b0 + g; b < b1; b += kCgResGroups<WIN>) {
     const int lp = (b - b0) * kBlock + lt;
     const int i = rows.row_of(lp);
     double v[2] = {0.0, 0.0};
@@ -2148,13 +2185,13 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
   if (!grid_sync(A.bar, phase)) return;
   {
     double d0[2];
-    tree_total_cta<2>(A.part_a, A.nblk_sell, d0, s_tree);
+    tree_total_cta<2, WIN>(A.part_a, A.nblk_sell, d0, s_tree);
     if (d0[0] == 0.0 || isnan(d0[0]) || isnan(d0[1]))
       status = KS_BREAKDOWN;
     else
       alpha = d0[1] / d0[0];
     gamma = d0[1];
-    for (int m = threadIdx.x; m < nc; m += kCgResThreads) coarse_input(m, ct[m], sum_value(V, 1, 1, m, iscale));
+    for (int m = threadIdx.x; m < nc; m += kCgResThreads<WIN>) coarse_input(m, ct[m], sum_value(V, 1, 1, m, iscale));
   }
   while (status == KS_RUNNING) {
     double *part = (it & 1) ? A.part_a : A.part_b;
@@ -2191,7 +2228,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     };
     own(b0 + g);
     rows.fill(uj);
-    for (int b = b0 + g; b < b1; b += kCgResGroups) {
+    for (int b = b0 + g; b < b1; b += kCgResGroups<WIN>) {
       double v[4] = {0.0, 0.0, 0.0, 0.0};
       if (i >= 0) {
         const double acc = rnd(rows.product(b, (b - b0) * kBlock + lt, uj));
@@ -2215,7 +2252,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
           s_stage[V.npos_max + ps] = acc;
         }
       }
-      own(b + kCgResGroups);
+      own(b + kCgResGroups<WIN>);
       group_partial<4>(v, part, b, g, s_grp);
     }
     if (nc > 0) {
@@ -2224,7 +2261,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     }
     if (!grid_sync(A.bar, phase)) return;
     double t[4];
-    tree_total_cta<4>(part, A.nblk_sell, t, s_tree);
+    tree_total_cta<4, WIN>(part, A.nblk_sell, t, s_tree);
     ++it;
     pc ^= 1;
     rn2 = A.scaled ? t[3] : t[2];
@@ -2250,7 +2287,7 @@ __global__ void __launch_bounds__(kCgResThreads, 1) k_cg2l_resident(Cg2lArgs C) 
     alpha = t[0] / den;
     beta = beta_new;
     gamma = t[0];
-    for (int m = threadIdx.x; m < nc; m += kCgResThreads)
+    for (int m = threadIdx.x; m < nc; m += kCgResThreads<WIN>)
       coarse_input(m, sum_value(V, buf, 0, m, iscale), sum_value(V, buf, 1, m, iscale));
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
