@@ -1254,7 +1254,7 @@ struct cfsa_ns {
     c.invL = invL;
     c.x = x;
     c.r = pr;
-    c.z = pz;
+    c.z = pt;
     c.q = pq;
     c.p[0] = pp;
     c.p[1] = ps;
@@ -1458,6 +1458,7 @@ struct cfsa_ns {
         launch_cg2l(cg2l_args(x, s_out, cs), false, stream);
       } else if (krylov == CFSA_KRYLOV_CG1) {
         CgResidentArgs rz = resident_caps(0, 2048);
+        c.z = pt;
         rz.P = c;
         Cg1Args c1{};
         c1.R = rz;
