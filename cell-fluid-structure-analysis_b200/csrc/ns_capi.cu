@@ -121,15 +121,15 @@ struct CoarseBuffers {
   int *first = nullptr, *id = nullptr, *slot = nullptr, *agg = nullptr, *rows = nullptr, *row_pos = nullptr,
       *scal = nullptr, *list = nullptr, *cnt = nullptr, *ptr = nullptr, *npieces = nullptr, *need = nullptr,
       *nneed = nullptr;
-  double *bounds = nullptr, *A = nullptr, *T = nullptr, *Z = nullptr;
+  double *bounds = nullptr, *A = nullptr, *diag = nullptr, *T = nullptr, *Z = nullptr;
   int4 *pieces = nullptr;
   size_t cap_key = 0, cap_gacc = 0, cap_first = 0, cap_id = 0, cap_slot = 0, cap_agg = 0, cap_rows = 0, cap_pos = 0,
          cap_scal = 0, cap_list = 0, cap_cnt = 0, cap_ptr = 0, cap_npieces = 0, cap_need = 0, cap_nneed = 0,
-         cap_bounds = 0, cap_A = 0, cap_T = 0, cap_Z = 0, cap_pieces = 0;
+         cap_bounds = 0, cap_A = 0, cap_diag = 0, cap_T = 0, cap_Z = 0, cap_pieces = 0;
   ~CoarseBuffers() {
     for (void *p : {(void *)key, (void *)gacc, (void *)first, (void *)id, (void *)slot, (void *)agg, (void *)rows,
                     (void *)row_pos, (void *)scal, (void *)list, (void *)cnt, (void *)ptr, (void *)npieces,
-                    (void *)need, (void *)nneed, (void *)bounds, (void *)A, (void *)T, (void *)Z, (void *)pieces})
+                    (void *)need, (void *)nneed, (void *)bounds, (void *)A, (void *)diag, (void *)T, (void *)Z, (void *)pieces})
       cudaFree(p);
   }
 };
@@ -882,6 +882,7 @@ struct cfsa_ns {
       coarse_grow(B.cnt, B.cap_cnt, (size_t)nc);
       coarse_grow(B.ptr, B.cap_ptr, (size_t)nc + 1);
       coarse_grow(B.A, B.cap_A, nn);
+      coarse_grow(B.diag, B.cap_diag, (size_t)nc * kPanel);
       coarse_grow(B.T, B.cap_T, nn);
       coarse_grow(B.Z, B.cap_Z, nn);
       coarse_grow(B.gacc, B.cap_gacc, (size_t)27 * nc);
@@ -901,13 +902,13 @@ struct cfsa_ns {
       for (int j0 = 0; j0 < nc; j0 += kPanel) {
         const unsigned int g = (unsigned int)((nc - j0 + kPanel - 1) / kPanel);
         if (j0 > 0) k_chol_update<<<g, 1024, 0, stream>>>(nc, j0, B.A);
-        k_chol_panel<<<g, 32, 0, stream>>>(nc, j0, B.A, B.scal + 2);
+        k_chol_panel<<<g, 32, 0, stream>>>(nc, j0, B.A, B.diag, B.scal + 2);
       }
       CK(cudaGetLastError());
       int spd = 0;
       CK(cudaMemcpyAsync(&spd, B.scal + 2, sizeof(int), cudaMemcpyDeviceToHost, stream));
       const dim3 tiles((nc + 31) / 32, (nc + 31) / 32);
-      k_transpose<<<tiles, kBlock, 0, stream>>>(nc, B.A, B.T);
+      k_transpose<<<tiles, kBlock, 0, stream>>>(nc, B.A, B.diag, B.T);
       CK(cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nc * sizeof(double))));
       k_coarse_inverse<<<nc, 512, nc * sizeof(double), stream>>>(nc, B.T, B.A);
       k_coarse_z<<<dim3((nc + 31) / 32, (nc + 7) / 8), kBlock, 0, stream>>>(nc, B.A, B.Z);

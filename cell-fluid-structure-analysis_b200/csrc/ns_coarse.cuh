@@ -189,7 +189,9 @@ __global__ void k_coarse_matrix(int nc, const int *__restrict__ ptr, const int *
 
 // Cholesky A_c = G G^T in panels of kPanel columns, G over the lower triangle of the matrix A. Element
 // (i, j) subtracts G(i,k) G(j,k) for k = 0, 1, ... in order: first the columns before the panel
-// (k_chol_update), then those inside it (k_chol_panel).
+// (k_chol_update), then those inside it (k_chol_panel). The factored diagonal blocks go to `diag`
+// ([n][kPanel]) and not back to A: the CTAs of a panel launch are not ordered, and one that starts late
+// must still find the unfactored block there. Later panels read rows below the block only.
 constexpr int kPanel = 32;
 
 __global__ void k_chol_update(int n, int j0, double *__restrict__ A) {
@@ -209,8 +211,8 @@ __global__ void k_chol_update(int n, int j0, double *__restrict__ A) {
 }
 
 // One warp per CTA: every CTA factors the diagonal block (lane = row), then takes its 32 rows below it
-// (CTA 0 writes the block instead). A pivot that is not positive clears *spd.
-__global__ void k_chol_panel(int n, int j0, double *__restrict__ A, int *spd) {
+// (CTA 0 writes the factored block to `diag` instead). A pivot that is not positive clears *spd.
+__global__ void k_chol_panel(int n, int j0, double *__restrict__ A, double *__restrict__ diag, int *spd) {
   __shared__ double s_g[kPanel][kPanel + 1];
   const int lane = threadIdx.x, w = min(kPanel, n - j0);
   double a[kPanel];
@@ -232,7 +234,7 @@ __global__ void k_chol_panel(int n, int j0, double *__restrict__ A, int *spd) {
   }
   __syncwarp();
   if (blockIdx.x == 0) {
-    for (int k = 0; k <= lane && lane < w; ++k) A[(size_t)(j0 + lane) * n + j0 + k] = s_g[lane][k];
+    for (int k = 0; k <= lane && lane < w; ++k) diag[(size_t)(j0 + lane) * kPanel + k] = s_g[lane][k];
     if (lane == 0 && !ok) *spd = 0;
     return;
   }
@@ -250,11 +252,18 @@ __global__ void k_chol_panel(int n, int j0, double *__restrict__ A, int *spd) {
   for (int k = 0; k < kPanel; ++k) A[(size_t)i * n + j0 + k] = a[k];
 }
 
-__global__ void k_transpose(int n, const double *__restrict__ A, double *__restrict__ T) {
+// T = G transposed: the lower triangle of A with the diagonal blocks from `diag` (tiles are panels).
+__global__ void k_transpose(int n, const double *__restrict__ A, const double *__restrict__ diag,
+                            double *__restrict__ T) {
+  static_assert(kPanel == 32, "a tile of the transposition is a panel");
   __shared__ double s[32][33];
   const int x = 32 * blockIdx.x + (threadIdx.x & 31), y0 = 32 * blockIdx.y;
   for (int r = threadIdx.x >> 5; r < 32; r += blockDim.x >> 5)
-    if (x < n && y0 + r < n) s[r][threadIdx.x & 31] = A[(size_t)(y0 + r) * n + x];
+    if (x <= y0 + r && y0 + r < n)
+      s[r][threadIdx.x & 31] = (blockIdx.x == blockIdx.y) ? diag[(size_t)(y0 + r) * kPanel + (threadIdx.x & 31)]
+                                                          : A[(size_t)(y0 + r) * n + x];
+    else
+      s[r][threadIdx.x & 31] = 0.0;  // above the diagonal
   __syncthreads();
   const int tx = y0 + (int)(threadIdx.x & 31);
   for (int r = threadIdx.x >> 5; r < 32; r += blockDim.x >> 5)

@@ -1,5 +1,7 @@
 """Resident Krylov solves at the sizes where their partitions can go wrong, bit for bit against the
 oracle (same sums in the same order), and the pressure solvers with and without column windows."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -92,3 +94,37 @@ def test_coarse_space_matches_oracle(cf, po, shape, target):
     assert s.pisoStep() and o.piso_step() == 0
     ref = o.state()
     assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
+
+
+def test_coarse_space_rebuilt_while_another_handle_solves(cf):
+    """The CTAs of one launch of the factorisation are not ordered: with another handle's resident solves
+    holding the SMs they start one by one, and the coarse space must still come out the same to the bit."""
+    m, busy = mesh(cf, (6, 30)), mesh(cf, (8, 60))
+    x = m.vertices()
+    s = solver(cf, m, cf.KRYLOV_CG, cf.KRYLOV_CG2L)
+    s.setCoarseTarget(700)
+    assert s.pisoStep()
+    u, p = s.getVelocity().copy(), s.getPressure().copy()
+    assert s.pisoStep()
+    ref = s.getVelocity().copy(), s.getPressure().copy()
+    t = solver(cf, busy, cf.KRYLOV_CG, cf.KRYLOV_CG, 1e-12)
+    stop, ok = threading.Event(), []
+
+    def keep_stepping():
+        while not stop.is_set():
+            ok.append(t.pisoStep())
+
+    worker = threading.Thread(target=keep_stepping)
+    worker.start()
+    try:
+        for _ in range(20):
+            s.updateVertices(x * [1.0, 1.01, 0.99])
+            s.coarseSize()
+            s.updateVertices(x)
+            s.setFields(u, p)
+            assert s.pisoStep()
+            assert np.array_equal(s.getVelocity(), ref[0]) and np.array_equal(s.getPressure(), ref[1])
+    finally:
+        stop.set()
+        worker.join()
+    assert ok and all(ok)
