@@ -453,6 +453,19 @@ struct cfsa_ns {
     return r;
   }
 
+  // Raises the kernel's limit of dynamic shared memory to all that the device leaves beside its static
+  // part, and checks that a CTA with `smem` bytes fits. The limit belongs to the function and not to the
+  // handle: every handle sets the same value, so none lowers it for another handle's larger mesh, nor for
+  // a launch that another thread is about to make.
+  void allow_shared(const void *fn, int threads, size_t smem, const char *what) const {
+    cudaFuncAttributes fa{};
+    CK(cudaFuncGetAttributes(&fa, fn));
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - (int)fa.sharedSizeBytes));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+    if (per_sm < 1) throw CudaError{std::string(what) + ": kernel does not fit on an SM"};
+  }
+
   void build_pattern(bool p2, int nrows, std::vector<int> &h_rp, int *&d_rp, int *&d_ci,
                      int64_t &nnz, int *d_err) {
     int *counts = dalloc<int>(nrows);
@@ -727,12 +740,7 @@ struct cfsa_ns {
           {(const void *)k_cg_resident<true>, kCgResThreads<true>},    {(const void *)k_cg_resident<false>, kCgResThreads<false>},
           {(const void *)k_cg1_resident<true>, kCgResThreads<true>},   {(const void *)k_cg1_resident<false>, kCgResThreads<false>},
           {(const void *)k_bicg_resident<true>, kCgResThreads<true>},  {(const void *)k_bicg_resident<false>, kCgResThreads<false>}};
-      for (const auto &[fn, threads] : kernels) {
-        int o = 0;
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_res_smem));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, threads, cg_res_smem));
-        if (o < 1) throw CudaError{"resident pressure solver does not fit on an SM"};
-      }
+      for (const auto &[fn, threads] : kernels) allow_shared(fn, threads, cg_res_smem, "resident pressure solver");
     }
     if (const char *e = std::getenv("CFSA_CG_LOOP")) cg_persistent = cg_persistent && (std::atoi(e) == 0);
     // CFSA_CG_KERNEL=persistent selects the 256-thread persistent kernel over the resident one
@@ -909,7 +917,7 @@ struct cfsa_ns {
       CK(cudaMemcpyAsync(&spd, B.scal + 2, sizeof(int), cudaMemcpyDeviceToHost, stream));
       const dim3 tiles((nc + 31) / 32, (nc + 31) / 32);
       k_transpose<<<tiles, kBlock, 0, stream>>>(nc, B.A, B.diag, B.T);
-      CK(cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nc * sizeof(double))));
+      allow_shared((const void *)k_coarse_inverse, 512, nc * sizeof(double), "inverse of the coarse space");
       k_coarse_inverse<<<nc, 512, nc * sizeof(double), stream>>>(nc, B.T, B.A);
       k_coarse_z<<<dim3((nc + 31) / 32, (nc + 7) / 8), kBlock, 0, stream>>>(nc, B.A, B.Z);
       CoarseListArgs l{};
@@ -927,7 +935,7 @@ struct cfsa_ns {
       l.nneed = B.nneed;
       l.need_stride = nc;
       const size_t list_smem = ((size_t)cg_res_bpc_sell * kBlock + 2 * (size_t)nc + (nc + 31) / 32) * sizeof(int);
-      CK(cudaFuncSetAttribute(k_coarse_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem));
+      allow_shared((const void *)k_coarse_lists, 1024, list_smem, "lists of the coarse space");
       k_coarse_lists<<<cg_res_grid, 1024, list_smem, stream>>>(l);
       CK(cudaGetLastError());
       CK(cudaStreamSynchronize(stream));
@@ -967,12 +975,7 @@ struct cfsa_ns {
     if (!cg2l_caps.row_cap) throw CudaError{"two-level pressure preconditioner: coarse space too large for shared memory"};
     cg2l_smem = (size_t)coarse_bytes +
                 resident_rows_bytes(cg2l_caps.row_cap, cg2l_caps.win_cap, cg2l_caps.ent_cap, cg2l_caps.val_cap);
-    for (const auto &[fn, threads] : kernels) {
-      CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg2l_smem));
-      int o = 0;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, threads, cg2l_smem));
-      if (o < 1) throw CudaError{"two-level pressure preconditioner: kernel does not fit on an SM"};
-    }
+    for (const auto &[fn, threads] : kernels) allow_shared(fn, threads, cg2l_smem, "two-level pressure preconditioner");
     // the view is a captured launch argument; the shared-memory layout follows from it
     if (std::memcmp(&V, &coarse_view, sizeof(V)) != 0) graph_dirty = true;
     coarse_view = V;

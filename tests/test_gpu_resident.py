@@ -128,3 +128,22 @@ def test_coarse_space_rebuilt_while_another_handle_solves(cf):
         stop.set()
         worker.join()
     assert ok and all(ok)
+
+
+# The resident kernels' dynamic shared memory follows the handle's mesh, but the limit set for it belongs
+# to the function: a smaller handle made later must not lower it for a larger one.
+@pytest.mark.parametrize("pressure", [0, 1, 2, 3], ids=["cg", "bicgstab", "cg1", "cg2l"])
+def test_small_handle_leaves_larger_one_its_shared_memory(cf, pressure):
+    big, small = mesh(cf, (10, 58)), mesh(cf, (1, 2))
+    alone = solver(cf, big, cf.KRYLOV_CG, pressure, 1e-8)
+    assert alone.pisoStep() and alone.simpleStep()
+    s = solver(cf, big, cf.KRYLOV_CG, pressure, 1e-8)
+    t = solver(cf, small, cf.KRYLOV_CG, pressure, 1e-8)
+    assert t.pisoStep()
+    assert s.pisoStep()  # captured after the small handle was made
+    t.updateVertices(small.vertices() * [1.0, 1.01, 0.99])  # rebuilds the small coarse space
+    assert t.pisoStep()
+    assert s.simpleStep()  # launched without a graph
+    assert np.array_equal(s.getVelocity(), alone.getVelocity()) and np.array_equal(s.getPressure(), alone.getPressure())
+    rhs = np.ones(s.nv)
+    assert np.array_equal(s.solvePressureBiCGSTAB(rhs, None, 1e-8, 50)[0], alone.solvePressureBiCGSTAB(rhs, None, 1e-8, 50)[0])
