@@ -215,6 +215,7 @@ def load_library(path: str | os.PathLike | None = None) -> C.CDLL:
         "cfsa_ns_get_inv_lumped_mass": (i32, [vp, vp]),
         "cfsa_ns_profile_kernel": (i32, [vp, i32, i32, vp, vp]),
         "cfsa_ns_set_barrier_spin_limit": (i32, [vp, C.c_int64]),
+        "cfsa_ns_set_momentum_barrier_spin_limit": (i32, [vp, C.c_int64]),
         "cfsa_ns_solve_pressure_bicgstab": (i32, [vp, vp, vp, dbl, i32]),
         "cfsa_ns_compute_divergence_noalloc": (i32, [vp, vp, vp]),
         "cfsa_ns_objective": (i32, [vp, vp, vp]),
@@ -715,6 +716,10 @@ class NavierStokesSolver:
         """Polls a waiting CTA of the resident pressure solvers makes at a grid barrier before it
         gives up (the step then fails with CUDA_ERROR); < 0 restores the default."""
         self._check(self._lib.cfsa_ns_set_barrier_spin_limit(self._h, int(polls)))
+
+    def setMomentumBarrierSpinLimit(self, polls: int):
+        """The same for the momentum solves."""
+        self._check(self._lib.cfsa_ns_set_momentum_barrier_spin_limit(self._h, int(polls)))
 
     def invLumpedMass(self) -> np.ndarray:
         out = np.empty(self.N2)

@@ -226,7 +226,8 @@ struct cfsa_ns {
   double *pv2 = nullptr, *pp2 = nullptr;  // second buffers of the pressure BiCGSTAB's v and p
   unsigned int *bar_count = nullptr;
   int *bar_err = nullptr;
-  long long bar_spin_limit = kBarrierSpinLimit;
+  long long bar_spin_limit = kBarrierSpinLimit;      // pressure solves
+  long long mom_bar_spin_limit = kBarrierSpinLimit;  // momentum solves
   // raw Poisson operator of solvePressureBiCGSTAB (no penalty rows), column-scaled by its inverse
   // diagonal like Lt; built on first use and again after the geometry changed
   double *Lraw_t = nullptr, *diag_raw = nullptr, *inv_raw = nullptr;
@@ -1060,7 +1061,7 @@ struct cfsa_ns {
     const int chunks = resident_chunks(S);
     const size_t slot_bytes = (size_t)chunks * 6 * sizeof(double);
     ResidentArgs r{};
-    r.bar = GridBarrier{bar_count, bar_err, kBarrierSpinLimit};
+    r.bar = GridBarrier{bar_count, bar_err, mom_bar_spin_limit};
     r.part = res_part;
     r.stride = res_stride;
     r.slots = slot_bytes > kMaxSlotBytes ? res_slots : nullptr;
@@ -1379,7 +1380,7 @@ struct cfsa_ns {
     a.R.P.nblk_nat = (int)blocks_for(nv);
     a.R.P.part_a = cg_part_a;
     a.R.P.part_b = cg_part_b;
-    a.R.P.bar = GridBarrier{bar_count, bar_err, kBarrierSpinLimit};
+    a.R.P.bar = GridBarrier{bar_count, bar_err, bar_spin_limit};
     a.p2 = pp2;
     a.v2 = pv2;
     clear_barrier(stream);
@@ -2655,6 +2656,7 @@ int cfsa_ns_momentum_predictor(cfsa_ns *h) {
     h->enqueue_momentum(false);
     CK(cudaMemcpyAsync(h->h_st, h->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    if (h->h_st->code == CFSA_CUDA_ERROR) h->err = step_failure(h->h_st->code);
     return h->h_st->code;
   });
 }
@@ -2668,6 +2670,7 @@ int cfsa_ns_pressure_poisson(cfsa_ns *h) {
     h->enqueue_pressure_update();
     CK(cudaMemcpyAsync(h->h_st, h->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    if (h->h_st->code == CFSA_CUDA_ERROR) h->err = step_failure(h->h_st->code);
     return h->h_st->code;
   });
 }
@@ -2679,6 +2682,7 @@ int cfsa_ns_solve_pressure_bicgstab(cfsa_ns *h, const double *rhs, double *x, do
     const int code = h->solve_poisson_raw(rhs, x, tol, maxit);
     if (code == CFSA_NOT_CONVERGED) h->err = "BiCGSTAB failed: no convergence within the iteration cap";
     if (code == CFSA_BREAKDOWN) h->err = "BiCGSTAB failed: breakdown";
+    if (code == CFSA_CUDA_ERROR) h->err = "BiCGSTAB failed: gave up waiting at a grid barrier";
     return code;
   });
 }
@@ -3161,12 +3165,21 @@ int cfsa_ns_get_adjoint_stats(cfsa_ns *h, cfsa_adjoint_stats *out) {
 
 }  // extern "C"
 
-extern "C" int cfsa_ns_set_barrier_spin_limit(cfsa_ns *h, int64_t polls) {
+// The limits are captured launch arguments.
+static int set_spin_limit(cfsa_ns *h, long long cfsa_ns::*which, int64_t polls) {
   if (!h) return CFSA_BAD_ARG;
   const long long lim = polls < 0 ? kBarrierSpinLimit : (long long)polls;
-  if (lim != h->bar_spin_limit) h->graph_dirty = true;  // the limit is a captured launch argument
-  h->bar_spin_limit = lim;
+  if (lim != h->*which) h->graph_dirty = true;
+  h->*which = lim;
   return CFSA_OK;
+}
+
+extern "C" int cfsa_ns_set_barrier_spin_limit(cfsa_ns *h, int64_t polls) {
+  return set_spin_limit(h, &cfsa_ns::bar_spin_limit, polls);
+}
+
+extern "C" int cfsa_ns_set_momentum_barrier_spin_limit(cfsa_ns *h, int64_t polls) {
+  return set_spin_limit(h, &cfsa_ns::mom_bar_spin_limit, polls);
 }
 
 extern "C" int cfsa_ns_profile_kernel(cfsa_ns *h, int which, int iters, double *avg_ms,

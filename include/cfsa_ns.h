@@ -256,12 +256,14 @@ int cfsa_ns_get_inv_lumped_mass(cfsa_ns *h, double *out /*[N2]*/);
  * avg_ms: mean duration of one run; alg_bytes: algorithmic bytes one run must move (matrix values and
  * column indices, row metadata, each vector element read or written once). */
 int cfsa_ns_profile_kernel(cfsa_ns *h, int which, int iters, double *avg_ms, double *alg_bytes);
-/* Bound on the polls a CTA of the resident pressure solvers (CG, CFSA_KRYLOV_CG1, CG2L) makes at
- * a grid barrier before it gives up: the solve then stops, the step fails with CFSA_CUDA_ERROR
- * ("gave up waiting at a grid barrier"), time does not advance, and the handle stays usable.
- * polls < 0 restores the default (2^22 polls, over two seconds; the bound of the other resident solves); 0 gives up at the first wait, which
- * tests use to exercise the failure path. */
+/* Bound on the polls a CTA of the resident pressure solvers (CG, CFSA_KRYLOV_CG1, CG2L, BiCGSTAB and
+ * cfsa_ns_solve_pressure_bicgstab) makes at a grid barrier before it gives up: the solve then stops, the
+ * step fails with CFSA_CUDA_ERROR ("gave up waiting at a grid barrier"), time does not advance, and the
+ * handle stays usable. polls < 0 restores the default (2^22 polls, over two seconds); 0 gives up at the
+ * first wait, which tests use to exercise the failure path. */
 int cfsa_ns_set_barrier_spin_limit(cfsa_ns *h, int64_t polls);
+/* The same for the momentum solves (CG and BiCGSTAB, FP64 and mixed precision). */
+int cfsa_ns_set_momentum_barrier_spin_limit(cfsa_ns *h, int64_t polls);
 
 /* ---- allocation-free operator (no counterpart in the reference) ---- */
 /* Divergence (the computeDivergence operator above) for callers that cannot allocate device

@@ -147,3 +147,41 @@ def test_small_handle_leaves_larger_one_its_shared_memory(cf, pressure):
     assert np.array_equal(s.getVelocity(), alone.getVelocity()) and np.array_equal(s.getPressure(), alone.getPressure())
     rhs = np.ones(s.nv)
     assert np.array_equal(s.solvePressureBiCGSTAB(rhs, None, 1e-8, 50)[0], alone.solvePressureBiCGSTAB(rhs, None, 1e-8, 50)[0])
+
+
+# A wait that runs out in a momentum solve or in the pressure BiCGSTAB: the first wait gives up on its own,
+# the host reads the status word, and the handle steps on. The small mesh's momentum solve is one CTA.
+@pytest.mark.parametrize("shape", [(2, 5), (3, 12)], ids=["one_cta", "grid"])
+@pytest.mark.parametrize("solve", ["momentum_cg", "momentum_bicgstab", "mixed_cg", "mixed_bicgstab", "pressure_bicgstab"])
+@pytest.mark.parametrize("graph", [True, False], ids=["graph", "eager"])
+def test_resident_solve_wait_runs_out(cf, shape, solve, graph):
+    m = mesh(cf, shape)
+
+    def make():
+        s = solver(cf, m, cf.KRYLOV_CG if solve.endswith("_cg") else cf.KRYLOV_BICGSTAB, cf.KRYLOV_BICGSTAB)
+        if solve.startswith("mixed"):
+            s.setPrecision(cf.PRECISION_MIXED)
+        return s
+
+    ref, s = make(), make()
+    step = (lambda q: q.pisoStep()) if graph else (lambda q: q.simpleStep())
+    assert step(ref)
+    u0, p0 = s.getVelocity().copy(), s.getPressure().copy()
+    limit = s.setBarrierSpinLimit if solve.startswith("pressure") else s.setMomentumBarrierSpinLimit
+    limit(0)
+    with pytest.raises(cf.CfsaError, match="grid barrier") as e:
+        step(s)
+    assert e.value.code == cf.CUDA_ERROR
+    assert s.getTime() == 0.0
+    assert np.array_equal(s.getVelocity(), u0) and np.array_equal(s.getPressure(), p0)
+    half = s.solvePressurePoisson if solve == "pressure_bicgstab" else s.solveMomentumPredictor
+    with pytest.raises(cf.CfsaError, match="grid barrier"):
+        half()
+    if solve == "pressure_bicgstab":
+        with pytest.raises(cf.CfsaError, match="grid barrier"):
+            s.solvePressureBiCGSTAB(np.ones(s.nv))
+    limit(-1)
+    s.setFields(u0, p0)
+    assert step(s)
+    assert np.array_equal(s.getVelocity(), ref.getVelocity()) and np.array_equal(s.getPressure(), ref.getPressure())
+    assert s.getTime() == ref.getTime() > 0.0
