@@ -2239,20 +2239,24 @@ struct cfsa_ns {
     return CFSA_OK;
   }
 
+  // Waits for `stream`; a run that gave up at a grid barrier was cut short and has no time to report.
+  void check_barrier() {
+    int gave_up = 0;
+    CK(cudaMemcpyAsync(&gave_up, bar_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    if (gave_up) throw CudaError{"profile: the kernel gave up waiting at a grid barrier"};
+  }
+
   // Kernel timing on the live data with private Krylov states (solver state untouched).
   void profile_kernel(int which, int iters, double *avg_ms, double *alg_bytes) {
     NvtxRange nvtx_("cfsa profile kernel");  // lets a profiler select these launches
     ensure_operators();
     CK(cudaStreamSynchronize(stream));
     if (which == CFSA_KERNEL_MOMENTUM_SPMV_F32) {
-      MixedState hm{};
-      hm.active = 7;
-      CK(cudaMemcpyAsync(ms_prof, &hm, sizeof(hm), cudaMemcpyHostToDevice, stream));
       MixedArgs a = mixed_args(ustar, nullptr);
       a.ms = ms_prof;
-      // input: the velocity rounded to float (nonzero wherever the flow is, so neither method's
-      // dot product vanishes; a zero p.q would end the CG product early); fs and ft are FP32 Krylov
-      // scratch that every mixed solve rewrites before reading
+      // input: the velocity rounded to float; fs and ft are FP32 Krylov scratch that every mixed solve
+      // rewrites before reading
       k_to_f32<<<blocks_for(3 * N2), kBlock, 0, stream>>>(3 * N2, u, fs);
       a.p = fs;
       a.r0 = fs;
@@ -2263,11 +2267,6 @@ struct cfsa_ns {
       CK(cudaEventRecord(ev1, stream));
       *alg_bytes = 8.0 * (double)nnz2 + 8.0 * s2.nrows_pad + 4.0 * (s2.nslices + 1) + 36.0 * (double)N2;
     } else if (which == CFSA_KERNEL_MOMENTUM_SPMV) {
-      BicgState hs{};
-      hs.active = 7;
-      hs.ncomp = 3;
-      for (int c = 0; c < 3; ++c) hs.rho[c] = 1.0;
-      CK(cudaMemcpyAsync(bs_prof, &hs, sizeof(hs), cudaMemcpyHostToDevice, stream));
       BicgArgs a = momentum_args();
       a.bs = bs_prof;
       a.st = nullptr;
@@ -2320,8 +2319,7 @@ struct cfsa_ns {
         enqueue_pressure_krylov(false, pv, st_free);
         CK(cudaEventRecord(ev1, stream));
         CK(cudaMemcpyAsync(h_cs, cs, sizeof(CgState), cudaMemcpyDeviceToHost, stream));
-        CK(cudaEventSynchronize(ev1));
-        CK(cudaStreamSynchronize(stream));
+        check_barrier();
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, ev0, ev1));
         total += ms;
@@ -2340,7 +2338,10 @@ struct cfsa_ns {
       throw CudaError{"unknown kernel id"};
     }
     CK(cudaGetLastError());
-    CK(cudaEventSynchronize(ev1));
+    if (which == CFSA_KERNEL_PRESSURE_SPMV)
+      CK(cudaEventSynchronize(ev1));  // no barrier in it
+    else
+      check_barrier();
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, ev0, ev1));
     *avg_ms = (double)ms / (double)std::max(1, iters);

@@ -185,3 +185,21 @@ def test_resident_solve_wait_runs_out(cf, shape, solve, graph):
     assert step(s)
     assert np.array_equal(s.getVelocity(), ref.getVelocity()) and np.array_equal(s.getPressure(), ref.getPressure())
     assert s.getTime() == ref.getTime() > 0.0
+
+
+# A profiled run that was cut short at a grid barrier is an error, not a fast kernel.
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_profile_of_a_run_that_gave_up_fails(cf, precision):
+    s = solver(cf, mesh(cf, (3, 12)), cf.KRYLOV_CG, cf.KRYLOV_CG1)
+    assert s.pisoStep()
+    u = s.getVelocity().copy()
+    which = cf.KERNEL_MOMENTUM_SPMV_F32 if precision else cf.KERNEL_MOMENTUM_SPMV
+    for limit, kernel in ((s.setMomentumBarrierSpinLimit, which), (s.setBarrierSpinLimit, cf.KERNEL_PRESSURE_SOLVE)):
+        limit(0)
+        with pytest.raises(cf.CfsaError, match="grid barrier"):
+            s.profileKernel(kernel, 3)
+        s.profileKernel(cf.KERNEL_PRESSURE_SPMV, 3)  # has no barrier
+        limit(-1)
+        ms, by = s.profileKernel(kernel, 3)
+        assert ms > 0.0 and by > 0.0
+    assert np.array_equal(s.getVelocity(), u)
