@@ -326,8 +326,11 @@ __global__ void k_momentum_diag(int n, double dt, const int *__restrict__ dpos,
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int k = dpos[i];
-  double d = Mv[k] / dt + Kv[k];
-  if (bc[i] == BC_INLET || bc[i] == BC_WALL) d += kMomentumPenalty;
+  double d = 0.0;
+  if (k >= 0) {  // a vertex of no tet has an empty row
+    d = Mv[k] / dt + Kv[k];
+    if (bc[i] == BC_INLET || bc[i] == BC_WALL) d += kMomentumPenalty;
+  }
   diagA[i] = d;
   invA[i] = (d != 0.0) ? 1.0 / d : 1.0;
 }
@@ -364,9 +367,13 @@ __global__ void k_poisson_diag(int n, int outlet_type, int ref_node, const int *
                                double *__restrict__ diagL, double *__restrict__ invL) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double d = Lv[dpos[i]];
-  if ((outlet_type == 1 && i == ref_node) || (outlet_type == 0 && bc[i] == BC_OUTLET))
-    d += kPoissonPenalty;
+  const int k = dpos[i];
+  double d = 0.0;
+  if (k >= 0) {  // a vertex of no tet has an empty row
+    d = Lv[k];
+    if ((outlet_type == 1 && i == ref_node) || (outlet_type == 0 && bc[i] == BC_OUTLET))
+      d += kPoissonPenalty;
+  }
   diagL[i] = d;
   invL[i] = (d != 0.0) ? 1.0 / d : 1.0;
 }

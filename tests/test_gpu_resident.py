@@ -203,3 +203,29 @@ def test_profile_of_a_run_that_gave_up_fails(cf, precision):
         ms, by = s.profileKernel(kernel, 3)
         assert ms > 0.0 and by > 0.0
     assert np.array_equal(s.getVelocity(), u)
+
+
+# Vertices of no tet (left over in a mesh file): empty rows and columns, which neither the diagonals nor the
+# CTAs' shares of the rows may trip over.
+@pytest.mark.parametrize("extra", [1, 20])
+@pytest.mark.parametrize("momentum,pressure", [(0, 0), (1, 1), (0, 2), (0, 3)], ids=["cg", "bicgstab", "cg1", "cg2l"])
+def test_vertices_of_no_tet(cf, po, extra, momentum, pressure):
+    t = mesh(cf, (3, 12))
+    inside = t.vertices().min(0) + np.random.default_rng(7).uniform(0.3, 0.7, (extra, 3)) * np.ptp(t.vertices(), axis=0)
+    m = cf.Mesh.fromArrays(np.vstack([t.vertices(), inside]), t.tets())
+    m.setupBoundaryConditions((1.0, 0.0, 0.0), 1.0)
+    s = solver(cf, m, momentum, pressure)
+    o = po.Oracle(m.vertices(), m.tets())
+    o.set_fluid(RHO, NU)
+    o.set_params(dt=0.01, tol_mom=1e-11, tol_p=1e-11, maxit_mom=5000, maxit_p=20000,
+                 pressure_solver={0: 1, 1: 0, 2: 2, 3: 3}[pressure])
+    o.set_momentum_solver(1 if momentum == cf.KRYLOV_CG else 0)
+    o.initialize()
+    inlet = np.zeros((o.N2, 3))
+    inlet[:, 0] = 0.5
+    o.set_inlet(inlet)
+    for _ in range(2):
+        assert s.pisoStep() and o.piso_step() == 0
+    ref = o.state()
+    assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
+    assert s.stats()["pressure_iters"] == o.stats()["pressure_iters"] > 0
