@@ -78,6 +78,7 @@ std::vector<int> slice_runs(const std::vector<int> &sptr, int cut, int nslices, 
   const int64_t na = sptr[cut], n = sptr[nslices];
   for (int c = 0; c <= nruns; ++c)
     f.push_back(boundary(0, cut, na * c / nruns));
+  f[nruns] = cut;  // slices without entries (vertices of no tet) may end the first part
   for (int c = 0; c <= nruns; ++c) {
     const int64_t target = std::max(na, na + n * c / nruns - sptr[f[c]]);
     f.push_back(boundary(cut, nslices, target));

@@ -207,7 +207,8 @@ def test_profile_of_a_run_that_gave_up_fails(cf, precision):
 
 # Vertices of no tet (left over in a mesh file): empty rows and columns, which neither the diagonals nor the
 # CTAs' shares of the rows may trip over.
-@pytest.mark.parametrize("extra", [1, 20])
+# 600: whole 256-row blocks of empty rows end the vertex part.
+@pytest.mark.parametrize("extra", [1, 20, 600])
 @pytest.mark.parametrize("momentum,pressure", [(0, 0), (1, 1), (0, 2), (0, 3)], ids=["cg", "bicgstab", "cg1", "cg2l"])
 def test_vertices_of_no_tet(cf, po, extra, momentum, pressure):
     t = mesh(cf, (3, 12))
