@@ -223,6 +223,8 @@ struct cfsa_ns {
   size_t cg_res_smem = 0;
   double *res_part = nullptr;  // block partials of the resident Krylov solves, [2][kMaxRed][res_stride]
   int res_stride = 0;
+  int form_threads = 0;      // threads per CTA of the momentum solves; 0: by size
+  bool sums_global = false;  // chunk sums in res_slots at any size
   double *res_slots = nullptr;  // their chunk sums where shared memory would cost too much L1
   double *pv2 = nullptr, *pp2 = nullptr;  // second buffers of the pressure BiCGSTAB's v and p
   unsigned int *bar_count = nullptr;
@@ -744,6 +746,13 @@ struct cfsa_ns {
           {(const void *)k_bicg_resident<true>, kCgResThreads<true>},  {(const void *)k_bicg_resident<false>, kCgResThreads<false>}};
       for (const auto &[fn, threads] : kernels) allow_shared(fn, threads, cg_res_smem, "resident pressure solver");
     }
+    // CFSA_RESIDENT_THREADS=256|512|1024, CFSA_SUMS_GLOBAL=1: a momentum solve's form and the place of its
+    // chunk sums whatever the size, as on meshes that are larger or smaller
+    if (const char *e = std::getenv("CFSA_RESIDENT_THREADS")) {
+      const int t = std::atoi(e);
+      if (t == 256 || t == 512 || t == 1024) form_threads = t;
+    }
+    if (const char *e = std::getenv("CFSA_SUMS_GLOBAL")) sums_global = std::atoi(e) != 0;
     if (const char *e = std::getenv("CFSA_CG_LOOP")) cg_persistent = cg_persistent && (std::atoi(e) == 0);
     // CFSA_CG_KERNEL=persistent selects the 256-thread persistent kernel over the resident one
     if (const char *e = std::getenv("CFSA_CG_KERNEL"))
@@ -1053,10 +1062,14 @@ struct cfsa_ns {
   //   355,395     61.3 / 110     56.1 / 106    79.0 / 147
   //   696,987     104 / 215      112 / 234     151 / 304
   static constexpr int kFewRows = 90000, kManyRows = 450000;
-#define CFSA_RESIDENT(kernel, args, S, s, ...)                                                              \
-  ((S).nrows < kFewRows    ? launch_resident(kernel<256, 8 __VA_OPT__(, 8)>, 256, args, S, s)              \
-   : (S).nrows < kManyRows ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)             \
-                           : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
+  int resident_threads(const Sell &S) const {
+    if (form_threads) return form_threads;
+    return S.nrows < kFewRows ? 256 : S.nrows < kManyRows ? 512 : 1024;
+  }
+#define CFSA_RESIDENT(kernel, args, S, s, ...)                                                               \
+  (resident_threads(S) == 256   ? launch_resident(kernel<256, 8 __VA_OPT__(, 8)>, 256, args, S, s)          \
+   : resident_threads(S) == 512 ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)         \
+                                : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
   template <class Args>
   void launch_resident(void (*kernel)(Args, ResidentArgs), int threads, const Args &a, const Sell &S, cudaStream_t s) {
     const int chunks = resident_chunks(S);
@@ -1065,7 +1078,7 @@ struct cfsa_ns {
     r.bar = GridBarrier{bar_count, bar_err, mom_bar_spin_limit};
     r.part = res_part;
     r.stride = res_stride;
-    r.slots = slot_bytes > kMaxSlotBytes ? res_slots : nullptr;
+    r.slots = (sums_global || slot_bytes > kMaxSlotBytes) ? res_slots : nullptr;
     r.slots_per_cta = chunks * 6;
     clear_barrier(s);
     cudaLaunchConfig_t cfg = {};

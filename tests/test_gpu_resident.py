@@ -230,3 +230,58 @@ def test_vertices_of_no_tet(cf, po, extra, momentum, pressure):
     ref = o.state()
     assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
     assert s.stats()["pressure_iters"] == o.stats()["pressure_iters"] > 0
+
+
+# The momentum solves' forms (threads per CTA, chunk lengths, order of the vector phases) and the place of
+# their chunk sums are chosen by size; here each runs on small odd meshes.
+FORMS = [(t, g) for t in ("256", "512", "1024") for g in ("0", "1")]
+
+
+def formed(cf, monkeypatch, form, m, momentum, pressure, tol):
+    monkeypatch.setenv("CFSA_RESIDENT_THREADS", form[0])
+    monkeypatch.setenv("CFSA_SUMS_GLOBAL", form[1])
+    monkeypatch.setenv("CFSA_NO_WINDOWS", form[1])  # the pressure solve of meshes that large
+    return solver(cf, m, momentum, pressure, tol)
+
+
+# At 1e-30 BiCGSTAB passes its near-breakdown restart several times in both solves (on the oracle's side:
+# momentum n = 671, 3175 and 1995 and pressure n = 114, 481 and 320).
+@pytest.mark.parametrize("shape", [(2, 5), (3, 12), (9, 7, 3)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("momentum,tol", [(0, 1e-11), (1, 1e-30)], ids=["cg", "bicgstab_restarts"])
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f"{f[0]}{'_global' if f[1] == '1' else ''}")
+def test_forms_match_oracle(cf, po, monkeypatch, shape, momentum, tol, form):
+    m = mesh(cf, shape)
+    s = formed(cf, monkeypatch, form, m, momentum, cf.KRYLOV_BICGSTAB, tol)
+    o = po.Oracle(m.vertices(), m.tets())
+    o.set_fluid(RHO, NU)
+    o.set_params(dt=0.01, tol_mom=tol, tol_p=tol, maxit_mom=5000, maxit_p=20000, pressure_solver=0)
+    o.set_momentum_solver(1 if momentum == cf.KRYLOV_CG else 0)
+    o.initialize()
+    inlet = np.zeros((o.N2, 3))
+    inlet[:, 0] = 0.5
+    o.set_inlet(inlet)
+    for _ in range(2):
+        assert s.pisoStep() and o.piso_step() == 0
+    ref = o.state()
+    assert np.array_equal(s.getVelocity(), ref["u"]) and np.array_equal(s.getPressure(), ref["p"])
+    assert s.stats()["momentum_iters"] == o.stats()["momentum_iters"]
+
+
+@pytest.mark.parametrize("shape", [(2, 5), (9, 7, 3), (8, 31)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("momentum", [0, 1], ids=["cg", "bicgstab"])
+def test_mixed_forms_agree(cf, monkeypatch, shape, momentum):
+    m, got = mesh(cf, shape), []
+    for form in FORMS:
+        s = formed(cf, monkeypatch, form, m, momentum, cf.KRYLOV_CG2L, 1e-13)
+        s.setPrecision(cf.PRECISION_MIXED)
+        s.setConvergenceNorm(cf.NORM_JACOBI)
+        assert s.pisoSteps(2) == (True, 2)
+        got.append((s.getVelocity(), s.getPressure(), s.stats()["momentum_iters"], s.stats()["momentum_outer"]))
+    for g in got[1:]:
+        assert np.array_equal(g[0], got[0][0]) and np.array_equal(g[1], got[0][1])
+        assert g[2:] == got[0][2:] and max(g[3]) > 1
+    ref = solver(cf, m, momentum, cf.KRYLOV_CG2L, 1e-14)
+    ref.setConvergenceNorm(cf.NORM_JACOBI)
+    assert ref.pisoSteps(2) == (True, 2)
+    # both solves end at 1e-13 of their right-hand side in the scaled norm: 1e-6 as in the mixed tests
+    assert np.linalg.norm(got[0][0] - ref.getVelocity()) <= 1e-6 * np.linalg.norm(ref.getVelocity())
