@@ -1053,23 +1053,35 @@ struct cfsa_ns {
     const int nblk = (int)blocks_for(S.nrows);
     return std::max(S.max_run, kSlicesPerBlock * ((nblk + S.nruns - 1) / S.nruns));
   }
-  // Three forms of each kernel, fewer threads with longer chunks of a row in flight the fewer rows there
-  // are: rows to spare per thread hide a chunk's latency, a short run of rows wants it paid less often.
-  // Measured per momentum iteration, CG / BiCGSTAB, FP64, us (threads x entries per chunk):
-  //   rows        1024 x 4       512 x 8       256 x 8
-  //   45,347      38.8 /  67.9   26.7 / 53.1   24.9 /  45.1
-  //   144,499     43.1 /  85.9   32.3 / 61.7   42.1 /  77.9
-  //   355,395     61.3 / 110     56.1 / 106    79.0 / 147
-  //   696,987     104 / 215      112 / 234     151 / 304
-  static constexpr int kFewRows = 90000, kManyRows = 450000;
+  // Forms of the kernels by rows: fewer threads with longer chunks of a row in flight the fewer rows there
+  // are, since rows to spare per thread hide a chunk's latency and a short run of rows wants it paid less
+  // often. 1024 threads from kManyRows on; below, 512, and 256 for FP64 BiCGSTAB below kFewRows (it has the
+  // most vector phases, in which 256 threads take two chunks at once; the other solves are faster with 512
+  // at every size down to 95 rows). Measured, us per iteration with 256 / 512 / 1024 threads, tubes, and the
+  // same lines on a channel and a bifurcation of 140,000, 200,000 and 260,000 rows:
+  //   rows        FP64 CG            FP64 BiCGSTAB        mixed CG           mixed BiCGSTAB
+  //   549         15.4 13.9 14.0     26.5  28.1  24.5     14.7 12.5 12.5     28.2 24.9 23.9
+  //   17,577      20.1 18.3 22.2     33.2  37.8  36.6     19.2 17.7 19.9     34.4 33.1 35.1
+  //   45,347      23.9 23.2 28.8     38.6  47.1  50.9     23.8 21.7 24.1     41.9 39.8 42.6
+  //   78,875      29.4 24.7  -       49.4  51.3   -       27.3 22.3  -       49.9 41.6  -
+  //   91,495      30.5 26.1 31.3     50.1  52.0  54.1     28.6 23.2 25.0     52.2 43.2 45.2
+  //   105,377     33.1 26.7  -       57.4  54.4   -       31.8 23.7  -       59.5 45.2  -
+  //   131,537     38.4 30.4 33.5     66.7  59.8  60.1     37.0 26.7 27.2     69.5 51.5 49.4
+  //   156,047     44.0 32.9 34.6     75.8  63.8  62.4     42.7 29.0 28.3     78.4 54.8 51.2
+  //   180,557     47.0 34.6 35.4     78.7  67.4  64.9     44.0 30.6 29.6     80.6 58.4 53.5
+  //   200,165     50.5 37.8 36.4     86.8  74.8  66.7     48.0 33.0 30.1     90.0 63.0 54.8
+  //   354,341     75.6 55.2 50.8     129   109   95.1     69.9 45.6 39.3     126  84.7 71.0
+  //   686,181      -   93.8 78.8      -    196   156       -   72.7 58.3      -   139  109
+  static constexpr int kFewRows = 95000, kManyRows = 190000;
   int resident_threads(const Sell &S) const {
     if (form_threads) return form_threads;
     return S.nrows < kFewRows ? 256 : S.nrows < kManyRows ? 512 : 1024;
   }
-#define CFSA_RESIDENT(kernel, args, S, s, ...)                                                               \
-  (resident_threads(S) == 256   ? launch_resident(kernel<256, 8 __VA_OPT__(, 8)>, 256, args, S, s)          \
-   : resident_threads(S) == 512 ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)         \
-                                : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
+#define CFSA_RESIDENT(kernel, args, S, s, ...)                                                                   \
+  (resident_threads(S) <= 512 ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)               \
+                              : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
+#define CFSA_RESIDENT_BICG(kernel, args, S, s)                                                                   \
+  (resident_threads(S) == 256 ? launch_resident(kernel<256, 8>, 256, args, S, s) : CFSA_RESIDENT(kernel, args, S, s))
   template <class Args>
   void launch_resident(void (*kernel)(Args, ResidentArgs), int threads, const Args &a, const Sell &S, cudaStream_t s) {
     const int chunks = resident_chunks(S);
@@ -1176,7 +1188,7 @@ struct cfsa_ns {
       CK(cudaGetLastError());
       CFSA_RESIDENT(k_mcg_solve, a, s2, stream);
     } else {
-      CFSA_RESIDENT(k_bicg_solve3, a, s2, stream);
+      CFSA_RESIDENT_BICG(k_bicg_solve3, a, s2, stream);
     }
     k_check_bicg<<<1, 1, 0, stream>>>(bs_mom, 3, 0, s_out, bar_err);
     CK(cudaGetLastError());
@@ -2287,10 +2299,17 @@ struct cfsa_ns {
       a.v = ws;  // scratch output
       // the product phase of the momentum solve (BiCGSTAB: v = At p with r0.v; CG: q = A p with p.q);
       // same matrix stream, gathers and algorithmic bytes
-      if (mom_krylov == CFSA_KRYLOV_CG) a.r0 = a.pk;
-      CFSA_RESIDENT(k_momentum_product, (MomentumProductArgs{a, 1}), s2, stream);  // warm-up
+      const bool cg = mom_krylov == CFSA_KRYLOV_CG;
+      if (cg) a.r0 = a.pk;
+      auto run = [&](int n) {
+        if (cg)
+          CFSA_RESIDENT(k_momentum_product, (MomentumProductArgs{a, n}), s2, stream);
+        else
+          CFSA_RESIDENT_BICG(k_momentum_product, (MomentumProductArgs{a, n}), s2, stream);
+      };
+      run(1);  // warm-up
       CK(cudaEventRecord(ev0, stream));
-      CFSA_RESIDENT(k_momentum_product, (MomentumProductArgs{a, iters}), s2, stream);
+      run(iters);
       CK(cudaEventRecord(ev1, stream));
       *alg_bytes = 12.0 * (double)nnz2 + 8.0 * s2.nrows_pad + 4.0 * (s2.nslices + 1) + 72.0 * (double)N2;
     } else if (which == CFSA_KERNEL_PRESSURE_SPMV) {
