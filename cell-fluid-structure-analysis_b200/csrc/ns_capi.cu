@@ -47,8 +47,10 @@ struct Windows {
   WindowView view() const { return WindowView{ptr, col, idx}; }
 };
 
-// Operators of at most this many rows are solved by one CTA, whose barriers are block-wide ones: a
-// momentum CG iteration of 549 rows takes 17 us in one CTA and 20 us on several, of 1037 rows 23 and 20.
+// Operators of at most this many rows are solved by one CTA, whose barriers are block-wide ones. Momentum
+// iteration in one CTA / on several, us: 549 rows CG 13.5 / 14.8 and BiCGSTAB 25.6 / 26.4, mixed 12.1 / 14.1
+// and 24.1 / 27.7; 793 rows 14.6 / 15.2 and 30.2 / 27.2, mixed 13.4 / 14.7 and 24.8 / 26.6; 1,037 rows 16.9 /
+// 16.0 and 36.3 / 28.6, mixed 15.4 / 15.5 and 29.8 / 28.6.
 constexpr int kOneCtaRows = 768;
 
 struct Sell {
@@ -293,7 +295,7 @@ struct cfsa_ns {
   int64_t adj_launches_fixed = 0;
   int64_t batch_launches = 0;
   int64_t batch_iters[2] = {0, 0};
-  int launches_per_step = 0;  // kernels of one step outside the Krylov loop bodies
+  int launches_per_step = 0;  // kernels of one step outside the Krylov solves
 
   bool mom_dirty = true, poisson_dirty = true, graph_dirty = true;
   bool use_graph = true;
@@ -1713,8 +1715,8 @@ struct cfsa_ns {
 
   void reset_status() { CK(cudaMemsetAsync(st, 0, sizeof(DevStatus), stream)); }
 
-  // Kernels of one pressure-solve body run (counted by DevStatus::body_runs[1]) and the extra
-  // fixed kernels of a mixed-precision step, for the launch counts.
+  // Kernels of one pressure-solve body run (counted by DevStatus::body_runs[1]: a resident solve, a sweep
+  // or an iteration) and the extra fixed kernels of a mixed-precision step, for the launch counts.
   bool momentum_mixed() const { return precision != CFSA_PRECISION_FP64; }
   bool pressure_mixed() const { return precision == CFSA_PRECISION_MIXED_FULL && krylov == CFSA_KRYLOV_CG2L; }
   int pressure_body_kernels() const {
@@ -1734,9 +1736,9 @@ struct cfsa_ns {
     CK(cudaStreamSynchronize(stream));
     CK(cudaEventElapsedTime(&last_ms, ev0, ev1));
     const int pressure_body = pressure_body_kernels();
-    // momentum: 5 kernels per BiCGSTAB iteration, 3 per CG iteration; mixed momentum: 2 more per
-    // reliable update (x update, residual) and an init kernel per solve, as has FP64 CG; mixed
-    // two-level CG pressure: 4 kernels per sweep plus its init
+    // fixed kernels of a step and the init kernels of the methods that have one, one kernel per resident
+    // solve, and per body run of the other pressure forms pressure_body_kernels() (4 per sweep of the mixed
+    // two-level CG, 3 per iteration of the multi-kernel CG)
     batch_launches = (int64_t)launched_steps * (launches_per_step + mixed_fixed_kernels()) +
                      (int64_t)h_st->body_runs[0] + pressure_body * (int64_t)h_st->body_runs[1];
     batch_iters[0] = (int64_t)h_st->iters[0];
@@ -2157,7 +2159,7 @@ struct cfsa_ns {
     k_adj_mom_out<<<blocks_for(s2.nrows_pad), kBlock, 0, stream>>>(o);
     CK(cudaGetLastError());
     // correct, [sum,] chain per corrector, pressure rhs + check, momentum rhs + check,
-    // conv_tet, mom_out (Krylov loop bodies counted from the status)
+    // conv_tet, mom_out (Krylov solves and loop bodies counted from the status)
     adj_launches_fixed = 1 + ncorr * (normalize ? 2 : 1) + 2 + 2 + 2 + mixed_fixed_kernels();
   }
 

@@ -1405,7 +1405,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_cg_persistent(CgPersistentArgs A)
 // block-wide steps of an iteration (half a dozen) cost less with 16 warps than with 32. Two-level CG, us per
 // iteration with 1024 / 768 / 512 threads: 16.1 / 12.9 / 11.7 at 30k tets, 14.9 / 13.8 / 11.8 at 250k,
 // 24.7 / 20.8 / 19.0 at 1M. Without windows 1024: the gathers from L2 and HBM want warps in flight; CG on a
-// 4M-tet bifurcation takes 104 us per iteration with 512 threads and 79 with 1024.
+// 4M-tet bifurcation takes 104 us per iteration with 512 threads and 79 with 1024 (64 registers, of which the
+// two-level kernels spill 68 and 72 bytes).
 template <bool WIN>
 constexpr int kCgResThreads = WIN ? 512 : 1024;
 template <bool WIN>

@@ -109,10 +109,11 @@ struct Resident {
   // i, with acc[c] the row's product, own[c] = own(c, i) and part its NV sums. One thread per row adds
   // its entries in ascending column order (as sell_spmv_row), in chunks of U: indices and values, then
   // the gathers, then the sums. Bound: L1 serves the gathers, about six cycles of the SM for 32 lanes
-  // spread over eleven lines (70% of its throughput at 415k tets, DRAM 39%). With one or two FP64
-  // components, and in the form for small meshes, the next chunk's indices and values are requested
-  // along with the gathers; with three, or in FP32, the registers that holds are worth more to longer chunks: three components at 1M tets 118
-  // against 139 us (577 MB, 4.9 TB/s), FP32 81 against 98 us; two components 95 against 100 us.
+  // spread over eleven lines (under ncu at 415k tets 73% of its peak, DRAM 0.57 of the copy rate). With one
+  // or two FP64 components, and in the 256-thread form, the next chunk's indices and values are requested
+  // along with the gathers; with three, or in FP32, the registers that holds are worth more to longer
+  // chunks: three components at 1M tets 118 against 139 us (577 MB, 4.9 TB/s), FP32 81 against 98 us; two
+  // components 95 against 100 us.
   // load(c, j) reads entry j of x_c with a plain load, since other CTAs rewrite x between the phases of
   // a launch.
   template <int NV, int NC, int U, int MASK, class TV, class TA, class L, class O, class F>
@@ -183,11 +184,12 @@ struct Resident {
   }
 
   // Vector phase: apply(c, i, common(i), load(c, i), scalar(c), part) for every entry i < n of the CTA's
-  // natural blocks and every component c in `mask`, the loads ahead of the stores; value 3 v + c of the phase sums part[v] (NV = 0: no
-  // sums). With 1024 threads the components follow one another and two chunks' loads are in flight, which
-  // fits 64 registers where all components of one entry at a time spill (momentum CG iteration at 1M tets 180
-  // -> 161 us); with fewer threads there is room for all components at once, and short ranges want the
-  // latency paid once (250k tets 54 against 57 us).
+  // natural blocks and every component c in `mask`, the loads ahead of the stores; value 3 v + c of the phase
+  // sums part[v] (NV = 0: no sums). With 1024 threads the components follow one another and two chunks' loads
+  // are in flight, which leaves the 64 registers of a thread room (FP64 BiCGSTAB spills 36 bytes, the other
+  // solves none) where all components of one entry at a time did not (momentum CG iteration at 1M tets
+  // 180 -> 161 us); with fewer threads there is room for all components at once, and short ranges want the
+  // latency paid once (512 threads at 250k tets 54 against 57 us).
   template <int NV, class S, class C, class L, class F>
   __device__ __forceinline__ void vector(int n, int mask, S &&scalar, C &&common, L &&load, F &&apply) {
     using V = decltype(load(0, 0));
