@@ -1074,16 +1074,20 @@ struct cfsa_ns {
   //   200,165     50.5 37.8 36.4     86.8  74.8  66.7     48.0 33.0 30.1     90.0 63.0 54.8
   //   354,341     75.6 55.2 50.8     129   109   95.1     69.9 45.6 39.3     126  84.7 71.0
   //   686,181      -   93.8 78.8      -    196   156       -   72.7 58.3      -   139  109
+  // CFSA_RESIDENT_THREADS reaches the 256-thread kernels of the other solves too. (Without them the compiler's
+  // code for FP64 BiCGSTAB's is 2% slower, same registers: 40.8 against 39.9 us per iteration at 45,347 rows.)
   static constexpr int kFewRows = 95000, kManyRows = 190000;
-  int resident_threads(const Sell &S) const {
+  int resident_threads(const Sell &S, bool fp64_bicg) const {
     if (form_threads) return form_threads;
-    return S.nrows < kFewRows ? 256 : S.nrows < kManyRows ? 512 : 1024;
+    return (fp64_bicg && S.nrows < kFewRows) ? 256 : S.nrows < kManyRows ? 512 : 1024;
   }
-#define CFSA_RESIDENT(kernel, args, S, s, ...)                                                                   \
-  (resident_threads(S) <= 512 ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)               \
-                              : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
-#define CFSA_RESIDENT_BICG(kernel, args, S, s)                                                                   \
-  (resident_threads(S) == 256 ? launch_resident(kernel<256, 8>, 256, args, S, s) : CFSA_RESIDENT(kernel, args, S, s))
+#define CFSA_RESIDENT_FORM(threads, kernel, args, S, s, ...)                                             \
+  (threads == 256   ? launch_resident(kernel<256, 8 __VA_OPT__(, 8)>, 256, args, S, s)                  \
+   : threads == 512 ? launch_resident(kernel<512, 8 __VA_OPT__(, 10)>, 512, args, S, s)                 \
+                    : launch_resident(kernel<1024, 4 __VA_OPT__(, __VA_ARGS__)>, 1024, args, S, s))
+#define CFSA_RESIDENT(kernel, args, S, s, ...) \
+  CFSA_RESIDENT_FORM(resident_threads(S, false), kernel, args, S, s __VA_OPT__(, ) __VA_ARGS__)
+#define CFSA_RESIDENT_BICG(kernel, args, S, s) CFSA_RESIDENT_FORM(resident_threads(S, true), kernel, args, S, s)
   template <class Args>
   void launch_resident(void (*kernel)(Args, ResidentArgs), int threads, const Args &a, const Sell &S, cudaStream_t s) {
     const int chunks = resident_chunks(S);
@@ -2303,15 +2307,10 @@ struct cfsa_ns {
       // same matrix stream, gathers and algorithmic bytes
       const bool cg = mom_krylov == CFSA_KRYLOV_CG;
       if (cg) a.r0 = a.pk;
-      auto run = [&](int n) {
-        if (cg)
-          CFSA_RESIDENT(k_momentum_product, (MomentumProductArgs{a, n}), s2, stream);
-        else
-          CFSA_RESIDENT_BICG(k_momentum_product, (MomentumProductArgs{a, n}), s2, stream);
-      };
-      run(1);  // warm-up
+      const int threads = resident_threads(s2, !cg);
+      CFSA_RESIDENT_FORM(threads, k_momentum_product, (MomentumProductArgs{a, 1}), s2, stream);  // warm-up
       CK(cudaEventRecord(ev0, stream));
-      run(iters);
+      CFSA_RESIDENT_FORM(threads, k_momentum_product, (MomentumProductArgs{a, iters}), s2, stream);
       CK(cudaEventRecord(ev1, stream));
       *alg_bytes = 12.0 * (double)nnz2 + 8.0 * s2.nrows_pad + 4.0 * (s2.nslices + 1) + 72.0 * (double)N2;
     } else if (which == CFSA_KERNEL_PRESSURE_SPMV) {

@@ -233,8 +233,7 @@ def test_vertices_of_no_tet(cf, po, extra, momentum, pressure):
 
 
 # The momentum solves' forms (threads per CTA, chunk lengths, order of the vector phases) and the place of
-# their chunk sums are chosen by size; here each runs on small odd meshes. 256 threads are a form of FP64
-# BiCGSTAB only; the other solves take 512 for it.
+# their chunk sums are chosen by size; here each runs on small odd meshes.
 FORMS = [(t, g) for t in ("256", "512", "1024") for g in ("0", "1")]
 
 
