@@ -285,3 +285,16 @@ def test_mixed_forms_agree(cf, monkeypatch, shape, momentum):
     assert ref.pisoSteps(2) == (True, 2)
     # both solves end at 1e-13 of their right-hand side in the scaled norm: 1e-6 as in the mixed tests
     assert np.linalg.norm(got[0][0] - ref.getVelocity()) <= 1e-6 * np.linalg.norm(ref.getVelocity())
+
+
+@pytest.mark.parametrize("shape", [(4, 9), (11, 9, 7)], ids=lambda s: "x".join(map(str, s)))
+def test_windows_do_not_change_the_bits_of_float_sweeps(cf, monkeypatch, shape):
+    m, got = mesh(cf, shape), []
+    for off in ("0", "1"):
+        monkeypatch.setenv("CFSA_NO_WINDOWS", off)
+        s = solver(cf, m, cf.KRYLOV_CG, cf.KRYLOV_CG2L, 1e-10)
+        s.setPrecision(cf.PRECISION_MIXED_FULL)
+        assert s.pisoSteps(2) == (True, 2)
+        got.append((s.getVelocity(), s.getPressure(), s.stats()["pressure_iters"], s.stats()["pressure_outer"]))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    assert got[0][2:] == got[1][2:] and got[0][3] > 1
